@@ -128,7 +128,8 @@ struct tpd_engine {
     uint64_t keys64_cap = 0;
     uint32_t* d_vals[2] = {nullptr, nullptr};
     uint64_t* d_desc_sort = nullptr;
-    uint32_t* d_sort_work = nullptr;  // counted key-sort passes: partition counts and offsets (zero at rest)
+    uint32_t* d_sort_work = nullptr;  // counted key-sort passes: partition counts and offsets
+    uint32_t* d_part_first = nullptr;  // first item of every 4096-key partition
     uint32_t* d_ranges = nullptr;
     uint64_t pixel_cap = 0, tile_cap = 0;
     float* d_image = nullptr;
@@ -286,6 +287,7 @@ int ensure_key_capacity(tpd_engine* e, uint64_t want) {
     const size_t words = sort_counted_work_words(uint32_t(want));
     TPD_CUDA(e, dalloc(e->d_sort_work, words));
     TPD_CUDA(e, cudaMemset(e->d_sort_work, 0, words * 4));
+    TPD_CUDA(e, dalloc(e->d_part_first, want / 4096 + 1));
     e->capacity = want;
     return TPD_OK;
 }
@@ -404,14 +406,7 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     pa.depth_keys = e->d_dkeys[0];
     pa.depth_items = e->d_ditems[0];
     pa.depth_key_bits = e->depth_key_bits;
-    pa.tile_bits = e->key_bits - 32;  // the key sort's digit counts
     pa.ctl = e->d_ctl;
-    // counted key-sort passes (default): keygen counts the first pass's
-    // partition rows, which the preprocess clears
-    const bool counted = e->settings.key_sort_lookback == 0;
-    const uint32_t key_parts = std::max(1u, uint32_t((e->capacity + 4095u) / 4096u));
-    pa.zero_words = counted ? e->d_sort_work : nullptr;
-    pa.zero_count = counted ? uint64_t(key_parts) * 256u : 0u;
     launch_preprocess(pa, e->num_sms, s);
     mark(1);
     const uint32_t spin = e->settings.spin_limit ? e->settings.spin_limit : kDefaultSpin;
@@ -435,10 +430,31 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     const uint32_t* order_other = e->d_ditems[e->depth_in_alt ? 0 : 1];
     mark(2);
     const uint32_t cap = uint32_t(e->capacity);
-    launch_keygen_scan(e->d_splats, order, order_other, items, e->n, e->d_views, e->d_offsets, e->d_tiles[0],
-                       e->d_vals[0], cap, e->d_ranges, e->total_tiles, e->d_desc_pre,
-                       counted ? e->d_sort_work : nullptr, e->d_ctl, spin, e->settings.test_never_publish, e->num_sms,
-                       s);
+    const bool counted = e->settings.key_sort_lookback == 0;  // counted key-sort passes (default)
+    KeygenArgs ka{};
+    ka.splats = e->d_splats;
+    ka.items = order;
+    ka.items_other = order_other;
+    ka.n_items = items;
+    ka.n = e->n;
+    ka.views = e->d_views;
+    ka.offsets = e->d_offsets;
+    // the depth sort's key buffers are free now: the items' rectangles and slots
+    ka.item_rects = reinterpret_cast<uint2*>(e->d_dkeys[0]);
+    ka.item_slots = reinterpret_cast<uint2*>(e->d_dkeys[1]);
+    ka.part_first = e->d_part_first;
+    ka.tiles = e->d_tiles[0];
+    ka.vals = e->d_vals[0];
+    ka.capacity = cap;
+    ka.ranges = e->d_ranges;
+    ka.n_tiles = e->total_tiles;
+    ka.tile_bits = e->key_bits - 32;
+    ka.desc = e->d_desc_pre;
+    ka.counted_work = counted ? e->d_sort_work : nullptr;
+    ka.ctl = e->d_ctl;
+    ka.spin_limit = spin;
+    ka.never_publish = e->settings.test_never_publish;
+    launch_keygen(ka, e->num_sms, s);
     mark(3);
     SortPlan kp;
     kp.first_bit = 0;  // tile ids; the depth half of the keys is already in order
@@ -455,7 +471,7 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     // counted passes (default), or onesweep passes with a look-back
     if (counted) {
         kp.counted_work = e->d_sort_work;
-        kp.precounted = true;  // keygen counted the first pass's rows
+        kp.precounted = true;  // keygen counted the first pass
         kp.ctas_per_sm = e->settings.sort_ctas_per_sm == 2 ? 2 : 3;
     }
     e->sorted_in_alt = launch_sort(e->d_tiles[0], e->d_vals[0], e->d_tiles[1], e->d_vals[1], cap, kp, e->d_desc_sort,
@@ -788,6 +804,7 @@ void tpd_destroy(tpd_engine* e) {
     }
     dfree(e->d_desc_sort);
     dfree(e->d_sort_work);
+    dfree(e->d_part_first);
     dfree(e->d_keys64);
     dfree(e->d_ranges);
     dfree(e->d_image);

@@ -14,10 +14,8 @@
 // can give up with a copy in flight, and the CTA drains every copy it issued
 // before it exits. Besides the splat, each (view, Gaussian) gets a
 // depth-sort key (view << 32 | bits(viewZ)) whose digit histograms are
-// accumulated here, and the digits of the tile ids its keys will carry are
-// counted from its tile rectangle for the key sort (count_tile_row). The tile
-// counts are scanned afterwards in depth order, inside keygen.cu's fused scan
-// and key duplication (scan_tiles_kernel is the standalone scan). Arithmetic
+// accumulated here. The tile counts are scanned afterwards in depth order
+// (keygen.cu; scan_tiles_kernel is the standalone scan). Arithmetic
 // follows the shader source left to right with matrix products accumulated
 // k = 0..n-1; this file is compiled with --fmad=false so no product is fused
 // into an add.
@@ -113,10 +111,9 @@ struct Rec {
 };
 
 // project() for one Gaussian. Returns the tile count (0 when culled) and fills
-// s; rect gets the tile rectangle (x0, y0, x1, y1) when the count is not 0,
-// the one key duplication derives from the stored splat's px, py and radius.
+// s.
 __device__ __forceinline__ uint32_t project_one(const Rec& rec, const float* em, const ViewConst& v,
-                                                uint32_t deg, bool compat, Splat& s, uint4& rect) {
+                                                uint32_t deg, bool compat, Splat& s) {
     s = Splat{0.f, 0.f, 0.f, 0u, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const float4 pos_op = rec.f4(0);
     const float mean[3] = {pos_op.x, pos_op.y, pos_op.z};
@@ -187,7 +184,6 @@ __device__ __forceinline__ uint32_t project_one(const Rec& rec, const float* em,
     bounding_rect(px, py, radius, grid_x(v.width), grid_y(v.height), x0, y0, x1, y1);
     const uint32_t touched = (x1 - x0) * (y1 - y0);
     if (touched == 0) return 0;
-    rect = make_uint4(x0, y0, x1, y1);
 
     // camera position (common.slang:88-92) and view direction from the pre-model mean
     float campos[3];
@@ -254,49 +250,11 @@ __device__ __forceinline__ uint32_t project_one(const Rec& rec, const float* em,
 constexpr uint32_t kPreStages = 2;
 constexpr uint32_t kDepthPassesMax = 5;  // depth keys: 32 bits + log2(256 views)
 
-constexpr uint32_t kTileDigitsMax = 4;   // tile ids: at most 32 bits
-
 struct PreSmem {
     float rec[kPreStages][kPreThreads * kRecordFloats];  // 30,720 B per stage, 16-byte multiple
     uint32_t hist[kDepthPassesMax][256];                  // depth-key digit counts of this CTA
-    // tile-id digit counts of this CTA: digit 0 as a difference array over
-    // the 256 values (+ tall added to every value), the others directly
-    uint32_t tdiff[257];
-    uint32_t tall;
-    uint32_t thist[kTileDigitsMax - 1][256];
     uint32_t kept;                                        // depth keys of visible items in this CTA
 };
-
-// Adds the w consecutive tile ids a0 .. a0 + w - 1 (one row of a Gaussian's
-// tile rectangle, all below 2^tile_bits) to the CTA's digit counts of the
-// key sort: digit 0 (t & 255) takes w / 256 on every value and a range of
-// w % 256 values (wrapping) in the difference array; digit p >= 1 takes, for
-// each value v of t >> 8p in the row, the number of ids with that value.
-__device__ __forceinline__ void count_tile_row(PreSmem& S, uint32_t a0, uint32_t w, uint32_t ndig) {
-    if (w >= 256u) atomicAdd(&S.tall, w >> 8);
-    const uint32_t rem = w & 255u;
-    if (rem) {
-        const uint32_t st = a0 & 255u, e = st + rem;
-        atomicAdd(&S.tdiff[st], 1u);
-        if (e <= 256u) {
-            atomicAdd(&S.tdiff[e], 0xFFFFFFFFu);  // -1 (tdiff[256] is never read)
-        } else {
-            atomicAdd(&S.tdiff[0], 1u);
-            atomicAdd(&S.tdiff[e - 256u], 0xFFFFFFFFu);
-        }
-    }
-    const uint32_t last = a0 + (w - 1u);  // tile ids stay below 2^31
-    for (uint32_t p = 1; p < ndig; ++p) {
-        const uint32_t sh = 8u * p, v0 = a0 >> sh, v1 = last >> sh;
-        if (v0 == v1) {
-            atomicAdd(&S.thist[p - 1][v0 & 255u], w);
-        } else {
-            atomicAdd(&S.thist[p - 1][v0 & 255u], ((v0 + 1u) << sh) - a0);
-            for (uint32_t v = v0 + 1u; v < v1; ++v) atomicAdd(&S.thist[p - 1][v & 255u], 1u << sh);
-            atomicAdd(&S.thist[p - 1][v1 & 255u], last - (v1 << sh) + 1u);
-        }
-    }
-}
 
 // (3 CTAs per SM fit in shared memory: registers up to 170 per thread are free)
 __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessArgs a) {
@@ -305,14 +263,10 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
 
     const uint32_t tid = threadIdx.x;
     for (uint32_t k = tid; k < kDepthPassesMax * 256; k += kPreThreads) (&S.hist[0][0])[k] = 0;
-    for (uint32_t k = tid; k < 257; k += kPreThreads) S.tdiff[k] = 0;
     // launched as a dependent of frame_begin_kernel (the frame's control block).
     // No early trigger: the depth sort's first pass is one wave of CTAs, which
     // must be placed on empty SMs, not onto the first ones this grid frees
     pdl_wait();
-    for (uint32_t k = tid; k < (kTileDigitsMax - 1) * 256; k += kPreThreads) (&S.thist[0][0])[k] = 0;
-    if (tid == 0) S.tall = 0;
-    const uint32_t ndig = min(kTileDigitsMax, (a.tile_bits + 7) / 8);  // 0: no tile-digit counts
     if (tid == 0) S.kept = 0;
     uint32_t kept = 0;  // this thread's visible items (the depth sort drops the others)
     const uint32_t nchunks = (a.n + kPreThreads - 1) / kPreThreads;
@@ -328,15 +282,6 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
     };
     if (blockIdx.x < nchunks) issue(blockIdx.x, 0);
     cp_async_commit();
-    // (while the first records arrive) the words to clear: the key sort's
-    // precounted rows, which keygen adds its digit counts into
-    if (a.zero_words) {
-        uint4* z = reinterpret_cast<uint4*>(a.zero_words);
-        const uint64_t n4 = a.zero_count / 4u;
-        for (uint64_t k = uint64_t(blockIdx.x) * kPreThreads + tid; k < n4; k += uint64_t(gridDim.x) * kPreThreads)
-            z[k] = make_uint4(0u, 0u, 0u, 0u);
-    }
-
     uint32_t it = 0;
     for (uint32_t chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x, ++it) {
         const uint32_t stage = it & 1u;
@@ -354,7 +299,6 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
         const uint32_t e = (tid < cnt && a.ent_idx) ? a.ent_idx[i] : 0u;
         for (uint32_t v = 0; v < a.n_views; ++v) {
             Splat sp;
-            uint4 rect = make_uint4(0u, 0u, 0u, 0u);
             uint32_t tiles = 0;
             if (tid < cnt) {
                 const float* em = a.ent_mats + (size_t(v) * a.n_ent + e) * kEntityMatFloats;
@@ -362,7 +306,7 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
 #pragma unroll
                 for (int k = 0; k < kEntityMatFloats; ++k) emr[k] = __ldg(em + k);
                 tiles = project_one(Rec{S.rec[stage] + tid * kRecordFloats}, emr, a.views[v], a.sh_degree,
-                                    a.band3_compat != 0, sp, rect);
+                                    a.band3_compat != 0, sp);
             } else {
                 sp = Splat{0.f, 0.f, 0.f, 0u, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             }
@@ -387,56 +331,10 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
                     }
                 }
             }
-            if (ndig) {
-                // the keys the warp's items will emit, the tile ids of their
-                // rectangles: the rows of all 32 rectangles are spread over the
-                // lanes (row r goes to lane r % 32, which finds the rectangle
-                // holding it by a binary search over the warp's row prefix)
-                const uint32_t lane = tid & 31u;
-                const uint32_t h = tiles ? rect.w - rect.y : 0u;
-                const uint32_t incl = warp_inclusive_scan(h);
-                const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-                if (total) {
-                    const ViewConst& vc = a.views[v];
-                    const uint32_t gx = grid_x(vc.width);
-                    const uint32_t row0 = vc.tile_base + rect.y * gx + rect.x, w = rect.z - rect.x, excl = incl - h;
-                    for (uint32_t r0 = 0; r0 < total; r0 += 32u) {
-                        const uint32_t r = r0 + lane;
-                        uint32_t own = 0;  // lanes whose rows all come before row r
-#pragma unroll
-                        for (uint32_t step = 16; step; step >>= 1)
-                            if (__shfl_sync(0xFFFFFFFFu, incl, own + step - 1u) <= r) own += step;
-                        own = min(own, 31u);
-                        const uint32_t o_row0 = __shfl_sync(0xFFFFFFFFu, row0, own);
-                        const uint32_t o_w = __shfl_sync(0xFFFFFFFFu, w, own);
-                        const uint32_t o_excl = __shfl_sync(0xFFFFFFFFu, excl, own);
-                        if (r < total) count_tile_row(S, o_row0 + (r - o_excl) * gx, o_w, ndig);
-                    }
-                }
-            }
         }
         __syncthreads();  // every thread is done with this stage before it is refilled
     }
     cp_async_wait_all();  // nothing is left in flight (the last groups are empty)
-    if (ndig) {
-        __syncthreads();
-        // digit 0: inclusive prefix of the difference array (two values per
-        // thread, 128 threads), plus the counts added to every value
-        const uint32_t d0 = 2u * tid, d1 = d0 + 1u;
-        const uint32_t v0 = S.tdiff[d0], pair = v0 + S.tdiff[d1];
-        const uint32_t incl = warp_inclusive_scan(pair);
-        __shared__ uint32_t wsum[kPreThreads / 32];
-        if ((tid & 31u) == 31u) wsum[tid >> 5] = incl;
-        __syncthreads();
-        uint32_t before = 0;
-        for (uint32_t w = 0; w < (tid >> 5); ++w) before += wsum[w];
-        const uint32_t c1 = before + incl + S.tall, c0 = c1 - S.tdiff[d1];
-        if (c0) atomicAdd(&a.ctl->sort_hist[0][d0], c0);
-        if (c1) atomicAdd(&a.ctl->sort_hist[0][d1], c1);
-        for (uint32_t p = 1; p < ndig; ++p)
-            for (uint32_t d = tid; d < 256; d += kPreThreads)
-                if (S.thist[p - 1][d]) atomicAdd(&a.ctl->sort_hist[p][d], S.thist[p - 1][d]);
-    }
     if (!a.depth_keys) return;
     kept = warp_sum(kept);
     if ((tid & 31u) == 0 && kept) atomicAdd(&S.kept, kept);
@@ -450,7 +348,7 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
 // Exclusive scan of Splat.tiles over partitions of 256 threads x 4 items
 // (prefix.slang:40-158), partitions taken by atomic ticket. Total ->
 // ctl->total_keys, non-empty count -> ctl->visible. (The frame scans its
-// counts in depth order inside keygen_scan_kernel.)
+// counts in depth order, scan_items_kernel.)
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanItems = 4;
 

@@ -8,11 +8,11 @@
 //
 // GB300 form (onesweep): 8-bit digits, so a 45-bit (tile | depth) key takes 6
 // passes instead of 23.
-//  1. In the frame the digit histograms come from earlier kernels: the
-//     preprocess counts the depth keys' digits and the tile ids' digits (from
-//     each Gaussian's tile rectangle); sort_histogram_kernel builds them for
-//     standalone sorts (one read of the keys, warp match-any aggregation into
-//     shared memory, one global atomic per bin per CTA).
+//  1. In the frame the digit histograms come from earlier kernels (the
+//     preprocess counts the depth keys' digits, key duplication those of the
+//     tile ids); sort_histogram_kernel builds them for standalone sorts (one
+//     read of the keys, warp match-any aggregation into shared memory, one
+//     global atomic per bin per CTA).
 //  2. onesweep_kernel, once per pass: a persistent CTA takes 4096-key
 //     partitions by atomic ticket, loads them with coalesced warp-striped
 //     loads, ranks keys per warp (bit ballots, or match-any in the 512-thread
@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "tpd_common.cuh"
+#include "tpd_counted.cuh"
 #include "tpd_kernels.h"
 #include "tpd_scan.cuh"
 
@@ -43,7 +44,6 @@ namespace {
 constexpr uint32_t kRadixBits = 8;
 constexpr uint32_t kRadix = 1u << kRadixBits;
 constexpr uint32_t kSortThreads = 256;
-constexpr uint32_t kSortWarps = kSortThreads / 32;
 // Keys per thread of a radix pass: 16 (4096-key partitions) for large sorts;
 // 8 or 4 give more, shorter partitions when the sort is too small to fill the
 // GPU with 4096-key partitions (the depth sort of 1M Gaussians).
@@ -85,21 +85,6 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
-}
-
-// Block-wide exclusive scan of one value per thread (kWarps warps); returns the exclusive prefix.
-template <uint32_t kWarps = kSortWarps>
-__device__ __forceinline__ uint32_t block_exclusive_scan256(uint32_t v, uint32_t* wsum) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t incl = warp_inclusive_scan(v);
-    if (lane == 31) wsum[warp] = incl;
-    __syncthreads();
-    uint32_t base = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kWarps; ++w)
-        if (w < warp) base += wsum[w];
-    __syncthreads();
-    return base + incl - v;
 }
 
 __global__ void sort_begin_kernel(FrameCtl* ctl, uint32_t total) {
@@ -284,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     // global exclusive digit offsets (histogram of this pass, scanned)
     const uint32_t h = digit_thread && TPD_INBOUNDS(ctl, 16, pass, 8) ? hist[pass][tid] : 0u;
     {
-        const uint32_t ex = block_exclusive_scan256<kWarps>(h, S.wsum);
+        const uint32_t ex = block_exclusive_scan<kWarps>(h, S.wsum);
         if (digit_thread) S.gdig[tid] = ex;
     }
     if constexpr (kPass == kPassCompacted) {
@@ -393,7 +378,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
             dp = desc + size_t(TPD_INBOUNDS(ctl, 13, part, nparts) ? part : 0) * kRadix + tid;
             st_relaxed_u64(dp, make_desc(part == 0 ? kFlagPrefix : kFlagAggregate, tag, count));
         }
-        const uint32_t lstart = block_exclusive_scan256<kWarps>(count, S.wsum);  // (its barriers cover whist)
+        const uint32_t lstart = block_exclusive_scan<kWarps>(count, S.wsum);  // (its barriers cover whist)
         if (digit_thread) S.lstart[tid] = lstart;
         if (kDrop && tid == kRadix - 1) S.valid = lstart + count;
         __syncthreads();
@@ -479,72 +464,18 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 // partition, after load and rank 3.0, scan 0.4, write-out 2.6). A counted pass
 // computes every partition's digit offsets beforehand instead:
 //  1. partition_count_kernel, one CTA per 4096-key partition: the partition's
-//     digit counts (per-warp shared-memory counts) as a row of work[]. The
-//     last CTA of each chunk of kChunkParts partitions to finish (an atomic
-//     arrival count; nobody waits) scans the chunk's rows per digit in place
-//     into offsets within the chunk and writes the chunk's totals; the last
-//     chunk to finish scans the chunk totals, starting from the pass's global
-//     digit offsets, into each chunk's base. Arrival counts are reset by the
-//     CTA that finishes them, so the work area is zero at rest.
+//     digit counts (per-warp shared-memory counts), stored as a row of the
+//     work area and scanned by the last CTAs to arrive (counted_finish in
+//     tpd_counted.cuh; nobody waits). The first pass of the frame's key sort
+//     is counted by the kernel that writes its keys (keygen.cu) instead.
 //  2. scatter_kernel, one CTA per partition: load, rank (bit ballots, stable
-//     in warp-striped order), reorder in shared memory and write out at
-//     chunk base + offset within chunk, as onesweep_kernel does but with its
-//     offsets known: no partition waits for another.
+//     in warp-striped order), reorder in shared memory and write out at the
+//     partition's global digit offsets, as onesweep_kernel does but with them
+//     known: no partition waits for another.
 // The permutation is the same stable one.
-constexpr uint32_t kChunkParts = 32;
-
-// Layout of a counted pass's work area (u32 words), for P partitions:
-// [0, 256 P) rows of digit counts, then offsets within their chunk;
-// [256 P, 256 P + 256 C) chunk totals, then chunk bases (C chunks);
-// [256 (P + C), + C) chunk arrival counts; then one arrival count of chunks.
-__host__ __device__ inline size_t counted_chunks(uint32_t parts) { return (parts + kChunkParts - 1) / kChunkParts; }
-__host__ __device__ inline size_t counted_work_words(uint32_t parts) {
-    const size_t c = counted_chunks(parts);
-    return 256 * (size_t(parts) + c) + c + 1;
-}
-
-__device__ __forceinline__ uint32_t ld_cg_u32(const uint32_t* p) { return __ldcg(p); }
-
-// Rows of the chunk's partitions [first, first + csize) -> offsets within the
-// chunk, in place, and the chunk's total per digit into chunk_rows (thread =
-// digit; the rows are loaded together, then scanned).
-__device__ __forceinline__ void scan_chunk_rows(uint32_t* rows, uint32_t* chunk_rows, uint32_t chunk, uint32_t first,
-                                                uint32_t csize, uint32_t tid) {
-    uint32_t c[kChunkParts];
-#pragma unroll
-    for (uint32_t q = 0; q < kChunkParts; ++q)
-        c[q] = q < csize ? ld_cg_u32(rows + size_t(first + q) * 256 + tid) : 0u;
-    uint32_t run = 0;
-#pragma unroll
-    for (uint32_t q = 0; q < kChunkParts; ++q) {
-        if (q < csize) rows[size_t(first + q) * 256 + tid] = run;
-        run += c[q];
-    }
-    chunk_rows[size_t(chunk) * 256 + tid] = run;
-}
-
-// The last chunk: each chunk's total -> its base, from the pass's global digit
-// offsets (the exclusive scan of hist_digit over digits). Called by the whole CTA.
-__device__ __forceinline__ void scan_chunk_bases(uint32_t* chunk_rows, uint32_t nchunks, uint32_t hist_digit,
-                                                 uint32_t* wsum, uint32_t tid) {
-    uint32_t gbase = block_exclusive_scan256<8>(hist_digit, wsum);
-    uint32_t c[kChunkParts];
-    for (uint32_t c0 = 0; c0 < nchunks; c0 += kChunkParts) {  // chunk totals, kChunkParts at a time
-#pragma unroll
-        for (uint32_t q = 0; q < kChunkParts; ++q)
-            c[q] = c0 + q < nchunks ? ld_cg_u32(chunk_rows + size_t(c0 + q) * 256 + tid) : 0u;
-#pragma unroll
-        for (uint32_t q = 0; q < kChunkParts; ++q) {
-            if (c0 + q < nchunks) chunk_rows[size_t(c0 + q) * 256 + tid] = gbase;
-            gbase += c[q];
-        }
-    }
-}
-
 template <int kItems, typename KeyT>
 __global__ void __launch_bounds__(256) partition_count_kernel(const KeyT* __restrict__ keys, uint32_t capacity,
-                                                              uint32_t pass, uint32_t shift, uint32_t bits,
-                                                              const uint32_t (*hist)[256], uint32_t fixed_count,
+                                                              uint32_t shift, uint32_t bits, uint32_t fixed_count,
                                                               uint32_t max_parts, uint32_t* __restrict__ work,
                                                               FrameCtl* ctl, uint32_t abort_mask) {
     constexpr uint32_t kTile = 256 * kItems;
@@ -591,80 +522,7 @@ __global__ void __launch_bounds__(256) partition_count_kernel(const KeyT* __rest
     uint32_t total = 0;
 #pragma unroll
     for (uint32_t w = 0; w < 8; ++w) total += hw[w][tid];
-    uint32_t* rows = work;
-    const uint32_t nchunks = uint32_t(counted_chunks(nparts));
-    uint32_t* chunk_rows = work + 256 * size_t(max_parts);
-    uint32_t* arrivals = chunk_rows + 256 * counted_chunks(max_parts);
-    rows[size_t(part) * 256 + tid] = total;
-    // the CTA's row is visible device-wide before its arrival is counted: the
-    // barrier orders every thread's store before thread 0's fence, which
-    // makes them visible with its own (a fence is cumulative); the last
-    // arriver's fence after its count orders its reads after all rows
-    __syncthreads();
-    const uint32_t chunk = part / kChunkParts;
-    const uint32_t first = chunk * kChunkParts, csize = min(kChunkParts, nparts - first);
-    if (tid == 0) {
-        __threadfence();
-        last = atomicAdd(&arrivals[chunk], 1u) == csize - 1u;
-        if (last) __threadfence();
-    }
-    __syncthreads();
-    if (!last) return;
-    // the chunk's last CTA: offsets within the chunk, in place, and its total
-    scan_chunk_rows(rows, chunk_rows, chunk, first, csize, tid);
-    __syncthreads();
-    if (tid == 0) {
-        arrivals[chunk] = 0;
-        __threadfence();
-        last = atomicAdd(&arrivals[counted_chunks(max_parts)], 1u) == nchunks - 1u;
-        if (last) __threadfence();
-    }
-    __syncthreads();
-    if (!last) return;
-    // the last chunk: each chunk's base, from the pass's global digit offsets
-    scan_chunk_bases(chunk_rows, nchunks, TPD_INBOUNDS(ctl, 19, pass, 8) ? hist[pass][tid] : 0u, wsum, tid);
-    if (tid == 0) arrivals[counted_chunks(max_parts)] = 0;
-}
-
-// The first pass of a sort whose partition rows were counted by the kernel
-// that wrote the keys (keygen_scan_kernel adds each partition's digit counts
-// into rows[] with atomics, on rows that were zero): no keys are read. One
-// CTA per chunk of kChunkParts partitions scans its rows in place and writes
-// the chunk's totals; the last chunk to finish (an arrival count, reset by
-// it) scans the chunk totals into chunk bases, as partition_count_kernel's
-// last arrivers do.
-__global__ void __launch_bounds__(256) chunk_scan_kernel(uint32_t capacity, uint32_t pass,
-                                                         const uint32_t (*hist)[256], uint32_t fixed_count,
-                                                         uint32_t max_parts, uint32_t* __restrict__ work,
-                                                         FrameCtl* ctl, uint32_t abort_mask) {
-    __shared__ uint32_t wsum[8];
-    __shared__ bool last;
-    const uint32_t tid = threadIdx.x;
-    pdl_wait();     // the rows come from the kernel before this one
-    pdl_trigger();  // the scatter may be scheduled; it waits for this grid
-    const uint32_t K = (ctl->status & abort_mask) ? 0u : min(fixed_count ? fixed_count : ctl->total_keys, capacity);
-    const uint32_t nparts = min((K + 4095u) / 4096u, max_parts);
-    const uint32_t nchunks = uint32_t(counted_chunks(nparts));
-    const uint32_t chunk = blockIdx.x;
-    if (chunk >= nchunks) return;  // (uniform)
-    uint32_t* rows = work;
-    uint32_t* chunk_rows = work + 256 * size_t(max_parts);
-    uint32_t* arrivals = chunk_rows + 256 * counted_chunks(max_parts);
-    const uint32_t first = chunk * kChunkParts, csize = min(kChunkParts, nparts - first);
-    scan_chunk_rows(rows, chunk_rows, chunk, first, csize, tid);
-    // the chunk totals are visible device-wide before the arrival is counted
-    // (barrier, then thread 0's cumulative fence); the last arriver's fence
-    // after its count orders its reads after every chunk's totals
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        last = atomicAdd(&arrivals[counted_chunks(max_parts)], 1u) == nchunks - 1u;
-        if (last) __threadfence();
-    }
-    __syncthreads();
-    if (!last) return;
-    scan_chunk_bases(chunk_rows, nchunks, TPD_INBOUNDS(ctl, 19, pass, 8) ? hist[pass][tid] : 0u, wsum, tid);
-    if (tid == 0) arrivals[counted_chunks(max_parts)] = 0;
+    counted_finish(CountedWork(work, max_parts), nparts, part, total, wsum, last);
 }
 
 // kBits: the pass's digit width (1..8); the lanes with the same digit are
@@ -674,13 +532,17 @@ template <int kItems, int kThreads, int kMinBlocks, int kBits, typename KeyT>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
     scatter_kernel(const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, KeyT* __restrict__ keys_out,
                    uint32_t* __restrict__ vals_out, uint32_t capacity, uint32_t shift, uint32_t bits,
-                   uint32_t fixed_count, uint32_t max_parts, const uint32_t* __restrict__ work, FrameCtl* ctl,
-                   uint32_t* __restrict__ ranges, uint32_t n_tiles, uint32_t abort_mask) {
+                   uint32_t fixed_count, uint32_t max_parts, uint32_t* __restrict__ work, FrameCtl* ctl,
+                   uint32_t* __restrict__ ranges, uint32_t n_tiles, uint32_t abort_mask, bool keys_just_written) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr uint32_t kSortTile = kThreads * kItems, kWarps = kThreads / 32;
     OnesweepSmem<kItems, kThreads, KeyT>& S = *reinterpret_cast<OnesweepSmem<kItems, kThreads, KeyT>*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const bool digit_thread = tid < kRadix;
+    static_assert(kThreads == kRadix, "a thread per digit");
+    // the keys and values come from the kernel before the counting one, so they
+    // are loaded while that one finishes; or (keys_just_written) from the
+    // kernel right before this one, which counted them as it wrote them
+    if (keys_just_written) pdl_wait();
     const uint32_t K = (ctl->status & abort_mask) ? 0u : min(fixed_count ? fixed_count : ctl->total_keys, capacity);
     const uint32_t nparts = min((K + kSortTile - 1) / kSortTile, max_parts);
     const uint32_t part = blockIdx.x;
@@ -704,17 +566,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
                 vr[i] = 0u;
             }
         }
-        // this partition's digit offsets: chunk base + offset within the chunk,
-        // written by the counting kernel (this kernel may have started while it
-        // ran: its keys and values come from the kernel before that one)
+        // this partition's digit offsets, written by the counting kernel (this
+        // kernel may have started while it ran)
         pdl_wait();
         pdl_trigger();  // the next kernel (the next counting kernel, or the blend) may be scheduled; it waits for this grid
-        uint32_t goff = 0;
-        if (digit_thread) {
-            const uint32_t* chunk_rows = work + 256 * size_t(max_parts);
-            goff = ld_cg_u32(chunk_rows + size_t(part / kChunkParts) * 256 + tid) +
-                   ld_cg_u32(work + size_t(part) * 256 + tid);
-        }
+        const uint32_t goff = counted_offset(CountedWork(work, max_parts), nparts, part, S.wsum);
 #pragma unroll
         for (uint32_t i = tid; i < kWarps * kRadix; i += kThreads) (&S.whist[0][0])[i] = 0;
         __syncthreads();
@@ -749,19 +605,15 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
         }
         __syncthreads();
         uint32_t count = 0;
-        if (digit_thread) {
 #pragma unroll
-            for (uint32_t w = 0; w < kWarps; ++w) {
-                const uint32_t c = S.whist[w][tid];
-                S.whist[w][tid] = count;
-                count += c;
-            }
+        for (uint32_t w = 0; w < kWarps; ++w) {
+            const uint32_t c = S.whist[w][tid];
+            S.whist[w][tid] = count;
+            count += c;
         }
-        const uint32_t lstart = block_exclusive_scan256<kWarps>(count, S.wsum);  // (its barriers cover whist)
-        if (digit_thread) {
-            S.lstart[tid] = lstart;
-            S.gmap[tid] = goff - lstart;
-        }
+        const uint32_t lstart = block_exclusive_scan<kWarps>(count, S.wsum);  // (its barriers cover whist)
+        S.lstart[tid] = lstart;
+        S.gmap[tid] = goff - lstart;
         __syncthreads();
 #pragma unroll
         for (uint32_t i = 0; i < kItems; ++i) {
@@ -863,15 +715,15 @@ int scatter_setup() {
 
 // Counted passes (see partition_count_kernel): per pass a counting launch and
 // a scatter launch, one CTA per 4096-key partition each. work: the counted
-// work area (counted_work_words(max partitions) u32, zero at rest).
+// work area (counted_work_words(max partitions) u32, its arrival counts zero at rest).
 template <int kItems, int kThreads, int kMinBlocks, int kBits, typename KeyT>
 void launch_scatter(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout, uint32_t capacity, uint32_t shift,
                     uint32_t bits, const SortPlan& plan, uint32_t max_parts, uint32_t* work, FrameCtl* ctl,
-                    uint32_t* ranges, uint32_t abort, cudaStream_t s) {
+                    uint32_t* ranges, uint32_t abort, bool keys_just_written, cudaStream_t s) {
     device_once(scatter_setup<kItems, kThreads, kMinBlocks, kBits, KeyT>);
     launch_dependent(scatter_kernel<kItems, kThreads, kMinBlocks, kBits, KeyT>, dim3(max_parts), dim3(kThreads),
                      sizeof(OnesweepSmem<kItems, kThreads, KeyT>), s, kin, vin, kout, vout, capacity, shift, bits,
-                     plan.fixed_count, max_parts, work, ctl, ranges, plan.n_tiles, abort);
+                     plan.fixed_count, max_parts, work, ctl, ranges, plan.n_tiles, abort, keys_just_written);
 }
 
 // The scatter of one pass of `bits` bits: ballots for exactly that width (the
@@ -879,10 +731,10 @@ void launch_scatter(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout, uint32
 template <int kItems, int kThreads, int kMinBlocks, typename KeyT>
 void launch_scatter_bits(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout, uint32_t capacity, uint32_t shift,
                          uint32_t bits, const SortPlan& plan, uint32_t max_parts, uint32_t* work, FrameCtl* ctl,
-                         uint32_t* ranges, uint32_t abort, cudaStream_t s) {
+                         uint32_t* ranges, uint32_t abort, bool keys_just_written, cudaStream_t s) {
 #define TPD_SCATTER(R) \
     launch_scatter<kItems, kThreads, kMinBlocks, R, KeyT>(kin, vin, kout, vout, capacity, shift, bits, plan, \
-                                                          max_parts, work, ctl, ranges, abort, s)
+                                                          max_parts, work, ctl, ranges, abort, keys_just_written, s)
     if constexpr (kMinBlocks != 3) {
         TPD_SCATTER(8);
     } else {
@@ -902,28 +754,23 @@ void launch_scatter_bits(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout, u
 
 // Counted passes (see partition_count_kernel): per pass a counting launch and
 // a scatter launch, one CTA per 4096-key partition each. work: the counted
-// work area (counted_work_words(max partitions) u32, zero at rest).
+// work area (counted_work_words(max partitions) u32, its arrival counts zero at rest).
 template <int kItems, int kThreads, int kMinBlocks, typename KeyT>
 void launch_counted_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout, uint32_t capacity, uint32_t p0,
-                           uint32_t p1, const SortPlan& plan, uint32_t (*hist)[256], uint32_t* work, FrameCtl* ctl,
-                           cudaStream_t s) {
+                           uint32_t p1, const SortPlan& plan, uint32_t* work, FrameCtl* ctl, cudaStream_t s) {
     static_assert(kThreads * kItems == 4096, "counted passes use 4096-key partitions");
     const uint32_t max_parts = std::max(1u, (capacity + 4095u) / 4096u);
     const uint32_t abort = kStatusFatal | (plan.skip_on_overflow ? kStatusKeyOverflow : 0u);
     for (uint32_t p = p0; p < p1; ++p) {
         const uint32_t shift = p * kRadixBits;
         const uint32_t bits = std::min(kRadixBits, plan.key_bits - shift);
-        if (p == p0 && plan.precounted)
-            launch_dependent(chunk_scan_kernel, dim3(uint32_t(counted_chunks(max_parts))), dim3(256), 0, s, capacity,
-                             p, static_cast<const uint32_t(*)[256]>(hist), plan.fixed_count, max_parts, work, ctl,
-                             abort);
-        else
-            launch_dependent(partition_count_kernel<16, KeyT>, dim3(max_parts), dim3(256), 0, s, kin, capacity, p,
-                             shift, bits, static_cast<const uint32_t(*)[256]>(hist), plan.fixed_count, max_parts,
-                             work, ctl, abort);
+        const bool counted = p == p0 && plan.precounted;
+        if (!counted)
+            launch_dependent(partition_count_kernel<16, KeyT>, dim3(max_parts), dim3(256), 0, s, kin, capacity, shift,
+                             bits, plan.fixed_count, max_parts, work, ctl, abort);
         launch_scatter_bits<kItems, kThreads, kMinBlocks, KeyT>(kin, vin, kout, vout, capacity, shift, bits, plan,
                                                                 max_parts, work, ctl,
-                                                                p + 1 == p1 ? plan.ranges : nullptr, abort, s);
+                                                                p + 1 == p1 ? plan.ranges : nullptr, abort, counted, s);
         std::swap(kin, kout);
         std::swap(vin, vout);
     }
@@ -963,10 +810,10 @@ bool launch_sort_t(KeyT* keys, uint32_t* vals, KeyT* keys_alt, uint32_t* vals_al
     if constexpr (sizeof(KeyT) == 4) {  // counted passes: 32-bit keys (for 64-bit keys onesweep is faster)
         if (plan.counted_work) {
             if (plan.ctas_per_sm == 2)
-                launch_counted_passes<16, 256, 2>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan, hist,
+                launch_counted_passes<16, 256, 2>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan,
                                                   plan.counted_work, ctl, s);
             else
-                launch_counted_passes<16, 256, 3>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan, hist,
+                launch_counted_passes<16, 256, 3>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan,
                                                   plan.counted_work, ctl, s);
             return ((p1 - p0) & 1u) != 0;
         }

@@ -59,14 +59,7 @@ struct PreprocessArgs {
     uint64_t* depth_keys;
     uint32_t* depth_items;
     uint32_t depth_key_bits;  // 32 + bits of (n_views - 1); its digit histograms go to ctl->depth_hist
-    // > 0: the 8-bit digit counts of the frame's tile ids (all keys the
-    // visible items will emit, tile ids below 2^tile_bits) go to ctl->sort_hist[0..]
-    uint32_t tile_bits;
     FrameCtl* ctl;
-    // words set to zero after the kernel's dependency wait (nullptr: none):
-    // the key sort's precounted rows, for keygen's counts
-    uint32_t* zero_words;
-    uint64_t zero_count;
 };
 
 constexpr uint32_t kMaxViews = 256;
@@ -90,31 +83,47 @@ void launch_preprocess(const PreprocessArgs& a, int num_sms, cudaStream_t s);
 void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint64_t* desc, FrameCtl* ctl,
                        uint32_t spin_limit, uint32_t never_publish, cudaStream_t s);
 
-// Items (view, Gaussian) in depth order per partition of the fused scan and
-// key duplication: its look-back descriptors number n_items / kKeygenPart + 2.
-constexpr uint32_t kKeygenPart = 512;
+// Items (view, Gaussian) in depth order per partition of the depth-order
+// scan: its look-back descriptors number n_items / kKeygenPart + 2.
+constexpr uint32_t kKeygenPart = 1024;
 
 // The tile counts of the ctl->depth_count (view, Gaussian) items in depth
 // order (items[r] = v * n + i < n_items) scanned into exclusive key offsets
-// offsets[r] (prefix.slang), fused with keygen.slang's key duplication: keys
+// offsets[r] (prefix.slang), then keygen.slang's key duplication: keys
 // (tile_base + tile) << 32 | bits(viewZ) with vals = Gaussian index. The
 // items come in depth order, so only the tile id of each key is written
 // (tiles[], u32): the depth half of a key is the depth of its value's splat
 // (launch_materialize_keys). K goes to ctl->total_keys and the non-empty
-// count to ctl->visible; keys beyond capacity are dropped and flag the frame
-// (kStatusKeyOverflow). Also presets ranges (2 x n_tiles u32) to
-// (0xFFFFFFFF, 0) for the key sort's last pass. The digit counts of the tile
-// ids come from the preprocess (tile_bits).
-// items: where the depth sort leaves the order with no pass skipped;
-// items_other: the other buffer, which holds it when ctl->depth_skips is odd.
-// desc: look-back descriptors (tag ctl->tag * 32 + kTagScan), never cleared.
-// count_rows (or nullptr): the key sort's first counted pass's partition
-// rows, zero on entry (PreprocessArgs.zero_words): each written key adds one
-// to count_rows[256 * (slot / 4096) + (tile & 255)] (SortPlan.precounted).
-void launch_keygen_scan(const Splat* splats, const uint32_t* items, const uint32_t* items_other, uint32_t n_items,
-                        uint32_t n, const ViewConst* views, uint32_t* offsets, uint32_t* tiles, uint32_t* vals,
-                        uint32_t capacity, uint32_t* ranges, uint32_t n_tiles, uint64_t* desc, uint32_t* count_rows,
-                        FrameCtl* ctl, uint32_t spin_limit, uint32_t never_publish, int num_sms, cudaStream_t s);
+// count to ctl->visible; more keys than the capacity flag the frame
+// (kStatusKeyOverflow) and none are written. Also presets ranges (2 x n_tiles
+// u32) to (0xFFFFFFFF, 0) for the key sort's last pass.
+struct KeygenArgs {
+    const Splat* splats;
+    const uint32_t* items;        // where the depth sort leaves the order with no pass skipped
+    const uint32_t* items_other;  // the other buffer, which holds it when ctl->depth_skips is odd
+    uint32_t n_items;             // views x n
+    uint32_t n;                   // Gaussians per view
+    const ViewConst* views;
+    uint32_t* offsets;            // n_items
+    uint2* item_rects;            // n_items: scratch between the two kernels
+    uint2* item_slots;            // n_items: scratch between the two kernels
+    uint32_t* part_first;         // ceil(capacity / 4096): scratch between the two kernels
+    uint32_t* tiles;              // capacity
+    uint32_t* vals;               // capacity
+    uint32_t capacity;
+    uint32_t* ranges;
+    uint32_t n_tiles;
+    uint32_t tile_bits;           // tile ids are below 2^tile_bits
+    uint64_t* desc;               // look-back descriptors (tag ctl->tag * 32 + kTagScan), never cleared
+    // the key sort's counted work area: the first pass is counted and its
+    // offsets are ready afterwards (SortPlan.precounted); nullptr: the digit
+    // counts of the tile ids go to ctl->sort_hist instead
+    uint32_t* counted_work;
+    FrameCtl* ctl;
+    uint32_t spin_limit;
+    uint32_t never_publish;
+};
+void launch_keygen(const KeygenArgs& a, int num_sms, cudaStream_t s);
 
 // keys[i] = tiles[i] << 32 | bits(viewZ of splat vals[i] in the tile's view),
 // i < min(ctl->total_keys, capacity): the 64-bit (tile | depth) keys of a
@@ -145,8 +154,8 @@ struct SortPlan {
     uint32_t* ranges = nullptr;        // key sort: the last pass also writes the tile ranges (preset by keygen)
     uint32_t n_tiles = 0;
     uint32_t fixed_count = 0;          // nonzero: sort this many pairs, else min(ctl->total_keys, capacity)
-    // a frame whose keys overflowed the capacity (its histograms count keys
-    // that were not written) sorts nothing; it is rendered again
+    // a frame whose keys overflowed the capacity sorts nothing (none were
+    // written); it is rendered again
     bool skip_on_overflow = false;
     // depth sort: the first pass drops the keys whose low 32 bits are
     // 0xFFFFFFFF (culled items) and keeps ctl->depth_count, which the later
@@ -155,14 +164,12 @@ struct SortPlan {
     cudaEvent_t after_hist = nullptr;  // recorded between the histogram and the first pass
     // non-null, 32-bit keys: counted passes (every partition's digit offsets
     // counted and scanned beforehand, no look-back; plain pass kinds only) using this work
-    // area of sort_counted_work_words(capacity) u32, zero at rest (every
-    // launch leaves it so)
+    // area of sort_counted_work_words(capacity) u32, zeroed once (every launch
+    // leaves its arrival counts at zero)
     uint32_t* counted_work = nullptr;
-    // counted passes: the first pass's partition rows (the first
-    // 256 x ceil(capacity / 4096) words of counted_work) already hold every
-    // 4096-key partition's digit counts, added by the kernel that wrote the
-    // keys onto rows that were zero (launch_keygen_scan with count_rows); the
-    // pass only scans them
+    // counted passes: the first pass's digit offsets are already in
+    // counted_work, put there by the kernel that wrote the keys right before
+    // this sort (launch_keygen)
     bool precounted = false;
 };
 size_t sort_counted_work_words(uint32_t capacity);
