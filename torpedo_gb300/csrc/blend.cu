@@ -399,64 +399,174 @@ __global__ void pack_rgba8_kernel(const float* rgb, uint32_t* rgba, size_t pixel
     rgba[i] = rgba8_unorm(rgb[i * 3 + 0], rgb[i * 3 + 1], rgb[i * 3 + 2]);
 }
 
-constexpr int kG2D = 9;  // px, py, conic.x, conic.y, conic.z, opacity, r, g, b
-
-// Sums v[0..7] over the warp with a transposed butterfly: each of the first
-// three exchanges halves the values a lane holds, the last two add single
-// values. Afterwards lane 4j holds the warp sum of v[j] (j = 0..7).
-__device__ __forceinline__ float warp_sum8_transposed(const float (&v)[8], uint32_t lane) {
-    float a[4], b[2], c;
-    const bool u4 = (lane >> 4) & 1u, u3 = (lane >> 3) & 1u, u2 = (lane >> 2) & 1u;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float send = u4 ? v[i] : v[i + 4];
-        const float keep = u4 ? v[i + 4] : v[i];
-        a[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 16);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float send = u3 ? a[i] : a[i + 2];
-        const float keep = u3 ? a[i + 2] : a[i];
-        b[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 8);
-    }
-    {
-        const float send = u2 ? b[0] : b[1];
-        const float keep = u2 ? b[1] : b[0];
-        c = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 4);
-    }
-    c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
-    c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
-    return c;
-}
-
-// The adjoint, with the forward's layout: a CTA of 128 threads per tile,
-// warp w on the 8x8 block at (8 (w & 1), 8 (w >> 1)), lane l on pixels
-// (l & 7, l >> 3) and (l & 7, (l >> 3) + 4), pair arithmetic packed in f32x2.
-// Rounds of kBwdRound list entries from the back: staging double-buffered,
-// per-round gradient sums in one of two shared buffers. The barrier at the
-// end of a round completes its sums; each thread then adds its share of them
-// to global memory and zeroes what it added, so the buffer is clean when it
-// comes round again two rounds later. The staged indices that the flush
-// reads live in three buffers (the next round's staging overwrites the one of
-// the round before the last).
+// ---- adjoint
+//
+// A CTA of 64 threads per tile. The tile is eight blocks of 8x4 pixels (block
+// 2k + c: rows 4k .. 4k + 3, columns 8c .. 8c + 7); eight lanes own a block,
+// one pixel column of four rows each, so warp w holds blocks 4w .. 4w + 3.
+// Every block walks its own list of the entries that reach it (from the back:
+// slot k of a round holds its k-th entry from the end): a warp's step takes
+// one entry per block, and the four entries usually differ. The pixels of a
+// lane share dx, and their arithmetic runs two rows at a time in packed f32x2
+// operations, per pixel with the forward's operations, order and rounding for
+// p2, alpha and the tests. A staged entry holds the values that the packed
+// operations take duplicated in register-pair order.
+//
+// Per pixel, with g = dL/dimage, and going from the back: T after an entry
+// gives T / (1 - alpha) in front of it, w = alpha T_front is its weight, and
+// A, the colours behind it blended with each other and dotted with g, follows
+// A <- A + alpha (g.c - A); then dL/dalpha = T_front (g.c - A). A skipped pair
+// has alpha = 0, which leaves T and A as they are (1 / (1 - 0) is exactly 1).
+//
+// Sums per (block, entry). With P = dL/dpower (power = p2 ln2) the record's
+// gradients follow from nine sums over pixels: P, P dx, P dy, P dx^2, P dx dy,
+// P dy^2 and w g (three). A lane's four pixels share dx, so it adds P, P dy
+// and P dy^2 over them first and multiplies by dx afterwards; eight of the
+// nine are then summed over the block's eight lanes by a transposed butterfly
+// (seven exchanges, lane j ends with sum j), the ninth by three more. A block
+// meets an entry once per round, so the sums are stored, not added: no
+// shared-memory atomics. At the end of the round one thread per entry adds
+// the blocks' sums (those whose bit is set), turns them into gradients with
+// the entry's conic, and adds them to the global record with vector atomics.
+//
+// Against one 8x8 block per warp with two pixels a lane and the nine gradients
+// of every pixel pair summed by shuffles and shared-memory atomics: 104M
+// instead of 185M warp instructions for 200,000 Gaussians at 800x800, 234 ->
+// 150 us; 8 views of 500,000 at 1280x720 1856 -> 1198 us; 5,003 at 201x151 90
+// -> 59 us; 8 views of 6M at 2160p 20.5 -> 13.5 ms. It issues on 54% of the
+// cycles (16 warps per SM, by its registers and the blocks' sums; rounds of 32
+// with 20 warps measured 3% slower, rounds of 128 with 8 warps 38%), ALU and
+// FMA pipes at 47% and 41%; the last tiles leave 15% of the SM time idle.
+// The forward gains nothing from this layout (249 us at 1M Gaussians and
+// 1080p either way, and a mid-sized frame's longest tile takes 94 us on two
+// warps instead of 72 on four), so it keeps one 8x8 block per warp.
 //
 // List entries per round (an engine setting the autotuner picks): 64 by
-// default (17 KB of shared memory, 8 CTAs per SM at 64 registers); 32 (8 CTAs)
-// or 128 (35 KB, 6 CTAs).
+// default, 32 or 128.
+constexpr uint32_t kAdjThreads = 64;
+constexpr uint32_t kBlendBlocks = 8;  // 8x4 blocks of a tile
+
+struct BlockStaged {  // 80 bytes
+    float4 s;         // x, qa, thr, 0
+    float4 yb;        // y, y, qb, qb
+    float4 qco;       // qc, qc, opacity, opacity
+    float4 rg;        // r, r, g, g
+    float2 b;         // b, b
+    float2 pad;
+};
+
+__device__ __forceinline__ void stage_block_values(float4 c, float4 tex, float4 co, float ox, float oy, BlockStaged& d,
+                                                   uint8_t& mask) {
+    const float thr = co.w > 0.0f ? -__log2f(255.0f * co.w) : kInf;  // +inf: never blends
+    const float4 q = make_float4(-0.5f * kLog2e * co.x, -kLog2e * co.y, -0.5f * kLog2e * co.z, thr);
+    d.s = make_float4(tex.x, q.x, thr, 0.0f);
+    d.yb = make_float4(tex.y, tex.y, q.y, q.y);
+    d.qco = make_float4(q.z, q.z, co.w, co.w);
+    d.rg = make_float4(c.x, c.x, c.y, c.y);
+    d.b = make_float2(c.z, c.z);
+    mask = uint8_t(block_mask<4>(tex.x, tex.y, q, ox, oy));
+}
+
+__device__ __forceinline__ void stage_block_empty(BlockStaged& d) {
+    d.s = make_float4(0.f, 0.f, kInf, 0.f);
+    d.yb = d.qco = d.rg = make_float4(0.f, 0.f, 0.f, 0.f);
+    d.b = make_float2(0.f, 0.f);
+}
+
+// Entries of a round for each block of a warp, in list order (BlockLists).
+template <uint32_t kRound>
+struct BlockLists {
+    static constexpr uint32_t kEmpty = kRound;  // the staged slot that never blends
+    uint16_t e[kBlendBlocks][kRound + 2];
+};
+
+// The lists of the calling warp's four blocks for a round of n entries:
+// `nibble(e)` gives entry e's bits for them (called for e < n). Returns the
+// steps of the walk, a multiple of two: the longest list's length, to which
+// the shorter ones are filled up with the empty slot.
+template <uint32_t kRound, typename Nibble>
+__device__ __forceinline__ uint32_t build_block_lists(BlockLists<kRound>& L, uint32_t warp, uint32_t lane, uint32_t n,
+                                                      Nibble nibble) {
+    uint32_t cnt[4] = {0u, 0u, 0u, 0u};
+    const uint32_t lt = (1u << lane) - 1u;
+    for (uint32_t c = 0; c < n; c += 32u) {
+        const uint32_t e = c + lane;
+        const uint32_t m = e < n ? nibble(e) : 0u;
+#pragma unroll
+        for (uint32_t g = 0; g < 4; ++g) {
+            const bool on = (m >> g) & 1u;
+            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
+            if (on) L.e[4 * warp + g][cnt[g] + __popc(bal & lt)] = uint16_t(e);
+            cnt[g] += __popc(bal);
+        }
+    }
+    const uint32_t steps = (max(max(cnt[0], cnt[1]), max(cnt[2], cnt[3])) + 1u) & ~1u;
+    const uint32_t g = lane >> 3;
+    const uint32_t mine = g == 0 ? cnt[0] : g == 1 ? cnt[1] : g == 2 ? cnt[2] : cnt[3];
+    for (uint32_t i = mine + (lane & 7u); i < steps; i += 8u) L.e[4 * warp + g][i] = uint16_t(L.kEmpty);
+    __syncwarp();
+    return steps;
+}
+
+// A lane's four pixels: the column and rows, in packed order.
+struct LanePixels {
+    uint32_t x, y;       // the first row's pixel
+    float nx;            // -x
+    float2 ny0, ny1;     // -(y, y + 1), -(y + 2, y + 3)
+    bool in[4];
+    __device__ __forceinline__ LanePixels(uint32_t tx, uint32_t ty, uint32_t warp, uint32_t lane, uint32_t W,
+                                          uint32_t H) {
+        const uint32_t block = 4u * warp + (lane >> 3);
+        x = tx * kBlockX + 8u * (block & 1u) + (lane & 7u);
+        y = ty * kBlockY + 4u * (block >> 1);
+        nx = -float(x);
+        ny0 = make_float2(-float(y), -float(y + 1u));
+        ny1 = make_float2(-float(y + 2u), -float(y + 3u));
+#pragma unroll
+        for (uint32_t r = 0; r < 4; ++r) in[r] = x < W && y + r < H;
+    }
+};
+
 template <uint32_t kBwdRound>
-constexpr int bwd_min_blocks() { return kBwdRound >= 128 ? 6 : 8; }
+constexpr int bwd_min_blocks() { return kBwdRound >= 128 ? 4 : kBwdRound >= 64 ? 8 : 10; }
 template <uint32_t kBwdRound>
 struct BlendBackwardSmem {
-    PairStaged e[2][kBwdRound];
-    uint8_t mask[2][kBwdRound];
-    float acc[2][kBwdRound][kG2DStride];
-    uint32_t idx[3][kBwdRound];
-    uint32_t wmax[kFwdThreads / 32];
+    BlockStaged e[kBwdRound + 1];                     // slot kBwdRound: an entry that never blends
+    float sums[kBlendBlocks][(kBwdRound + 1) * 8];   // eight per (block, entry); a row's length sets blocks 8 banks apart
+    float sum9[kBlendBlocks][kBwdRound + 1];
+    BlockLists<kBwdRound> lists;
+    uint32_t idx[kBwdRound];
+    uint32_t wmax[kAdjThreads / 32];
+    uint8_t mask[kBwdRound];
+    uint8_t met[kAdjThreads / 32][kBwdRound];  // blocks of the warp that have sums of the entry
 };
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ float hsum(float2 a) { return a.x + a.y; }
 
-// One tile of the adjoint (the whole CTA; barriers as in blend_tile).
+// Sums v[0..7] over each group of eight lanes with a transposed butterfly:
+// each exchange halves the values a lane holds. Lane j of a group returns the
+// sum of v[j].
+__device__ __forceinline__ float group_sum8_transposed(const float (&v)[8], uint32_t lane) {
+    float a[4], b[2];
+    const bool u2 = (lane >> 2) & 1u, u1 = (lane >> 1) & 1u, u0 = lane & 1u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float send = u2 ? v[i] : v[i + 4], keep = u2 ? v[i + 4] : v[i];
+        a[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 4);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float send = u1 ? a[i] : a[i + 2], keep = u1 ? a[i + 2] : a[i];
+        b[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, 2);
+    }
+    const float send = u0 ? b[0] : b[1], keep = u0 ? b[1] : b[0];
+    return keep + __shfl_xor_sync(0xFFFFFFFFu, send, 1);
+}
+
+// One tile of the adjoint (the whole CTA). Two barriers per round: after the
+// walk (the blocks' sums are complete) and after the flush, which also stages
+// the next round's entries in place of this one's.
 template <uint32_t kBwdRound>
 __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, uint32_t tile,
                                                     BlendBackwardSmem<kBwdRound>& SM) {
@@ -464,194 +574,191 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
     uint32_t vi, W, H, tx, ty;
     load_view_tile(a.views, a.tile_view, tile, vi, W, H, tx, ty);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t px = tx * kBlockX + 8u * (warp & 1u) + (lane & 7u);
-    const uint32_t pya = ty * kBlockY + 8u * (warp >> 1) + (lane >> 3), pyb = pya + 4u;
+    const LanePixels P(tx, ty, warp, lane, W, H);
     const float ox = float(tx * kBlockX), oy = float(ty * kBlockY);
-    const bool in_a = px < W && pya < H, in_b = px < W && pyb < H;
-    const float2 npx = f2(-float(px), -float(px));
-    const float2 npy = f2(-float(pya), -float(pyb));
     const uint32_t K = min(a.ctl->total_keys, a.capacity);
     const uint32_t end = min(a.ranges[tile * 2 + 1], K), start = min(a.ranges[tile * 2 + 0], end);
     const Splat* vsplats = a.splats + size_t(vi) * a.n;
 
     const size_t img0 = a.image_offset ? a.image_offset[vi] : 0ull;
-    const size_t pa = img0 + size_t(pya) * W + px, pb = img0 + size_t(pyb) * W + px;
-    float2 T = f2(1.0f, 1.0f), g0 = f2(0.f, 0.f), g1 = g0, g2 = g0;
-    uint32_t last_a = 0, last_b = 0;
-    if (in_a) {
-        T.x = a.final_T[pa];
-        last_a = min(a.n_contrib[pa], end - start);
-        g0.x = a.dL_dimage[pa * 3 + 0];
-        g1.x = a.dL_dimage[pa * 3 + 1];
-        g2.x = a.dL_dimage[pa * 3 + 2];
-    }
-    if (in_b) {
-        T.y = a.final_T[pb];
-        last_b = min(a.n_contrib[pb], end - start);
-        g0.y = a.dL_dimage[pb * 3 + 0];
-        g1.y = a.dL_dimage[pb * 3 + 1];
-        g2.y = a.dL_dimage[pb * 3 + 2];
-    }
-    // the block walks back from the largest last-contributor index over its
-    // pixels; a warp takes entries below its own largest index only
-    uint32_t warp_last = max(last_a, last_b);
+    float Tp[4], gp[3][4];
+    uint32_t last[4], blk_last = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) warp_last = max(warp_last, __shfl_xor_sync(0xFFFFFFFFu, warp_last, o));
-    if (lane == 0) SM.wmax[warp] = warp_last;
-    for (uint32_t k = tid; k < 2 * kBwdRound * kG2DStride; k += kFwdThreads) (&SM.acc[0][0][0])[k] = 0.f;
+    for (uint32_t q = 0; q < 4; ++q) {
+        Tp[q] = 1.0f;
+        gp[0][q] = gp[1][q] = gp[2][q] = 0.0f;
+        last[q] = 0;
+        if (P.in[q]) {
+            const size_t p = img0 + size_t(P.y + q) * W + P.x;
+            Tp[q] = a.final_T[p];
+            last[q] = min(a.n_contrib[p], end - start);
+#pragma unroll
+            for (uint32_t c = 0; c < 3; ++c) gp[c][q] = a.dL_dimage[p * 3 + c];
+        }
+        blk_last = max(blk_last, last[q]);
+    }
+    float2 T[2], nA[2], g0[2], g1[2], g2[2];
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+        T[h] = f2(Tp[2 * h], Tp[2 * h + 1]);
+        nA[h] = f2(0.f, 0.f);  // -A
+        g0[h] = f2(gp[0][2 * h], gp[0][2 * h + 1]);
+        g1[h] = f2(gp[1][2 * h], gp[1][2 * h + 1]);
+        g2[h] = f2(gp[2][2 * h], gp[2][2 * h + 1]);
+    }
+    // a block takes the entries below the largest last-contributor index over
+    // its pixels; the tile is walked back from the largest of all
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) blk_last = max(blk_last, __shfl_xor_sync(0xFFFFFFFFu, blk_last, o));
+    uint32_t bl[4];
+#pragma unroll
+    for (uint32_t g = 0; g < 4; ++g) bl[g] = __shfl_sync(0xFFFFFFFFu, blk_last, 8 * g);
+    if (lane == 0) SM.wmax[warp] = max(max(bl[0], bl[1]), max(bl[2], bl[3]));
+    if (tid == 0) stage_block_empty(SM.e[kBwdRound]);
     __syncthreads();
-    uint32_t max_last = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kFwdThreads / 32; ++w) max_last = max(max_last, SM.wmax[w]);
-
-    float2 S0 = f2(0.f, 0.f), S1 = S0, S2 = S0;  // colour accumulated behind the current entry
+    const uint32_t max_last = max(SM.wmax[0], SM.wmax[1]);
     float* g2d_view = a.g2d + size_t(vi) * a.g2d_view_stride;
-    // stages the round whose list positions (relative) end at r_end: slot k
-    // holds position r_end - 1 - k
-    auto stage_round = [&](int32_t r_end, uint32_t b, uint32_t bi) {
-        const uint32_t n = uint32_t(min(int32_t(kBwdRound), r_end));
-        for (uint32_t k = tid; k < n; k += kFwdThreads) {
-            const uint32_t e = uint32_t(r_end) - 1u - k;
-            uint32_t idx = a.vals[start + e];
-            if (idx < a.n) {
-                stage_pair_entry(vsplats + idx, ox, oy, SM.e[b][k], SM.mask[b][k]);
-            } else {  // only reachable with corrupted lists
-                idx = 0;
-                stage_pair_empty(SM.e[b][k], SM.mask[b][k]);
-            }
-            SM.idx[bi][k] = idx;
-        }
-    };
-    if (max_last > 0) stage_round(int32_t(max_last), 0, 0);
-    __syncthreads();
-    // the next round's entry of this thread (one per thread: kBwdRound <=
-    // kFwdThreads), loaded before the current round is walked and staged after
-    // it, so the gathers' latency hides behind the walk
-    static_assert(kBwdRound <= kFwdThreads, "one staged entry per thread");
-    bool pf = false;
-    uint32_t pf_idx = 0;
-    float4 pf_c = make_float4(0.f, 0.f, 0.f, 0.f), pf_tex = pf_c, pf_co = pf_c;
-    auto load_next = [&](int32_t r_end) {
-        pf = tid < uint32_t(min(int32_t(kBwdRound), r_end));
-        if (!pf) return;
-        pf_idx = a.vals[start + uint32_t(r_end) - 1u - tid];
-        if (pf_idx < a.n) {
-            const float4* p = reinterpret_cast<const float4*>(vsplats + pf_idx);
-            pf_c = __ldg(p + 0);
-            pf_tex = __ldg(p + 1);
-            pf_co = __ldg(p + 2);
-        }
-    };
-    auto store_next = [&](uint32_t b, uint32_t bi) {
-        if (!pf) return;
-        if (pf_idx < a.n) {
-            stage_pair_values(pf_c, pf_tex, pf_co, ox, oy, SM.e[b][tid], SM.mask[b][tid]);
-        } else {  // only reachable with corrupted lists
-            pf_idx = 0;
-            stage_pair_empty(SM.e[b][tid], SM.mask[b][tid]);
-        }
-        SM.idx[bi][tid] = pf_idx;
-    };
-    const float2 one = f2(1.0f, 1.0f), mone = f2(-1.0f, -1.0f), mhalf = f2(-0.5f, -0.5f), ln2 = f2(kLn2, kLn2);
-    uint32_t r = 0;
-    for (int32_t r_end = int32_t(max_last); r_end > 0; r_end -= int32_t(kBwdRound), ++r) {
-        const uint32_t b = r & 1u, bi = r % 3u;
-        const uint32_t n = uint32_t(min(int32_t(kBwdRound), r_end));
-        if (r_end > int32_t(kBwdRound)) load_next(r_end - int32_t(kBwdRound));
-        else pf = false;
-        // entries jj >= skip have list positions r_end - 1 - jj below warp_last
-        const uint32_t skip = uint32_t(r_end) > warp_last ? uint32_t(r_end) - warp_last : 0u;
-        for (uint32_t g = skip & ~31u; g < n; g += 32) {
-            const uint32_t jl = g + lane;
-            uint32_t m = __ballot_sync(0xFFFFFFFFu, jl < n && jl >= skip && ((SM.mask[b][jl] >> warp) & 1u));
-            while (m) {
-                const uint32_t jj = g + uint32_t(__ffs(m) - 1);
-                m &= m - 1u;
-                const uint32_t e = uint32_t(r_end) - 1u - jj;
-                const PairStaged& E = SM.e[b][jj];
-                const float4 xy = E.xy, qab = E.qab, qco = E.qco, rg = E.rg, bt = E.bt;
-                // p2 for both pixels, as in the forward
-                const float2 dx = __fadd2_rn(f2(xy.x, xy.y), npx);
-                const float2 dy = __fadd2_rn(f2(xy.z, xy.w), npy);
-                const float2 qadx = __fmul2_rn(f2(qab.x, qab.y), dx);
-                const float2 t = __ffma2_rn(f2(qab.z, qab.w), dy, qadx);
-                const float2 qcdy = __fmul2_rn(f2(qco.x, qco.y), dy);
-                const float2 p2 = __ffma2_rn(t, dx, __fmul2_rn(qcdy, dy));
-                const bool ca = in_a && e < last_a && !pair_skipped(p2.x, bt.z);
-                const bool cb = in_b && e < last_b && !pair_skipped(p2.y, bt.z);
-                // branch-free body: zero weight and gradient scale for pairs
-                // that do not count; every term below is finite, so they add
-                // exactly nothing
-                const float2 G = f2(ex2_approx(p2.x), ex2_approx(p2.y));
-                const float2 raw = __fmul2_rn(f2(qco.z, qco.w), G);
-                const float2 alpha = f2(fminf(kAlphaMax, raw.x), fminf(kAlphaMax, raw.y));
-                const float2 om = __ffma2_rn(mone, alpha, one);  // 1 - alpha >= 0.01
-                const float2 inv = f2(__fdividef(1.0f, om.x), __fdividef(1.0f, om.y));
-                const float2 Tb = __fmul2_rn(T, inv);  // transmittance in front of this entry
-                const float2 aTb = __fmul2_rn(alpha, Tb);
-                const float2 w = f2(ca ? aTb.x : 0.0f, cb ? aTb.y : 0.0f);
-                // dL/dalpha = sum_c g_c (col_c Tb - S_c / (1 - alpha))
-                const float2 ninv = __fmul2_rn(inv, mone);
-                const float2 d0 = __ffma2_rn(f2(rg.x, rg.y), Tb, __fmul2_rn(S0, ninv));
-                const float2 d1 = __ffma2_rn(f2(rg.z, rg.w), Tb, __fmul2_rn(S1, ninv));
-                const float2 d2 = __ffma2_rn(f2(bt.x, bt.y), Tb, __fmul2_rn(S2, ninv));
-                const float2 dA = __ffma2_rn(g2, d2, __ffma2_rn(g1, d1, __fmul2_rn(g0, d0)));
-                S0 = __ffma2_rn(f2(rg.x, rg.y), w, S0);
-                S1 = __ffma2_rn(f2(rg.z, rg.w), w, S1);
-                S2 = __ffma2_rn(f2(bt.x, bt.y), w, S2);
-                T = f2(ca ? Tb.x : T.x, cb ? Tb.y : T.y);
-                // power = p2 ln2; d power / d(dx, dy) = ln2 (2 qa dx + qb dy, 2 qc dy + qb dx)
-                const bool ua = ca && raw.x <= kAlphaMax, ub = cb && raw.y <= kAlphaMax;
-                const float2 dAa = __fmul2_rn(dA, alpha);
-                const float2 dpow = f2(ua ? dAa.x : 0.0f, ub ? dAa.y : 0.0f);
-                const float2 dpl = __fmul2_rn(dpow, ln2), hdp = __fmul2_rn(dpow, mhalf);
-                const float2 dAG = __fmul2_rn(dA, G);
-                float2 gv[kG2D];
-                gv[0] = __fmul2_rn(dpl, __fadd2_rn(t, qadx));                                  // 2 qa dx + qb dy
-                gv[1] = __fmul2_rn(dpl, __ffma2_rn(f2(qab.z, qab.w), dx, __fadd2_rn(qcdy, qcdy)));  // 2 qc dy + qb dx
-                gv[2] = __fmul2_rn(hdp, __fmul2_rn(dx, dx));
-                gv[3] = __fmul2_rn(__fmul2_rn(dpow, mone), __fmul2_rn(dx, dy));
-                gv[4] = __fmul2_rn(hdp, __fmul2_rn(dy, dy));
-                gv[5] = f2(ua ? dAG.x : 0.0f, ub ? dAG.y : 0.0f);
-                gv[6] = __fmul2_rn(g0, w);
-                gv[7] = __fmul2_rn(g1, w);
-                gv[8] = __fmul2_rn(g2, w);
-                if (__any_sync(0xFFFFFFFFu, ca || cb)) {
-                    // the lane's two pixels first, then the warp
-                    const float lo[8] = {gv[0].x + gv[0].y, gv[1].x + gv[1].y, gv[2].x + gv[2].y, gv[3].x + gv[3].y,
-                                         gv[4].x + gv[4].y, gv[5].x + gv[5].y, gv[6].x + gv[6].y, gv[7].x + gv[7].y};
-                    const float rs = warp_sum8_transposed(lo, lane);
-                    float b9 = gv[8].x + gv[8].y;
+
+    // A round's entries, kPer per thread (with fewer entries than threads the
+    // warps take turns): loaded before the previous round is walked and staged
+    // after it, so the gathers' latency hides behind the walk. Slot k of the
+    // round whose list positions end at r_end holds position r_end - 1 - k.
+    constexpr uint32_t kPer = kBwdRound > kAdjThreads ? kBwdRound / kAdjThreads : 1u;
+    uint32_t pf_idx[kPer];
+    float4 pf_c[kPer], pf_tex[kPer], pf_co[kPer];
+    auto load_round = [&](uint32_t r_end, uint32_t turn) {
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) b9 += __shfl_xor_sync(0xFFFFFFFFu, b9, o);
-                    if ((lane & 3u) == 0) atomicAdd(&SM.acc[b][jj][lane >> 2], rs);
-                    if (lane == 0) atomicAdd(&SM.acc[b][jj][8], b9);
+        for (uint32_t u = 0; u < kPer; ++u) {
+            const uint32_t k = (tid ^ turn) + u * kAdjThreads;
+            pf_idx[u] = 0xFFFFFFFFu;
+            if (k < min(kBwdRound, r_end)) {
+                pf_idx[u] = a.vals[start + r_end - 1u - k];
+                if (pf_idx[u] < a.n) {
+                    const float4* p = reinterpret_cast<const float4*>(vsplats + pf_idx[u]);
+                    pf_c[u] = __ldg(p + 0);
+                    pf_tex[u] = __ldg(p + 1);
+                    pf_co[u] = __ldg(p + 2);
                 }
             }
         }
-        store_next(b ^ 1u, (r + 1) % 3u);
-        __syncthreads();  // round r's sums complete; the other stage buffer is filled
-        // one 16-byte vector atomic per non-zero quarter of an entry's record;
-        // the thread that adds a quarter also zeroes it for round r + 2
-        for (uint32_t k = tid; k < n * 3; k += kFwdThreads) {
-            const uint32_t jj = k / 3, c = k % 3;
-            float4* slot = reinterpret_cast<float4*>(&SM.acc[b][jj][0]) + c;
-            const float4 v = *slot;
-            if (v.x != 0.0f || v.y != 0.0f || v.z != 0.0f || v.w != 0.0f) {
-                atomicAdd(reinterpret_cast<float4*>(g2d_view + size_t(SM.idx[bi][jj]) * kG2DStride) + c, v);
-                *slot = make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto store_round = [&](uint32_t r_end, uint32_t turn) {
+#pragma unroll
+        for (uint32_t u = 0; u < kPer; ++u) {
+            const uint32_t k = (tid ^ turn) + u * kAdjThreads;
+            if (k < min(kBwdRound, r_end)) {
+                if (pf_idx[u] < a.n) {
+                    stage_block_values(pf_c[u], pf_tex[u], pf_co[u], ox, oy, SM.e[k], SM.mask[k]);
+                } else {  // only reachable with corrupted lists
+                    stage_block_empty(SM.e[k]);
+                    SM.mask[k] = 0u;
+                }
+                SM.idx[k] = pf_idx[u];
             }
         }
+    };
+    const float2 one = f2(1.0f, 1.0f), mone = f2(-1.0f, -1.0f);
+    const uint32_t block = 4u * warp + (lane >> 3), j = lane & 7u;
+    load_round(max_last, 0u);
+    store_round(max_last, 0u);
+    __syncthreads();
+    uint32_t turn = 0;
+    for (uint32_t r_end = max_last; r_end > 0;) {
+        const uint32_t n = min(kBwdRound, r_end), next_end = r_end - n;
+        turn ^= 32u;
+        if (next_end) load_round(next_end, turn);
+        const uint32_t steps = build_block_lists<kBwdRound>(SM.lists, warp, lane, n, [&](uint32_t e) {
+            uint32_t m = uint32_t(SM.mask[e]) >> (4u * warp);
+#pragma unroll
+            for (uint32_t g = 0; g < 4; ++g)
+                if (e + bl[g] < r_end) m &= ~(1u << g);  // behind the block's last contributor
+            SM.met[warp][e] = uint8_t(m & 15u);
+            return m;
+        });
+        const uint16_t* list = SM.lists.e[block];
+        for (uint32_t i = 0; i < steps; ++i) {
+            const uint32_t jj = list[i];
+            const BlockStaged& E = SM.e[jj];
+            const uint32_t pos = r_end - 1u - jj;
+            const float4 sc = E.s, yb = E.yb, qco = E.qco, rg = E.rg;
+            const float2 bb = E.b;
+            const float dx = __fadd_rn(sc.x, P.nx), qadx = __fmul_rn(sc.y, dx);
+            float2 dpow[2], w[2], dy[2];
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                // p2 for both pixels, as in the forward
+                dy[h] = __fadd2_rn(f2(yb.x, yb.y), h ? P.ny1 : P.ny0);
+                const float2 t = __ffma2_rn(f2(yb.z, yb.w), dy[h], f2(qadx, qadx));
+                const float2 p2 = __ffma2_rn(t, f2(dx, dx), __fmul2_rn(__fmul2_rn(f2(qco.x, qco.y), dy[h]), dy[h]));
+                const bool ca = pos < last[2 * h] && !pair_skipped(p2.x, sc.z);
+                const bool cb = pos < last[2 * h + 1] && !pair_skipped(p2.y, sc.z);
+                const float2 raw = __fmul2_rn(f2(qco.z, qco.w), f2(ex2_approx(p2.x), ex2_approx(p2.y)));
+                const float2 alpha =
+                    f2(ca ? fminf(kAlphaMax, raw.x) : 0.0f, cb ? fminf(kAlphaMax, raw.y) : 0.0f);
+                const float2 om = __ffma2_rn(mone, alpha, one);  // 1 - alpha >= 0.01
+                T[h] = __fmul2_rn(T[h], f2(__fdividef(1.0f, om.x), __fdividef(1.0f, om.y)));  // in front of the entry
+                w[h] = __fmul2_rn(alpha, T[h]);
+                const float2 gc = __ffma2_rn(g2[h], bb, __ffma2_rn(g1[h], f2(rg.z, rg.w), __fmul2_rn(g0[h], f2(rg.x, rg.y))));
+                const float2 ad = __fmul2_rn(alpha, __fadd2_rn(gc, nA[h]));  // alpha (g.c - A)
+                nA[h] = __ffma2_rn(mone, ad, nA[h]);
+                const float2 dp = __fmul2_rn(T[h], ad);  // alpha dL/dalpha = dL/dpower, unless alpha is clamped
+                dpow[h] = f2(raw.x <= kAlphaMax ? dp.x : 0.0f, raw.y <= kAlphaMax ? dp.y : 0.0f);
+            }
+            const float2 s0 = __fmul2_rn(dpow[0], dy[0]), s1 = __fmul2_rn(dpow[1], dy[1]);
+            const float p0 = hsum(__fadd2_rn(dpow[0], dpow[1])), py = hsum(__fadd2_rn(s0, s1));
+            const float pyy = hsum(__ffma2_rn(s1, dy[1], __fmul2_rn(s0, dy[0])));
+            const float px = p0 * dx;
+            const float v[8] = {px, py, px * dx, py * dx, pyy, p0,
+                                hsum(__ffma2_rn(g0[1], w[1], __fmul2_rn(g0[0], w[0]))),
+                                hsum(__ffma2_rn(g1[1], w[1], __fmul2_rn(g1[0], w[0])))};
+            float v9 = hsum(__ffma2_rn(g2[1], w[1], __fmul2_rn(g2[0], w[0])));
+            SM.sums[block][jj * 8u + j] = group_sum8_transposed(v, lane);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) v9 += __shfl_xor_sync(0xFFFFFFFFu, v9, o);
+            if (j == 0) SM.sum9[block][jj] = v9;
+        }
+        __syncthreads();  // the round's sums are complete
+        // warp 0: the record's first 16 bytes; warp 1: the other 20
+        for (uint32_t k = lane; k < n; k += 32u) {
+            const uint32_t met = uint32_t(SM.met[0][k]) | uint32_t(SM.met[1][k]) << 4;
+            if (!met) continue;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            float v9 = 0.f;
+#pragma unroll
+            for (uint32_t b = 0; b < kBlendBlocks; ++b) {
+                if (!((met >> b) & 1u)) continue;
+                const float4 x = *reinterpret_cast<const float4*>(&SM.sums[b][k * 8u + 4u * warp]);
+                v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
+                if (warp) v9 += SM.sum9[b][k];
+            }
+            const BlockStaged& E = SM.e[k];
+            float* rec = g2d_view + size_t(SM.idx[k]) * kG2DStride;
+            if (warp == 0) {
+                // d power / d(dx, dy) = ln2 (2 qa dx + qb dy, 2 qc dy + qb dx)
+                const float qa = E.s.y, qb = E.yb.z, qc = E.qco.x;
+                v = make_float4(kLn2 * (2.0f * qa * v.x + qb * v.y), kLn2 * (2.0f * qc * v.y + qb * v.x), -0.5f * v.z,
+                                -v.w);
+            } else {
+                v = make_float4(-0.5f * v.x, __fdividef(v.y, E.qco.z), v.z, v.w);  // alpha = opacity exp(power)
+                if (v9 != 0.0f) atomicAdd(rec + 8, v9);
+            }
+            if (v.x != 0.0f || v.y != 0.0f || v.z != 0.0f || v.w != 0.0f)
+                atomicAdd(reinterpret_cast<float4*>(rec) + warp, v);
+        }
+        __syncthreads();  // (the flush has read the entries that are staged over)
+        if (next_end) store_round(next_end, turn);
+        __syncthreads();
+        r_end = next_end;
     }
-    __syncthreads();  // the flush of the last round is done before SM is used again
 }
 
 // One CTA per tile, tile order[b] for CTA b; or (kPersistent) one CTA per
 // resident slot taking the tiles from the queue in that order.
 template <uint32_t kBwdRound, bool kPersistent>
-__global__ void __launch_bounds__(kFwdThreads, bwd_min_blocks<kBwdRound>())
+__global__ void __launch_bounds__(kAdjThreads, bwd_min_blocks<kBwdRound>())
     blend_backward_kernel(BlendBackwardArgs a) {
-    __shared__ __align__(16) BlendBackwardSmem<kBwdRound> SM;
+    extern __shared__ __align__(16) unsigned char bwd_smem[];
+    BlendBackwardSmem<kBwdRound>& SM = *reinterpret_cast<BlendBackwardSmem<kBwdRound>*>(bwd_smem);
     pdl_wait();  // launched as a dependent of the stream's previous kernel: its output is read below
     pdl_trigger();
     if (a.ctl->status & (kStatusFatal | kStatusKeyOverflow)) return;  // no valid frame to differentiate
@@ -713,15 +820,20 @@ void launch_tile_order(const uint32_t* ranges, uint32_t n_tiles, FrameCtl* ctl, 
 namespace {
 
 template <typename Kernel>
-int resident_ctas(Kernel k) {
+int resident_ctas(Kernel k, uint32_t threads, size_t smem) {
     int r = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k, kFwdThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k, int(threads), smem);
     return r > 0 ? r : 1;
 }
 template <uint32_t R, bool P, bool K>
-int blend_occupancy() { return resident_ctas(blend_kernel<R, P, K>); }
+int blend_occupancy() { return resident_ctas(blend_kernel<R, P, K>, kFwdThreads, 0); }
+// the adjoint's shared-memory opt-in (a round of 128 takes above 48 KB) and its resident CTAs
 template <uint32_t R, bool P>
-int blend_backward_occupancy() { return resident_ctas(blend_backward_kernel<R, P>); }
+int blend_backward_setup() {
+    cudaFuncSetAttribute(blend_backward_kernel<R, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         int(sizeof(BlendBackwardSmem<R>)));
+    return resident_ctas(blend_backward_kernel<R, P>, kAdjThreads, sizeof(BlendBackwardSmem<R>));
+}
 
 template <uint32_t R, bool P, bool K>
 void launch_blend_k(const BlendArgs& a, int num_sms, cudaStream_t s) {
@@ -744,9 +856,9 @@ void launch_blend_t(const BlendArgs& a, int num_sms, cudaStream_t s) {
 
 template <uint32_t R, bool P>
 void launch_blend_backward_t(const BlendBackwardArgs& a, int num_sms, cudaStream_t s) {
-    const uint32_t grid = P ? std::min<uint32_t>(a.n_tiles, uint32_t(num_sms * device_once(blend_backward_occupancy<R, P>)))
-                            : a.n_tiles;
-    launch_dependent(blend_backward_kernel<R, P>, dim3(grid), dim3(kFwdThreads), 0, s, a);
+    const int resident = device_once(blend_backward_setup<R, P>);
+    const uint32_t grid = P ? std::min<uint32_t>(a.n_tiles, uint32_t(num_sms * resident)) : a.n_tiles;
+    launch_dependent(blend_backward_kernel<R, P>, dim3(grid), dim3(kAdjThreads), sizeof(BlendBackwardSmem<R>), s, a);
 }
 
 }  // namespace
