@@ -403,19 +403,32 @@ __global__ void __launch_bounds__(kScanThreads)
 
 // Raw parameters -> records (activation as in GaussianGeometry.cpp:112-115:
 // sigmoid opacity, exp scale, modifier 1; the quaternion is copied as given).
-__global__ void pack_records_kernel(const float* means, const float* log_scales, const float* quats,
-                                    const float* logits, const float* sh, uint32_t n, float* recs) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float* r = recs + size_t(i) * kRecordFloats;
-    r[0] = means[i * 3 + 0];
-    r[1] = means[i * 3 + 1];
-    r[2] = means[i * 3 + 2];
-    r[3] = 1.0f / (1.0f + expf(-logits[i]));
-    for (int k = 0; k < 4; ++k) r[4 + k] = quats[i * 4 + k];
-    for (int k = 0; k < 3; ++k) r[8 + k] = expf(log_scales[i * 3 + k]);
-    r[11] = 1.0f;
-    for (int k = 0; k < 48; ++k) r[12 + k] = sh[size_t(i) * 48 + k];
+// One thread per 16 bytes of a record (15 of them), so the records are written
+// and the 192 bytes of SH read coalesced; a thread per record took 106 us for
+// 200,000 records, this 23 (96 MB in and out, 14 us at copy speed). kVec: quats and sh are 16-byte aligned.
+template <bool kVec>
+__global__ void __launch_bounds__(256)
+    pack_records_kernel(const float* __restrict__ means, const float* __restrict__ log_scales,
+                        const float* __restrict__ quats, const float* __restrict__ logits,
+                        const float* __restrict__ sh, uint32_t n, float* __restrict__ recs) {
+    constexpr uint32_t kPieces = kRecordFloats / 4;
+    const uint64_t t = uint64_t(blockIdx.x) * 256u + threadIdx.x;
+    if (t >= uint64_t(n) * kPieces) return;
+    const size_t i = t / kPieces;
+    const uint32_t q = uint32_t(t - uint64_t(i) * kPieces);
+    auto four = [](const float* p) {
+        return kVec ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(p[0], p[1], p[2], p[3]);
+    };
+    float4 v;
+    if (q == 0)
+        v = make_float4(means[i * 3 + 0], means[i * 3 + 1], means[i * 3 + 2], 1.0f / (1.0f + expf(-logits[i])));
+    else if (q == 1)
+        v = four(quats + i * 4);
+    else if (q == 2)
+        v = make_float4(expf(log_scales[i * 3 + 0]), expf(log_scales[i * 3 + 1]), expf(log_scales[i * 3 + 2]), 1.0f);
+    else
+        v = four(sh + i * 48 + (q - 3u) * 4u);
+    reinterpret_cast<float4*>(recs)[t] = v;
 }
 
 }  // namespace
@@ -454,7 +467,12 @@ void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint6
 void launch_pack_records(const float* means, const float* log_scales, const float* quats, const float* logits,
                          const float* sh, uint32_t n, float* recs, cudaStream_t s) {
     if (n == 0) return;
-    pack_records_kernel<<<(n + 255) / 256, 256, 0, s>>>(means, log_scales, quats, logits, sh, n, recs);
+    const uint64_t blocks = (uint64_t(n) * (kRecordFloats / 4) + 255) / 256;
+    const bool vec = ((reinterpret_cast<uintptr_t>(quats) | reinterpret_cast<uintptr_t>(sh)) & 15u) == 0;
+    if (vec)
+        pack_records_kernel<true><<<unsigned(blocks), 256, 0, s>>>(means, log_scales, quats, logits, sh, n, recs);
+    else
+        pack_records_kernel<false><<<unsigned(blocks), 256, 0, s>>>(means, log_scales, quats, logits, sh, n, recs);
 }
 
 }  // namespace tpd
