@@ -93,6 +93,7 @@ struct tpd_engine {
     uint32_t n_ent = 1;
     bool compiled = false;
     float* d_recs = nullptr;
+    uint64_t recs_cap = 0;          // records d_recs holds
     uint32_t* d_ent_idx = nullptr;
     float* h_transforms = nullptr;  // pinned, n_ent x 16
     float* d_transforms = nullptr;
@@ -630,19 +631,39 @@ int set_views_internal(tpd_engine* e, const tpd_view* views, uint32_t nv) {
     return ensure_splat_buffers(e);
 }
 
-int alloc_scene(tpd_engine* e, uint32_t n, uint32_t n_ent) {
-    invalidate_graph(e);
+// Buffers of a scene of n records and n_ent entities. An optimisation loop
+// compiles a scene of the same size at every step, so buffers that fit are
+// kept (records: unless the scene halves, which gives them back), and so is
+// the captured frame where nothing it reads has moved: one entity, no
+// transforms, the same n. Allocating anew cost 0.3 to 0.5 ms a step and an
+// eager frame: forward and gradients of 5,003 Gaussians 554 -> 514 us, of
+// 200,000 at 800x800 1,034 -> 794 us (of these, 230 are the autograd call).
+int alloc_scene(tpd_engine* e, uint32_t n, uint32_t n_ent, bool entities) {
+    if (n_ent == 0) n_ent = 1;
+    // work in flight may read the buffers that are written next, and the
+    // inputs may come from another stream (freeing memory waited for both)
+    TPD_CUDA(e, cudaDeviceSynchronize());
+    const bool same_frame = e->compiled && e->n == n && n > 0 && e->n_ent == 1 && n_ent == 1 && !entities &&
+                            !e->d_ent_idx && e->identity_transforms;
+    if (!same_frame) invalidate_graph(e);
     e->frame_valid = false;
+    e->compiled = false;
     e->n = n;
-    e->n_ent = n_ent ? n_ent : 1;
-    TPD_CUDA(e, dalloc(e->d_recs, uint64_t(n) * kRecordFloats));
-    if (e->h_transforms) cudaFreeHost(e->h_transforms);
-    e->h_transforms = nullptr;
-    TPD_CUDA(e, cudaMallocHost(reinterpret_cast<void**>(&e->h_transforms), sizeof(float) * 16 * e->n_ent));
+    if (n > e->recs_cap || n < e->recs_cap / 2 || n == 0) {
+        e->recs_cap = 0;
+        TPD_CUDA(e, dalloc(e->d_recs, uint64_t(n) * kRecordFloats));
+        e->recs_cap = n;
+    }
+    if (!e->h_transforms || n_ent != e->n_ent) {
+        e->n_ent = n_ent;
+        if (e->h_transforms) cudaFreeHost(e->h_transforms);
+        e->h_transforms = nullptr;
+        TPD_CUDA(e, cudaMallocHost(reinterpret_cast<void**>(&e->h_transforms), sizeof(float) * 16 * e->n_ent));
+        TPD_CUDA(e, dalloc(e->d_transforms, uint64_t(e->n_ent) * 16));
+    }
     for (uint32_t k = 0; k < e->n_ent; ++k)
         for (int j = 0; j < 16; ++j) e->h_transforms[k * 16 + j] = (j % 5) == 0 ? 1.f : 0.f;
     e->identity_transforms = true;
-    TPD_CUDA(e, dalloc(e->d_transforms, uint64_t(e->n_ent) * 16));
     if (e->n_views) return ensure_splat_buffers(e);
     return TPD_OK;
 }
@@ -846,7 +867,7 @@ int tpd_compile(tpd_engine* e, const void* records, uint32_t n, const uint32_t* 
             if (entity_index[i] >= n_entities) return fail(e, TPD_ERR_ARG, "entity index out of range");
     }
     cudaSetDevice(e->device);
-    int rc = alloc_scene(e, n, n_entities);
+    int rc = alloc_scene(e, n, n_entities, entity_index != nullptr);
     if (rc != TPD_OK) return rc;
     if (n) TPD_CUDA(e, cudaMemcpy(e->d_recs, records, uint64_t(n) * kRecordBytes, cudaMemcpyHostToDevice));
     if (entity_index && n) {
@@ -865,7 +886,7 @@ int tpd_compile_params_device(tpd_engine* e, const float* means, const float* lo
     if (n > 0 && (!means || !log_scales || !quats || !opacity_logits || !sh))
         return fail(e, TPD_ERR_ARG, "parameter pointer is NULL");
     cudaSetDevice(e->device);
-    int rc = alloc_scene(e, n, 1);
+    int rc = alloc_scene(e, n, 1, false);
     if (rc != TPD_OK) return rc;
     dfree(e->d_ent_idx);
     launch_pack_records(means, log_scales, quats, opacity_logits, sh, n, e->d_recs, e->stream);
