@@ -11,8 +11,7 @@
 //  1. In the frame the digit histograms come from earlier kernels (the
 //     preprocess counts the depth keys' digits, key duplication those of the
 //     tile ids); sort_histogram_kernel builds them for standalone sorts (one
-//     read of the keys, warp match-any aggregation into shared memory, one
-//     global atomic per bin per CTA).
+//     read of the keys).
 //  2. onesweep_kernel, once per pass: a persistent CTA takes 4096-key
 //     partitions by atomic ticket, loads them with coalesced warp-striped
 //     loads, ranks keys per warp (bit ballots, or match-any in the 512-thread
@@ -59,7 +58,7 @@ constexpr int kPassDropCulled = 1; // as plain; keys whose low 32 bits are 0xFFF
 constexpr int kPassCompacted = 2;  // K = ctl->depth_count; a uniform digit skips the pass (ctl->depth_skips)
 
 constexpr uint32_t kHistThreads = 256;
-constexpr uint32_t kHistChunk = 2048;  // keys per grid-stride chunk of the histogram kernel
+constexpr uint32_t kHistChunk = 2048;  // keys per grid-stride chunk of the histogram kernel (256 threads x 8)
 
 // Reorder buffers hold one pad slot per 16 keys: digit runs of about 16 keys
 // (8-bit digits over a 4096-key partition) put the runs of consecutive digits
@@ -101,49 +100,56 @@ __global__ void sort_begin_kernel(FrameCtl* ctl, uint32_t total) {
     }
 }
 
-__device__ __forceinline__ void hist_add(uint32_t* h, uint32_t d) {
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-    const uint32_t leader = __ffs(peers) - 1;
-    if ((threadIdx.x & 31u) == leader && d < kRadix) atomicAdd(&h[d], __popc(peers));
-}
+// Digit counts of a standalone sort: one read of the keys, one shared-memory
+// increment per key and digit (an increment by one of one address from
+// several lanes is a single operation of the hardware), in four copies by warp
+// so that warps rarely meet, then one global atomic per non-zero bin and CTA.
+// 9M keys of 45 bits: 25 us (72 MB, 11 us at copy speed); with match-any
+// aggregation, six per key, it was 290 us. kHistKeys loads per thread are in flight at once.
+constexpr uint32_t kHistCopies = 4;
+constexpr uint32_t kHistKeys = 8;
 
 template <typename KeyT>
 __global__ void __launch_bounds__(kHistThreads)
     sort_histogram_kernel(const KeyT* __restrict__ keys, uint32_t capacity, uint32_t p0, uint32_t p1,
                           uint32_t key_bits, uint32_t (*hist)[256], FrameCtl* ctl) {
-    __shared__ uint32_t sh[8][kRadix];
+    __shared__ uint32_t sh[kHistCopies][8][kRadix];
     // launched as a dependent of the stream's previous kernel: its output is
     // read below. No early trigger: the next kernel is one wave of CTAs, which
     // must be placed on empty SMs, not onto the first ones this grid frees
     pdl_wait();
     const uint32_t tid = threadIdx.x;
-    for (uint32_t i = tid; i < 8 * kRadix; i += kHistThreads) (&sh[0][0])[i] = 0;
+    for (uint32_t i = tid; i < kHistCopies * 8 * kRadix; i += kHistThreads) (&sh[0][0][0])[i] = 0;
     __syncthreads();
     const uint32_t K = (ctl->status & kStatusFatal) ? 0u : min(ctl->total_keys, capacity);
-    uint32_t shift[8], mask[8];
+    uint32_t(*mine)[kRadix] = sh[(tid >> 5) % kHistCopies];
+    auto count = [&](KeyT k) {
 #pragma unroll
-    for (uint32_t p = 0; p < 8; ++p) {
-        shift[p] = p * kRadixBits;
-        const uint32_t b = (p * kRadixBits < key_bits) ? min(kRadixBits, key_bits - p * kRadixBits) : 0u;
-        mask[p] = (1u << b) - 1u;
-    }
-    // grid-stride over chunks of kHistChunk keys; the trip count is uniform per CTA
+        for (uint32_t p = 0; p < 8; ++p) {
+            if (p < p0 || p >= p1) continue;  // (uniform)
+            const uint32_t b = min(kRadixBits, key_bits - p * kRadixBits);
+            atomicAdd(&mine[p][uint32_t(uint64_t(k) >> (p * kRadixBits)) & ((1u << b) - 1u)], 1u);
+        }
+    };
     const uint32_t nchunks = (K + kHistChunk - 1) / kHistChunk;
     for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const uint32_t base = c * kHistChunk;
-#pragma unroll 2
-        for (uint32_t j = tid; j < kHistChunk; j += kHistThreads) {
-            const uint32_t idx = base + j;
-            const bool v = idx < K;
-            const uint64_t k = v ? uint64_t(keys[idx]) : 0ull;
-            for (uint32_t p = p0; p < p1; ++p)
-                hist_add(sh[p], v ? (uint32_t(k >> shift[p]) & mask[p]) : kInvalidDigit);
-        }
+        const uint32_t base = c * kHistChunk + tid;
+        KeyT k[kHistKeys];
+#pragma unroll
+        for (uint32_t j = 0; j < kHistKeys; ++j)
+            k[j] = base + j * kHistThreads < K ? keys[base + j * kHistThreads] : KeyT(0);
+#pragma unroll
+        for (uint32_t j = 0; j < kHistKeys; ++j)
+            if (base + j * kHistThreads < K) count(k[j]);
     }
     __syncthreads();
     for (uint32_t p = p0; p < p1; ++p)
-        for (uint32_t d = tid; d < kRadix; d += kHistThreads)
-            if (sh[p][d]) atomicAdd(&hist[p][d], sh[p][d]);
+        for (uint32_t d = tid; d < kRadix; d += kHistThreads) {
+            uint32_t c = 0;
+#pragma unroll
+            for (uint32_t q = 0; q < kHistCopies; ++q) c += sh[q][p][d];
+            if (c) atomicAdd(&hist[p][d], c);
+        }
 }
 
 // Resolves the exclusive prefix of one digit for partition `part` by walking
