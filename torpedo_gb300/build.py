@@ -27,6 +27,7 @@ SOURCES = {
     "preprocess.cu": ["--fmad=false"],
     "keygen.cu": [],
     "sort.cu": [],
+    "sort_small.cu": [],
     "blend.cu": [],
     "backward.cu": [],
     "engine.cu": [],

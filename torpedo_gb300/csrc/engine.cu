@@ -424,8 +424,13 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     dp.threads = e->settings.depth_sort_threads == 512 ? 512 : 256;
     dp.fixed_count = items;
     dp.compact_culled = true;  // culled items leave in the first pass; the rest sort ctl->depth_count
-    e->depth_in_alt = launch_sort(e->d_dkeys[0], e->d_ditems[0], e->d_dkeys[1], e->d_ditems[1], items, dp,
-                                  e->d_desc_depth, e->d_ctl, spin, e->num_sms, s);
+    if (items <= kSmallSortMax) {  // one launch instead of a pass per digit (sort_small.cu)
+        launch_small_depth_sort(e->d_dkeys[0], e->d_ditems[0], items, e->depth_key_bits, e->d_ctl, s);
+        e->depth_in_alt = false;
+    } else {
+        e->depth_in_alt = launch_sort(e->d_dkeys[0], e->d_ditems[0], e->d_dkeys[1], e->d_ditems[1], items, dp,
+                                      e->d_desc_depth, e->d_ctl, spin, e->num_sms, s);
+    }
     // the order is in the other buffer when a pass skipped (ctl->depth_skips odd)
     const uint32_t* order = e->d_ditems[e->depth_in_alt ? 1 : 0];
     const uint32_t* order_other = e->d_ditems[e->depth_in_alt ? 0 : 1];
@@ -635,9 +640,9 @@ int set_views_internal(tpd_engine* e, const tpd_view* views, uint32_t nv) {
 // compiles a scene of the same size at every step, so buffers that fit are
 // kept (records: unless the scene halves, which gives them back), and so is
 // the captured frame where nothing it reads has moved: one entity, no
-// transforms, the same n. Allocating anew cost 0.3 to 0.5 ms a step and an
-// eager frame: forward and gradients of 5,003 Gaussians 554 -> 514 us, of
-// 200,000 at 800x800 1,034 -> 794 us (of these, 230 are the autograd call).
+// transforms, the same n. Against allocating anew and an eager frame: forward
+// and gradients of 5,003 Gaussians 554 -> 514 us, of 200,000 at 800x800 1,034
+// -> 794 us (of these, 230 are the autograd call).
 int alloc_scene(tpd_engine* e, uint32_t n, uint32_t n_ent, bool entities) {
     if (n_ent == 0) n_ent = 1;
     // work in flight may read the buffers that are written next, and the
@@ -1363,6 +1368,11 @@ int tpd_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t*
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     FrameCtl* ctl = static_cast<FrameCtl*>(workspace);
     uint64_t* desc = reinterpret_cast<uint64_t*>(static_cast<char*>(workspace) + 256 * ((sizeof(FrameCtl) + 255) / 256));
+    if (n <= kSmallSortMax) {  // one launch (sort_small.cu)
+        launch_small_sort(keys, vals, keys_alt, vals_alt, n, key_bits, ctl, s);
+        *result_in_alt = 1;
+        return cudaGetLastError() == cudaSuccess ? TPD_OK : TPD_ERR_DEVICE;
+    }
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -180,6 +180,16 @@ bool launch_sort(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* v
 bool launch_sort(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, uint32_t capacity,
                  const SortPlan& plan, uint64_t* desc, FrameCtl* ctl, uint32_t spin_limit, int num_sms,
                  cudaStream_t s);
+// Few pairs: the whole sort as one launch (sort_small.cu). The depth form
+// writes the first ctl->depth_count items (their position in keys) in (view,
+// depth) order; the plain one sorts (keys, vals) on the low key_bits bits into
+// (keys_out, vals_out), other buffers than the inputs, and clears ctl->status.
+constexpr uint32_t kSmallSortMax = 12288;
+void launch_small_depth_sort(const uint64_t* keys, uint32_t* items_out, uint32_t n, uint32_t key_bits, FrameCtl* ctl,
+                             cudaStream_t s);
+void launch_small_sort(const uint64_t* keys, const uint32_t* vals, uint64_t* keys_out, uint32_t* vals_out, uint32_t n,
+                       uint32_t key_bits, FrameCtl* ctl, cudaStream_t s);
+
 // Clears status, histograms and tickets, sets total_keys and advances the tag
 // (standalone stage calls).
 void launch_sort_begin(FrameCtl* ctl, uint32_t total, cudaStream_t s);
