@@ -114,7 +114,7 @@ struct tpd_engine {
     uint64_t splat_cap = 0;  // entries of splats / offsets / depth keys (views x n)
     Splat* d_splats = nullptr;
     uint32_t* d_offsets = nullptr;  // key offsets of the items in depth order
-    uint64_t* d_dkeys[2] = {nullptr, nullptr};
+    uint64_t* d_dkeys[2] = {nullptr, nullptr};  // one allocation; [1] follows [0]
     uint32_t* d_ditems[2] = {nullptr, nullptr};
     uint64_t* d_desc_depth = nullptr;
     uint32_t depth_key_bits = 32;
@@ -249,10 +249,9 @@ int ensure_splat_buffers(tpd_engine* e) {
         invalidate_graph(e);
         TPD_CUDA(e, dalloc(e->d_splats, need));
         TPD_CUDA(e, dalloc(e->d_offsets, need));
-        for (int b = 0; b < 2; ++b) {
-            TPD_CUDA(e, dalloc(e->d_dkeys[b], need));
-            TPD_CUDA(e, dalloc(e->d_ditems[b], need));
-        }
+        TPD_CUDA(e, dalloc(e->d_dkeys[0], 2 * need));
+        e->d_dkeys[1] = e->d_dkeys[0] + need;
+        for (int b = 0; b < 2; ++b) TPD_CUDA(e, dalloc(e->d_ditems[b], need));
         const size_t de = sort_desc_entries(uint32_t(need), 4);  // room for the smallest partitions
         TPD_CUDA(e, dalloc(e->d_desc_depth, de));
         TPD_CUDA(e, cudaMemset(e->d_desc_depth, 0, de * 8));
@@ -445,9 +444,7 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     ka.n = e->n;
     ka.views = e->d_views;
     ka.offsets = e->d_offsets;
-    // the depth sort's key buffers are free now: the items' rectangles and slots
-    ka.item_rects = reinterpret_cast<uint2*>(e->d_dkeys[0]);
-    ka.item_slots = reinterpret_cast<uint2*>(e->d_dkeys[1]);
+    ka.item_info = reinterpret_cast<uint4*>(e->d_dkeys[0]);  // both depth-key buffers, free now
     ka.part_first = e->d_part_first;
     ka.tiles = e->d_tiles[0];
     ka.vals = e->d_vals[0];
@@ -817,10 +814,8 @@ void tpd_destroy(tpd_engine* e) {
     dfree(e->d_image_offset);
     dfree(e->d_splats);
     dfree(e->d_offsets);
-    for (int b = 0; b < 2; ++b) {
-        dfree(e->d_dkeys[b]);
-        dfree(e->d_ditems[b]);
-    }
+    dfree(e->d_dkeys[0]);
+    for (int b = 0; b < 2; ++b) dfree(e->d_ditems[b]);
     dfree(e->d_desc_depth);
     dfree(e->d_desc_pre);
     dfree(e->d_ent_mats);

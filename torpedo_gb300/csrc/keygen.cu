@@ -20,10 +20,11 @@
 // slots matters because depth order puts the nearest Gaussians, with the
 // largest rectangles, side by side: one kernel over 512-item partitions gave
 // the first CTA up to a million keys to write while the others were done
-// (1M Gaussians at 1080p from the edge of the cloud: 303 us, now 24 + 43;
-// 3M at 2160p: 1189 us, now 71 + 310; 10,000 at 256x256: 11 us with the scan of
-// the counts, now 6 + 8).
+// (1M Gaussians at 1080p from the edge of the cloud: 303 us, now T1;
+// 3M at 2160p: 1189 us, now T2; 10,000 at 256x256: 11 us with the scan of
+// the counts, now T3).
 #include <algorithm>
+#include <type_traits>
 
 #include "tpd_common.cuh"
 #include "tpd_counted.cuh"
@@ -76,10 +77,10 @@ __device__ __forceinline__ ItemRect item_rect(uint32_t item, bool valid, float4 
 //  3. one warp resolves the partition's exclusive prefix with the bounded
 //     decoupled look-back (prefix.slang:100-114 as restated in tpd_scan.cuh):
 //     the last partition's inclusive prefix is the frame's key count K;
-//  4. each lane stores its items' key offsets (the scan's output), their
-//     rectangles and (offset, Gaussian) pairs for expand_keys_kernel, and, for
-//     every multiple of 4096 among an item's slots, the item's position in
-//     part_first.
+//  4. each lane stores its items' key offsets (the scan's output), for
+//     expand_keys_kernel their rectangles, offsets and Gaussians (16 bytes an
+//     item), and, for every multiple of 4096 among an item's slots, the item's
+//     position in part_first.
 // A CTA takes a ticket only when it starts on the partition, so every
 // partition a look-back waits on is being worked on by a running CTA and
 // publishes its aggregate soon. Bound by the gathers (32 bytes of every
@@ -94,9 +95,8 @@ __global__ void __launch_bounds__(kScanItemsThreads)
     scan_items_kernel(const Splat* __restrict__ splats, const uint32_t* __restrict__ items,
                       const uint32_t* __restrict__ items_other, uint32_t n_items, uint32_t n,
                       const ViewConst* __restrict__ views, uint32_t* __restrict__ offsets,
-                      uint2* __restrict__ item_rects, uint2* __restrict__ item_slots,
-                      uint32_t* __restrict__ part_first, uint32_t capacity, uint32_t* __restrict__ ranges,
-                      uint32_t n_tiles, uint64_t* desc, FrameCtl* ctl, uint32_t spin_limit, uint32_t never_publish) {
+                      uint4* __restrict__ item_info, uint32_t* __restrict__ part_first, uint32_t capacity,
+                      uint32_t* __restrict__ ranges, uint32_t n_tiles, uint64_t* desc, FrameCtl* ctl, uint32_t spin_limit, uint32_t never_publish) {
     __shared__ ScanItemsSmem S;
     pdl_wait();     // launched as a dependent of the depth sort's last pass: its order is read below
     pdl_trigger();  // expand_keys_kernel may be scheduled (it waits for this grid)
@@ -168,8 +168,7 @@ __global__ void __launch_bounds__(kScanItemsThreads)
             const uint32_t r = r0 + 32u * c, first = base + incl[c] - rect[c].cnt;
             if (r < count) {
                 offsets[r] = first;
-                item_rects[r] = make_uint2(rect[c].t0, rect[c].wgx);
-                item_slots[r] = make_uint2(first, rect[c].gi);
+                item_info[r] = make_uint4(rect[c].t0, rect[c].wgx, first, rect[c].gi);
                 // (keys past the capacity are not written: the frame is flagged)
                 const uint32_t end = min(first + rect[c].cnt, capacity);
                 for (uint32_t p = (first + kCountedTile - 1) / kCountedTile; p * kCountedTile < end; ++p)
@@ -186,8 +185,10 @@ __global__ void __launch_bounds__(kScanItemsThreads)
 //     next partition's first slot; each marks its first slot in an owner map
 //     in shared memory, and a prefix maximum over the map gives every slot its
 //     item.
-//  2. Slots tid, tid + 256, ...: the slot's (row, column) in its item's
-//     rectangle, the key and value, stored coalesced.
+//  2. A thread takes four consecutive slots at a time, so that keys and values
+//     are stored 16 bytes at once. The first slot's (row, column) in its item's
+//     rectangle takes a division; the next slot is the next column or row of
+//     the same item, or the first of the next item.
 // A key is stored as its tile id alone: the low 32 bits of the reference's
 // key are the depth, already in order, and the depth of a key is that of its
 // value's splat, so the sort needs only the tile ids and the full keys can be
@@ -196,17 +197,18 @@ __global__ void __launch_bounds__(kScanItemsThreads)
 // written and finished into the global digit offsets of the key sort's first
 // pass (counted_finish), which then needs no counting kernel. work == nullptr
 // (look-back passes): every digit of the tile ids is added to ctl->sort_hist.
-// Bound by issue: about 35 instructions a key, the map included; the stores
-// are 8 bytes a key. 310 us for a 2160p frame of 3M Gaussians.
+// Bound by latency and issue; the stores are 8 bytes a key. With one key per
+// thread and step (35 instructions a key, two dependent loads) 1M Gaussians at
+// 1080p took 67 us with the scan, 8 views of 500,000 at 720p 216; now 57 and
+// 171.
 constexpr uint32_t kExpandThreads = 256;
 constexpr uint32_t kExpandSlots = kCountedTile / kExpandThreads;
 constexpr uint32_t kTileDigitsMax = 4;
 
 template <bool kCounted>
 __global__ void __launch_bounds__(kExpandThreads)
-    expand_keys_kernel(const uint2* __restrict__ item_rects, const uint2* __restrict__ item_slots,
-                       const uint32_t* __restrict__ part_first, uint32_t* __restrict__ tiles,
-                       uint32_t* __restrict__ vals, uint32_t n_items, uint32_t capacity, uint32_t max_parts,
+    expand_keys_kernel(const uint4* __restrict__ item_info, const uint32_t* __restrict__ part_first,
+                       uint32_t* __restrict__ tiles, uint32_t* __restrict__ vals, uint32_t n_items, uint32_t capacity, uint32_t max_parts,
                        uint32_t tile_bits, uint32_t* __restrict__ work, FrameCtl* ctl) {
     __shared__ __align__(16) uint16_t owner[kCountedTile];  // item of each slot, from the partition's first
     __shared__ uint32_t digits[kCounted ? 1 : kTileDigitsMax][256];
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(kExpandThreads)
     for (uint32_t p = 0; p < (kCounted ? 1u : kTileDigitsMax); ++p) digits[p][tid] = 0;
     __syncthreads();
     for (uint32_t k = tid + 1u; k < m; k += kExpandThreads) {  // (item 0 owns slot 0: the map's zeros)
-        const uint32_t slot = item_slots[first + k].x - base;
+        const uint32_t slot = item_info[first + k].z - base;
         if (slot < cnt) owner[slot] = uint16_t(k);
     }
     __syncthreads();
@@ -261,31 +263,64 @@ __global__ void __launch_bounds__(kExpandThreads)
     own4[2 * tid + 1] = *reinterpret_cast<const uint4*>(o + 8);
     __syncthreads();
     const uint32_t ndig = kCounted ? 1u : min(kTileDigitsMax, (tile_bits + 7u) / 8u);
-#pragma unroll 4
-    for (uint32_t q = 0; q < kExpandSlots; ++q) {
-        const uint32_t slot = q * kExpandThreads + tid;
-        if (slot >= cnt) break;
-        const uint32_t item = first + owner[slot];
-        const uint2 rect = __ldg(item_rects + item), at = __ldg(item_slots + item);
-        const uint32_t local = base + slot - at.x;  // < 2^24: exact in a float
-        const uint32_t w = rect.y & 0xFFFFu;
-        // row = local / w from a float quotient, corrected by one step
-        uint32_t ty = __float2uint_rz(__fdividef(float(local), float(w)));
-        int32_t rem = int32_t(local) - int32_t(ty * w);
-        if (rem < 0) {
-            --ty;
-            rem += int32_t(w);
-        } else if (rem >= int32_t(w)) {
-            ++ty;
-            rem -= int32_t(w);
-        }
-        const uint32_t tile = rect.x + ty * (rect.y >> 16) + uint32_t(rem);
-        tiles[base + slot] = tile;
-        vals[base + slot] = at.y;
+    // kFull: a whole partition (all but the last), without per-slot checks
+    auto expand = [&](auto full_tag) {
+        constexpr bool kFull = decltype(full_tag)::value;
 #pragma unroll
-        for (uint32_t p = 0; p < (kCounted ? 1u : kTileDigitsMax); ++p)
-            if (p < ndig) atomicAdd(&digits[p][(tile >> (8u * p)) & 255u], 1u);
-    }
+        for (uint32_t q = 0; q < kExpandSlots / 4u; ++q) {
+            const uint32_t slot = q * (4u * kExpandThreads) + 4u * tid;
+            if (!kFull && slot >= cnt) break;
+            const uint2 own = *reinterpret_cast<const uint2*>(owner + slot);  // four 16-bit owners
+            const uint32_t o[4] = {own.x & 0xFFFFu, own.x >> 16, own.y & 0xFFFFu, own.y >> 16};
+            uint4 info[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) info[u] = __ldg(item_info + first + o[u]);
+            uint32_t w = info[0].y & 0xFFFFu;
+            const uint32_t local = base + slot - info[0].z;  // < 2^24: exact in a float
+            // row = local / w from a float quotient, corrected by one step
+            uint32_t ty = __float2uint_rz(__fdividef(float(local), float(w)));
+            int32_t col = int32_t(local) - int32_t(ty * w);
+            if (col < 0) {
+                --ty;
+                col += int32_t(w);
+            } else if (col >= int32_t(w)) {
+                ++ty;
+                col -= int32_t(w);
+            }
+            uint32_t t[4], x = uint32_t(col);
+            t[0] = info[0].x + ty * (info[0].y >> 16) + x;
+#pragma unroll
+            for (uint32_t u = 1; u < 4; ++u) {
+                const bool next_item = o[u] != o[u - 1], next_row = x + 1u == w;
+                const uint32_t step = next_row ? (info[u].y >> 16) - w + 1u : 1u;
+                t[u] = next_item ? info[u].x : t[u - 1] + step;
+                x = next_item || next_row ? 0u : x + 1u;
+                w = info[u].y & 0xFFFFu;
+            }
+            if (kFull || slot + 4u <= cnt) {
+                *reinterpret_cast<uint4*>(tiles + base + slot) = make_uint4(t[0], t[1], t[2], t[3]);
+                *reinterpret_cast<uint4*>(vals + base + slot) = make_uint4(info[0].w, info[1].w, info[2].w, info[3].w);
+            } else {
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u)
+                    if (slot + u < cnt) {
+                        tiles[base + slot + u] = t[u];
+                        vals[base + slot + u] = info[u].w;
+                    }
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                if (!kFull && slot + u >= cnt) continue;
+#pragma unroll
+                for (uint32_t p = 0; p < (kCounted ? 1u : kTileDigitsMax); ++p)
+                    if (p < ndig) atomicAdd(&digits[p][(t[u] >> (8u * p)) & 255u], 1u);
+            }
+        }
+    };
+    if (cnt == kCountedTile)
+        expand(std::true_type{});
+    else
+        expand(std::false_type{});
     __syncthreads();
     if constexpr (kCounted) {
         counted_finish(CountedWork(work, max_parts), nparts, part, digits[0][tid], wsum, s_last);
@@ -310,13 +345,12 @@ void launch_keygen(const KeygenArgs& a, int num_sms, cudaStream_t s) {
     const uint64_t cap = uint64_t(num_sms > 0 ? num_sms : 148) * uint64_t(per_sm);  // persistent
     const uint64_t blocks = parts < cap ? parts : cap;
     launch_dependent(scan_items_kernel, dim3(unsigned(blocks)), dim3(kScanItemsThreads), 0, s, a.splats, a.items,
-                     a.items_other, a.n_items, a.n, a.views, a.offsets, a.item_rects, a.item_slots, a.part_first,
-                     a.capacity, a.ranges, a.n_tiles, a.desc, a.ctl, a.spin_limit, a.never_publish);
+                     a.items_other, a.n_items, a.n, a.views, a.offsets, a.item_info, a.part_first, a.capacity,
+                     a.ranges, a.n_tiles, a.desc, a.ctl, a.spin_limit, a.never_publish);
     const uint32_t max_parts = std::max(1u, uint32_t((uint64_t(a.capacity) + kCountedTile - 1) / kCountedTile));
     launch_dependent(a.counted_work ? expand_keys_kernel<true> : expand_keys_kernel<false>, dim3(max_parts),
-                     dim3(kExpandThreads), 0, s, static_cast<const uint2*>(a.item_rects),
-                     static_cast<const uint2*>(a.item_slots), static_cast<const uint32_t*>(a.part_first), a.tiles,
-                     a.vals, a.n_items, a.capacity, max_parts, a.tile_bits, a.counted_work, a.ctl);
+                     dim3(kExpandThreads), 0, s, static_cast<const uint4*>(a.item_info),
+                     static_cast<const uint32_t*>(a.part_first), a.tiles, a.vals, a.n_items, a.capacity, max_parts, a.tile_bits, a.counted_work, a.ctl);
 }
 
 namespace {

@@ -7,9 +7,9 @@
 //
 // GB300 layout: a CTA of 128 threads owns 128 consecutive records (30,720 B).
 // The CTA stages them into shared memory with coalesced 16-byte asynchronous
-// copies (cp.async, 15 per thread), double-buffered so the next chunk streams
-// in while this one is projected; threads then read their record with
-// conflict-free 16-byte loads (record stride 60 words). The copies complete
+// copies (cp.async, 15 per thread) while other CTAs of the SM project theirs;
+// threads then read their record with conflict-free 16-byte loads (record
+// stride 60 words). The copies complete
 // by a hardware wait (cp.async.wait_group), not a software spin, so no wait
 // can give up with a copy in flight, and the CTA drains every copy it issued
 // before it exits. Besides the splat, each (view, Gaussian) gets a
@@ -20,6 +20,7 @@
 // k = 0..n-1; this file is compiled with --fmad=false so no product is fused
 // into an add.
 #include <algorithm>
+#include <cstddef>
 
 #include "tpd_common.cuh"
 #include "tpd_kernels.h"
@@ -103,17 +104,52 @@ __global__ void frame_begin_kernel(FrameCtl* ctl, const float* transforms, uint3
     }
 }
 
-// Reads float k of a record staged in shared memory.
+// A record staged in shared memory, read 16 bytes at a time: at a stride of
+// 60 words that is free of bank conflicts, a single word is not (lanes meet on
+// eight banks, four each).
 struct Rec {
     const float* p;
-    __device__ __forceinline__ float operator[](int k) const { return p[k]; }
     __device__ __forceinline__ float4 f4(int q) const { return reinterpret_cast<const float4*>(p)[q]; }
+};
+
+__device__ __forceinline__ void unpack4(float4 f, float* to) {
+    to[0] = f.x;
+    to[1] = f.y;
+    to[2] = f.z;
+    to[3] = f.w;
+}
+
+// The constants of a view that project_one uses, in registers (four 16-byte loads).
+struct ViewRegs {
+    float view[12];  // rows 0..2 of the view matrix
+    float focal[2];
+    uint32_t width, height;
+    __device__ __forceinline__ explicit ViewRegs(const ViewConst* v) {
+        const float4* p = reinterpret_cast<const float4*>(v);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) unpack4(__ldg(p + r), view + 4 * r);
+        const float4 f = __ldg(p + 8);
+        focal[0] = f.x;
+        focal[1] = f.y;
+        width = __float_as_uint(f.z);
+        height = __float_as_uint(f.w);
+    }
+};
+static_assert(offsetof(ViewConst, focal) == 128 && offsetof(ViewConst, width) == 136 && sizeof(ViewConst) % 16 == 0,
+              "ViewRegs reads focal, width and height as 16 bytes");
+
+// The 3D covariance of a Gaussian, which no view changes: computed at the
+// first view that keeps the Gaussian. (It is symmetric to the bit: element
+// (i, j) multiplies and adds the same factors in the same order as (j, i).)
+struct Covariance {
+    float c[6];
+    bool known;
 };
 
 // project() for one Gaussian. Returns the tile count (0 when culled) and fills
 // s.
-__device__ __forceinline__ uint32_t project_one(const Rec& rec, const float* em, const ViewConst& v,
-                                                uint32_t deg, bool compat, Splat& s) {
+__device__ __forceinline__ uint32_t project_one(const Rec& rec, const float* em, const ViewRegs& v,
+                                                uint32_t deg, bool compat, Covariance& cov, Splat& s) {
     s = Splat{0.f, 0.f, 0.f, 0u, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const float4 pos_op = rec.f4(0);
     const float mean[3] = {pos_op.x, pos_op.y, pos_op.z};
@@ -141,16 +177,26 @@ __device__ __forceinline__ uint32_t project_one(const Rec& rec, const float* em,
     const float fy = (0.5f * float(v.height)) * v.focal[1];
 
     // computeCovariance (volume.slang:20-41)
-    const float4 q = rec.f4(1), sc = rec.f4(2);
-    const float S[9] = {sc.x * sc.w, 0.f, 0.f, 0.f, sc.y * sc.w, 0.f, 0.f, 0.f, sc.z * sc.w};
-    const float x = q.x, y = q.y, z = q.z, w = q.w;
-    const float R[9] = {1.0f - 2.0f * (y * y + z * z), 2.0f * (x * y - w * z), 2.0f * (x * z + w * y),
-                        2.0f * (x * y + w * z), 1.0f - 2.0f * (x * x + z * z), 2.0f * (y * z - w * x),
-                        2.0f * (x * z - w * y), 2.0f * (y * z + w * x), 1.0f - 2.0f * (x * x + y * y)};
-    float sigma[9], sigmaT[9], cov3[9];
-    mat3mul(R, S, sigma);
-    mat3T(sigma, sigmaT);
-    mat3mul(sigma, sigmaT, cov3);
+    if (!cov.known) {
+        const float4 q = rec.f4(1), sc = rec.f4(2);
+        const float S[9] = {sc.x * sc.w, 0.f, 0.f, 0.f, sc.y * sc.w, 0.f, 0.f, 0.f, sc.z * sc.w};
+        const float x = q.x, y = q.y, z = q.z, w = q.w;
+        const float R[9] = {1.0f - 2.0f * (y * y + z * z), 2.0f * (x * y - w * z), 2.0f * (x * z + w * y),
+                            2.0f * (x * y + w * z), 1.0f - 2.0f * (x * x + z * z), 2.0f * (y * z - w * x),
+                            2.0f * (x * z - w * y), 2.0f * (y * z + w * x), 1.0f - 2.0f * (x * x + y * y)};
+        float sigma[9], sigmaT[9], full[9];
+        mat3mul(R, S, sigma);
+        mat3T(sigma, sigmaT);
+        mat3mul(sigma, sigmaT, full);
+        cov.c[0] = full[0];
+        cov.c[1] = full[1];
+        cov.c[2] = full[2];
+        cov.c[3] = full[4];
+        cov.c[4] = full[5];
+        cov.c[5] = full[8];
+        cov.known = true;
+    }
+    const float cov3[9] = {cov.c[0], cov.c[1], cov.c[2], cov.c[1], cov.c[3], cov.c[4], cov.c[2], cov.c[4], cov.c[5]};
 
     // projectCovariance + computeJacobian (volume.slang:44-63)
     const float W3[9] = {v.view[0], v.view[1], v.view[2], v.view[4], v.view[5],
@@ -196,36 +242,59 @@ __device__ __forceinline__ uint32_t project_one(const Rec& rec, const float* em,
     const float dx = d0 / len, dy = d1 / len, dz = d2 / len;
 
     // evaluateSphericalHarmonics (common.slang:35-80)
-    float res[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) res[c] = cSH_C0 * rec[12 + c];
+    // the basis first, then a channel at a time, so that one channel's
+    // coefficients are in registers
+    float B[16], s12 = 0.f;
     if (deg > 0) {
-        auto F = [&](int idx, int c) { return rec[12 + (idx - 1) + c * 15 + 3]; };
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            res[c] = res[c] - (cSH_C1 * dy) * F(1, c) + (cSH_C1 * dz) * F(2, c) - (cSH_C1 * dx) * F(3, c);
+        B[1] = cSH_C1 * dy;
+        B[2] = cSH_C1 * dz;
+        B[3] = cSH_C1 * dx;
         if (deg > 1) {
             const float xx = dx * dx, yy = dy * dy, zz = dz * dz, xy = dx * dy, yz = dy * dz, zx = dz * dx;
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                res[c] = res[c] + (cSH_C2[0] * xy) * F(4, c) + (cSH_C2[1] * yz) * F(5, c) +
-                         (cSH_C2[2] * (2.0f * zz - xx - yy)) * F(6, c) + (cSH_C2[3] * zx) * F(7, c) +
-                         (cSH_C2[4] * (xx - yy)) * F(8, c);
+            B[4] = cSH_C2[0] * xy;
+            B[5] = cSH_C2[1] * yz;
+            B[6] = cSH_C2[2] * (2.0f * zz - xx - yy);
+            B[7] = cSH_C2[3] * zx;
+            B[8] = cSH_C2[4] * (xx - yy);
             if (deg > 2) {
-                const float s12 = (cSH_C3[3] * dz) * (2.0f * zz - 3.0f * xx - 3.0f * yy);
+                B[9] = (cSH_C3[0] * dy) * (3.0f * xx - yy);
+                B[10] = (cSH_C3[1] * xy) * dz;
+                B[11] = (cSH_C3[2] * dy) * (4.0f * zz - xx - yy);
+                s12 = (cSH_C3[3] * dz) * (2.0f * zz - 3.0f * xx - 3.0f * yy);
+                B[13] = (cSH_C3[4] * dx) * (4.0f * zz - xx - yy);
+                B[14] = (cSH_C3[5] * dz) * (xx - yy);
+                B[15] = (cSH_C3[6] * dx) * (xx - 3.0f * yy);
+            }
+        }
+    }
+    float res[3], dc[4];
+    unpack4(rec.f4(3), dc);  // words 12..15: the three DC terms, the first channel's first coefficient
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    float r = res[c] + ((cSH_C3[0] * dy) * (3.0f * xx - yy)) * F(9, c) +
-                              ((cSH_C3[1] * xy) * dz) * F(10, c) +
-                              ((cSH_C3[2] * dy) * (4.0f * zz - xx - yy)) * F(11, c);
-                    if (compat) r = r + s12 + F(12, c);  // common.slang:69 as written
-                    else r = r + s12 * F(12, c);
-                    r = r + ((cSH_C3[4] * dx) * (4.0f * zz - xx - yy)) * F(13, c) +
-                        ((cSH_C3[5] * dz) * (xx - yy)) * F(14, c) + ((cSH_C3[6] * dx) * (xx - 3.0f * yy)) * F(15, c);
-                    res[c] = r;
+    for (int c = 0; c < 3; ++c) {
+        // the channel's 15 coefficients: words 15 + 15 c .. 29 + 15 c
+        constexpr int kFirst[3] = {3, 7, 11};  // the 16-byte piece holding the first of them
+        const int skip = 15 + 15 * c - 4 * kFirst[c];
+        float f[20] = {};
+        auto F = [&](int idx) { return f[skip + idx - 1]; };
+        float r = cSH_C0 * dc[c];
+        if (deg > 0) {
+            unpack4(rec.f4(kFirst[c]), f);
+            unpack4(rec.f4(kFirst[c] + 1), f + 4);
+            r = r - B[1] * F(1) + B[2] * F(2) - B[3] * F(3);
+            if (deg > 1) {
+                unpack4(rec.f4(kFirst[c] + 2), f + 8);
+                unpack4(rec.f4(kFirst[c] + 3), f + 12);
+                r = r + B[4] * F(4) + B[5] * F(5) + B[6] * F(6) + B[7] * F(7) + B[8] * F(8);
+                if (deg > 2) {
+                    if (c < 2) unpack4(rec.f4(kFirst[c] + 4), f + 16);
+                    r = r + B[9] * F(9) + B[10] * F(10) + B[11] * F(11);
+                    if (compat) r = r + s12 + F(12);  // common.slang:69 as written
+                    else r = r + s12 * F(12);
+                    r = r + B[13] * F(13) + B[14] * F(14) + B[15] * F(15);
                 }
             }
         }
+        res[c] = r;
     }
 
     s.r = fmaxf(res[0] + 0.5f, 0.0f);
@@ -243,21 +312,24 @@ __device__ __forceinline__ uint32_t project_one(const Rec& rec, const float* em,
     return touched;
 }
 
-// Persistent CTAs over chunks of kPreThreads records: while a chunk is
-// projected, the next chunk's records stream into the other shared-memory
-// stage (asynchronous 16-byte copies, one commit group per chunk), so HBM
-// reads overlap the arithmetic.
-constexpr uint32_t kPreStages = 2;
+// Persistent CTAs over chunks of kPreThreads records, kCtas of them per SM:
+// while some project, the records of others stream in (asynchronous 16-byte
+// copies; one stage per CTA, since two stages at three CTAs hold no more bytes
+// in flight but fewer warps). One view is bound by the record stream and the
+// splat stores, and four CTAs are enough (1M Gaussians 69 us, six 76); with
+// several views per record the projection's latency counts and six, the most
+// that shared memory holds, are faster (500,000 x 8 views 137 us, four 156;
+// 1.5M x 8 views of which few see a Gaussian 350 against 392).
 constexpr uint32_t kDepthPassesMax = 5;  // depth keys: 32 bits + log2(256 views)
 
 struct PreSmem {
-    float rec[kPreStages][kPreThreads * kRecordFloats];  // 30,720 B per stage, 16-byte multiple
+    float rec[kPreThreads * kRecordFloats];              // 30,720 B
     uint32_t hist[kDepthPassesMax][256];                  // depth-key digit counts of this CTA
     uint32_t kept;                                        // depth keys of visible items in this CTA
 };
 
-// (3 CTAs per SM fit in shared memory: registers up to 170 per thread are free)
-__global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessArgs a) {
+template <int kCtas>
+__global__ void __launch_bounds__(kPreThreads, kCtas) preprocess_kernel(PreprocessArgs a) {
     extern __shared__ __align__(128) unsigned char pre_smem[];
     PreSmem& S = *reinterpret_cast<PreSmem*>(pre_smem);
 
@@ -271,32 +343,27 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
     uint32_t kept = 0;  // this thread's visible items (the depth sort drops the others)
     const uint32_t nchunks = (a.n + kPreThreads - 1) / kPreThreads;
     const uint32_t npass = min(kDepthPassesMax, (a.depth_key_bits + 7) / 8);
-    // chunk's records into stage: piece q (16 bytes) by thread q % 128, so a
+    // chunk's records into shared memory: piece q (16 bytes) by thread q % 128, so a
     // warp's copies are 512 consecutive bytes; a record is 15 whole pieces
-    auto issue = [&](uint32_t chunk, uint32_t stage) {
+    auto issue = [&](uint32_t chunk) {
         const uint32_t base = chunk * kPreThreads;
         const uint32_t pieces = min(kPreThreads, a.n - base) * (kRecordBytes / 16u);
         const char* src = reinterpret_cast<const char*>(a.recs + size_t(base) * kRecordFloats);
-        char* dst = reinterpret_cast<char*>(S.rec[stage]);
+        char* dst = reinterpret_cast<char*>(S.rec);
         for (uint32_t q = tid; q < pieces; q += kPreThreads) cp_async16(dst + 16u * q, src + 16u * q);
     };
-    if (blockIdx.x < nchunks) issue(blockIdx.x, 0);
-    cp_async_commit();
-    uint32_t it = 0;
-    for (uint32_t chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x, ++it) {
-        const uint32_t stage = it & 1u;
-        // the other stage was released by the barrier that ended the last
-        // iteration; a commit group per iteration (empty after the last
-        // chunk) keeps "all but the newest group" = this chunk
-        if (chunk + gridDim.x < nchunks) issue(chunk + gridDim.x, stage ^ 1u);
+    for (uint32_t chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x) {
+        issue(chunk);
         cp_async_commit();
-        cp_async_wait_all_but_newest();  // this thread's pieces of the chunk have landed
-        __syncthreads();                 // and every other thread's
+        cp_async_wait_all();  // this thread's pieces of the chunk have landed
+        __syncthreads();      // and every other thread's
 
         const uint32_t base = chunk * kPreThreads;
         const uint32_t cnt = min(kPreThreads, a.n - base);
         const uint32_t i = base + tid;
         const uint32_t e = (tid < cnt && a.ent_idx) ? a.ent_idx[i] : 0u;
+        Covariance cov;
+        cov.known = false;
         for (uint32_t v = 0; v < a.n_views; ++v) {
             Splat sp;
             uint32_t tiles = 0;
@@ -304,9 +371,10 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
                 const float* em = a.ent_mats + (size_t(v) * a.n_ent + e) * kEntityMatFloats;
                 float emr[kEntityMatFloats];
 #pragma unroll
-                for (int k = 0; k < kEntityMatFloats; ++k) emr[k] = __ldg(em + k);
-                tiles = project_one(Rec{S.rec[stage] + tid * kRecordFloats}, emr, a.views[v], a.sh_degree,
-                                    a.band3_compat != 0, sp);
+                for (int k = 0; k < kEntityMatFloats / 4; ++k)
+                    unpack4(__ldg(reinterpret_cast<const float4*>(em) + k), emr + 4 * k);
+                tiles = project_one(Rec{S.rec + tid * kRecordFloats}, emr, ViewRegs(a.views + v), a.sh_degree,
+                                    a.band3_compat != 0, cov, sp);
             } else {
                 sp = Splat{0.f, 0.f, 0.f, 0u, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             }
@@ -332,9 +400,8 @@ __global__ void __launch_bounds__(kPreThreads, 3) preprocess_kernel(PreprocessAr
                 }
             }
         }
-        __syncthreads();  // every thread is done with this stage before it is refilled
+        __syncthreads();  // every thread is done with the records before they are replaced
     }
-    cp_async_wait_all();  // nothing is left in flight (the last groups are empty)
     if (!a.depth_keys) return;
     kept = warp_sum(kept);
     if ((tid & 31u) == 0 && kept) atomicAdd(&S.kept, kept);
@@ -439,22 +506,30 @@ void launch_frame_begin(FrameCtl* ctl, const float* transforms, uint32_t n_ent, 
 }
 
 namespace {
-// The shared-memory opt-in (PreSmem is above 48 KB) and the resident CTAs per
-// SM, for the current device.
+// The resident CTAs per SM, for the current device.
+template <int kCtas>
 int preprocess_setup() {
-    cudaFuncSetAttribute(preprocess_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(PreSmem)));
     int r = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, preprocess_kernel, kPreThreads, sizeof(PreSmem));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, preprocess_kernel<kCtas>, kPreThreads, sizeof(PreSmem));
     return r > 0 ? r : 1;
+}
+
+template <int kCtas>
+void launch_preprocess_t(const PreprocessArgs& a, int num_sms, cudaStream_t s) {
+    static_assert(sizeof(PreSmem) <= 48 * 1024, "no shared-memory opt-in");
+    const int per_sm = device_once(preprocess_setup<kCtas>);
+    const uint32_t chunks = (a.n + kPreThreads - 1) / kPreThreads;
+    const uint32_t blocks = std::min<uint32_t>(chunks, uint32_t((num_sms > 0 ? num_sms : 148) * per_sm));
+    launch_dependent(preprocess_kernel<kCtas>, dim3(blocks), dim3(kPreThreads), sizeof(PreSmem), s, a);
 }
 }  // namespace
 
 void launch_preprocess(const PreprocessArgs& a, int num_sms, cudaStream_t s) {
     if (a.n == 0 || a.n_views == 0) return;
-    const int per_sm = device_once(preprocess_setup);
-    const uint32_t chunks = (a.n + kPreThreads - 1) / kPreThreads;
-    const uint32_t blocks = std::min<uint32_t>(chunks, uint32_t((num_sms > 0 ? num_sms : 148) * per_sm));
-    launch_dependent(preprocess_kernel, dim3(blocks), dim3(kPreThreads), sizeof(PreSmem), s, a);
+    if (a.n_views > 1)
+        launch_preprocess_t<6>(a, num_sms, s);
+    else
+        launch_preprocess_t<4>(a, num_sms, s);
 }
 
 void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint64_t* desc, FrameCtl* ctl,

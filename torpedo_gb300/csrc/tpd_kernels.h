@@ -105,11 +105,10 @@ struct KeygenArgs {
     uint32_t n;                   // Gaussians per view
     const ViewConst* views;
     uint32_t* offsets;            // n_items
-    uint2* item_rects;            // n_items: scratch between the two kernels
-    uint2* item_slots;            // n_items: scratch between the two kernels
+    uint4* item_info;             // n_items: scratch between the two kernels
     uint32_t* part_first;         // ceil(capacity / 4096): scratch between the two kernels
-    uint32_t* tiles;              // capacity
-    uint32_t* vals;               // capacity
+    uint32_t* tiles;              // capacity, 16-byte aligned
+    uint32_t* vals;               // capacity, 16-byte aligned
     uint32_t capacity;
     uint32_t* ranges;
     uint32_t n_tiles;
