@@ -10,8 +10,9 @@
 //   Sigma   = (R S)(R S)^T, R from the quaternion as stored (not normalised),
 //             S = diag(exp(log_scale) * modifier)
 //   opacity = sigmoid(logit)
-// One thread per Gaussian loops over views, so gradients of the batched
-// form accumulate in registers and are written once (no atomics).
+// Two threads per Gaussian, one for the colour's adjoint and one for the
+// others', loop over the views, so gradients of the batched form accumulate in
+// registers and are written once (no atomics).
 #include "tpd_common.cuh"
 #include "tpd_kernels.h"
 
@@ -50,145 +51,199 @@ __device__ __forceinline__ void sh_basis(int k, float x, float y, float z, float
     }
 }
 
-constexpr uint32_t kBwdThreads = 128;
+constexpr uint32_t kBwdThreads = 128;  // Gaussians per CTA
 
-// A block's records are staged into shared memory with coalesced 16-byte
-// loads (a record is 240 B, so thread-per-record loads would stride), and its
-// SH gradients leave through the same buffer as coalesced 16-byte stores.
-__global__ void __launch_bounds__(kBwdThreads) preprocess_backward_kernel(PreprocessBackwardArgs a) {
-    __shared__ __align__(16) float srec[kBwdThreads * kRecordFloats];  // 30 KB; reused for the SH gradients
-    pdl_wait();  // launched as a dependent of the stream's previous kernel: its output is read below
-    pdl_trigger();
-    const uint32_t base = blockIdx.x * kBwdThreads;
-    const uint32_t cnt = min(kBwdThreads, a.n - base);
-    {
-        const float4* src = reinterpret_cast<const float4*>(a.recs + size_t(base) * kRecordFloats);
-        float4* dst = reinterpret_cast<float4*>(srec);
-        for (uint32_t k = threadIdx.x; k < cnt * (kRecordFloats / 4); k += kBwdThreads) dst[k] = src[k];
+__device__ __forceinline__ void unpack4(float4 f, float* to) {
+    to[0] = f.x;
+    to[1] = f.y;
+    to[2] = f.z;
+    to[3] = f.w;
+}
+
+// The Gaussian of a thread and its views' data.
+struct Item {
+    const PreprocessBackwardArgs& a;
+    uint32_t i, e;      // Gaussian, entity
+    bool active;
+    const float* rec;   // its record in shared memory, 16-byte aligned
+    __device__ __forceinline__ float radius(uint32_t v) const {
+        return active && v < a.n_views ? a.splats[size_t(v) * a.n + i].radius : 0.0f;
     }
-    __syncthreads();
-    const uint32_t i = base + threadIdx.x;
-    const bool active = threadIdx.x < cnt;
-    const float* rec = srec + threadIdx.x * kRecordFloats;
-    if (!active) rec = srec;  // any staged record: results of inactive threads are not stored
-    const float m[3] = {rec[0], rec[1], rec[2]};
-    const float op = rec[3];
-    const float qx = rec[4], qy = rec[5], qz = rec[6], qw = rec[7];
-    const float s[3] = {rec[8] * rec[11], rec[9] * rec[11], rec[10] * rec[11]};
-    const uint32_t e = (a.ent_idx && active) ? a.ent_idx[i] : 0u;
-    const int nf = a.sh_degree >= 3 ? 15 : a.sh_degree == 2 ? 8 : a.sh_degree == 1 ? 3 : 0;
-    const bool compat = a.band3_compat != 0;
+    __device__ __forceinline__ const float4* splat(uint32_t v) const {
+        return reinterpret_cast<const float4*>(a.splats + size_t(v) * a.n + i);
+    }
+    __device__ __forceinline__ const float4* g2d(uint32_t v) const {
+        return reinterpret_cast<const float4*>(a.g2d + (size_t(v) * a.n + i) * kG2DStride);
+    }
+    __device__ __forceinline__ float4 f4(int q) const { return reinterpret_cast<const float4*>(rec)[q]; }
+};
 
-    // R and M = R S are view independent
-    const float R[9] = {1.f - 2.f * (qy * qy + qz * qz), 2.f * (qx * qy - qw * qz), 2.f * (qx * qz + qw * qy),
-                        2.f * (qx * qy + qw * qz), 1.f - 2.f * (qx * qx + qz * qz), 2.f * (qy * qz - qw * qx),
-                        2.f * (qx * qz - qw * qy), 2.f * (qy * qz + qw * qx), 1.f - 2.f * (qx * qx + qy * qy)};
-    float M[9], Sig[9];
+// Walks the views that the item is in. A view's radius (0: not in it) is
+// loaded two views ahead and, where it is not 0, load(v) one view ahead, so a
+// view without the Gaussian costs four bytes and the loads of one with it
+// overlap the work on the view before. take() moves what was loaded to the
+// work's registers. (Each lane walking only its own views measured slower: the
+// views' constants are then loaded per lane.)
+template <typename Load, typename Take, typename Work>
+__device__ __forceinline__ void for_each_view(const Item& it, Load load, Take take, Work work) {
+    float next = it.radius(0), next2 = it.radius(1);
+    if (next > 0.0f) load(0u);
+    for (uint32_t v = 0; v < it.a.n_views; ++v) {
+        const float radius = next;
+        take();
+        next = next2;
+        if (next > 0.0f) load(v + 1u);
+        next2 = it.radius(v + 2u);
+        if (radius > 0.0f) work(v);
+    }
+}
+
+// The colour half: dL/dcolour -> SH coefficients gsh and, through the view
+// direction, the mean (gm).
+__device__ __forceinline__ void colour_adjoint(const Item& it, float (&gsh)[48], float (&gm)[3]) {
+    const int nf = it.a.sh_degree >= 3 ? 15 : it.a.sh_degree == 2 ? 8 : it.a.sh_degree == 1 ? 3 : 0;
+    const bool compat = it.a.band3_compat != 0;
+    const float4 mo = it.f4(0);
+    float4 n_c = make_float4(0.f, 0.f, 0.f, 0.f), n_g1 = n_c, col = n_c, g1 = n_c;
+    float n_g8 = 0.f, g8 = 0.f;
+    auto load = [&](uint32_t v) {
+        n_c = it.splat(v)[0];
+        n_g1 = it.g2d(v)[1];
+        n_g8 = it.g2d(v)[2].x;
+    };
+    auto take = [&]() {
+        col = n_c;
+        g1 = n_g1;
+        g8 = n_g8;
+    };
+    for_each_view(it, load, take, [&](uint32_t v) {
+        const float graw[3] = {col.x > 0.f ? g1.z : 0.f, col.y > 0.f ? g1.w : 0.f, col.z > 0.f ? g8 : 0.f};
+        float V[12];
+        const float4* p = reinterpret_cast<const float4*>(it.a.views + v);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) unpack4(__ldg(p + r), V + 4 * r);
+        const float d0 = mo.x + (V[0] * V[3] + V[4] * V[7] + V[8] * V[11]);  // mean - camera position
+        const float d1 = mo.y + (V[1] * V[3] + V[5] * V[7] + V[9] * V[11]);
+        const float d2 = mo.z + (V[2] * V[3] + V[6] * V[7] + V[10] * V[11]);
+        const float inv_len = 1.0f / sqrtf(d0 * d0 + d1 * d1 + d2 * d2);
+        const float x = d0 * inv_len, y = d1 * inv_len, z = d2 * inv_len;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) gsh[c] += graw[c] * SH_C0;
+        // dL/ddir through feature k: its three coefficients weighted by the
+        // colour gradient, times the basis function's gradient
+        float wk[16], gd0 = 0.f, gd1 = 0.f, gd2 = 0.f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            // the channel's coefficients: words 15 + 15 c .. 29 + 15 c of the record
+            constexpr int kFirst[3] = {3, 7, 11};  // the 16-byte piece holding the first of them
+            float f[20];
+#pragma unroll
+            for (int q = 0; q < (c < 2 ? 5 : 4); ++q) unpack4(it.f4(kFirst[c] + q), f + 4 * q);
+#pragma unroll
+            for (int k = 1; k <= 15; ++k) {
+                const float t = f[15 + 15 * c - 4 * kFirst[c] + k - 1];
+                wk[k] = c == 0 ? graw[0] * t : wk[k] + graw[c] * t;
+            }
+        }
+        if (compat) wk[12] = graw[0] + graw[1] + graw[2];  // added, not multiplied, in the forward
+#pragma unroll
+        for (int k = 1; k <= 15; ++k) {
+            if (k > nf) break;
+            float b, b0, b1, b2;
+            sh_basis(k, x, y, z, b, b0, b1, b2);
+            if (k == 12 && compat) b = 1.0f;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) gsh[3 + c * 15 + (k - 1)] += graw[c] * b;
+            gd0 += wk[k] * b0;
+            gd1 += wk[k] * b1;
+            gd2 += wk[k] * b2;
+        }
+        const float dd = x * gd0 + y * gd1 + z * gd2;
+        gm[0] += (gd0 - x * dd) * inv_len;
+        gm[1] += (gd1 - y * dd) * inv_len;
+        gm[2] += (gd2 - z * dd) * inv_len;
+    });
+}
+
+// R from the quaternion as stored, M = R S.
+__device__ __forceinline__ void rotation_scale(const float4 q, const float4 sc, float (&R)[9], float (&s)[3], float (&M)[9]) {
+    const float qx = q.x, qy = q.y, qz = q.z, qw = q.w;
+    R[0] = 1.f - 2.f * (qy * qy + qz * qz);
+    R[1] = 2.f * (qx * qy - qw * qz);
+    R[2] = 2.f * (qx * qz + qw * qy);
+    R[3] = 2.f * (qx * qy + qw * qz);
+    R[4] = 1.f - 2.f * (qx * qx + qz * qz);
+    R[5] = 2.f * (qy * qz - qw * qx);
+    R[6] = 2.f * (qx * qz - qw * qy);
+    R[7] = 2.f * (qy * qz + qw * qx);
+    R[8] = 1.f - 2.f * (qx * qx + qy * qy);
+    s[0] = sc.x * sc.w;
+    s[1] = sc.y * sc.w;
+    s[2] = sc.z * sc.w;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
         for (int c = 0; c < 3; ++c) M[r * 3 + c] = R[r * 3 + c] * s[c];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) Sig[r * 3 + c] = M[r * 3 + 0] * M[c * 3 + 0] + M[r * 3 + 1] * M[c * 3 + 1] + M[r * 3 + 2] * M[c * 3 + 2];
+}
 
-    float gm[3] = {0.f, 0.f, 0.f}, gSigAcc[9];
+// The shape half: dL/d(px, py, conic, opacity) -> opacity logit, mean (gm),
+// and dL/dSigma + its transpose (gsig: elements (0,0), (0,1), (0,2), (1,1),
+// (1,2), (2,2)), which is all that is used of it.
+__device__ __forceinline__ void shape_adjoint(const Item& it, float& glogit, float (&gm)[3], float (&gsig)[6]) {
+    const float4 mo = it.f4(0);
+    const float m[3] = {mo.x, mo.y, mo.z}, op = mo.w;
+    float Sig[9];
+    {
+        float R[9], s[3], M[9];
+        rotation_scale(it.f4(1), it.f4(2), R, s, M);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) gSigAcc[k] = 0.f;
-    float glogit = 0.f;
-    float gsh[48];
+        for (int r = 0; r < 3; ++r)
 #pragma unroll
-    for (int k = 0; k < 48; ++k) gsh[k] = 0.f;
-
-    // the splat (colour, tiles | texel | conic, opacity) and its gradient
-    // record of view v, 16 bytes at a time; view v + 1's are loaded while
-    // view v is worked on (a gradient record is read whether or not the
-    // Gaussian is visible in that view: it is zero then)
-    float4 n_c, n_t, n_g0, n_g1, n_g2;
-    auto load_view = [&](uint32_t v) {
-        const float4* sp4 = reinterpret_cast<const float4*>(a.splats + size_t(v) * a.n + i);
-        n_c = sp4[0];
-        n_t = sp4[1];
-        const float4* g4 = reinterpret_cast<const float4*>(a.g2d + (size_t(v) * a.n + i) * kG2DStride);
-        n_g0 = g4[0];
-        n_g1 = g4[1];
-        n_g2 = g4[2];
+            for (int c = 0; c < 3; ++c)
+                Sig[r * 3 + c] = M[r * 3 + 0] * M[c * 3 + 0] + M[r * 3 + 1] * M[c * 3 + 1] + M[r * 3 + 2] * M[c * 3 + 2];
+    }
+    float4 n_g0 = make_float4(0.f, 0.f, 0.f, 0.f), n_g1 = n_g0, g0 = n_g0, g1 = n_g0;
+    auto load = [&](uint32_t v) {
+        n_g0 = it.g2d(v)[0];
+        n_g1 = it.g2d(v)[1];
     };
-    if (active && a.n_views) load_view(0);
-    for (uint32_t v = 0; v < a.n_views && active; ++v) {
-        const float4 sp_c = n_c, sp_t = n_t, ga4 = n_g0, gb4 = n_g1, gc4 = n_g2;
-        if (v + 1 < a.n_views) load_view(v + 1);
-        if (!(sp_t.w > 0.0f)) continue;
-        const float g[9] = {ga4.x, ga4.y, ga4.z, ga4.w, gb4.x, gb4.y, gb4.z, gb4.w, gc4.x};
-        const ViewConst& vc = a.views[v];
-        const float* em = a.ent_mats + (size_t(v) * a.n_ent + e) * kEntityMatFloats;
+    auto take = [&]() {
+        g0 = n_g0;
+        g1 = n_g1;
+    };
+    for_each_view(it, load, take, [&](uint32_t v) {
+        const float gpx = g0.x, gpy = g0.y, gA = g0.z, gB = g0.w, gC = g1.x, gop = g1.y;
+        // the view's constants and the entity's matrices, 16 bytes at a time
+        float V[12], em[kEntityMatFloats];
+        const float4* p = reinterpret_cast<const float4*>(it.a.views + v);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) unpack4(__ldg(p + r), V + 4 * r);
+        const float4 f = __ldg(p + 8);  // focal, width, height
+        const float Wd = float(__float_as_uint(f.z)), Hd = float(__float_as_uint(f.w));
+        const float fxp = 0.5f * Wd * f.x, fyp = 0.5f * Hd * f.y;
+        const float4* m4 =
+            reinterpret_cast<const float4*>(it.a.ent_mats + (size_t(v) * it.a.n_ent + it.e) * kEntityMatFloats);
+#pragma unroll
+        for (int k = 0; k < kEntityMatFloats / 4; ++k) unpack4(__ldg(m4 + k), em + 4 * k);
         float vp[3], cp[4];
 #pragma unroll
         for (int r = 0; r < 3; ++r) vp[r] = em[r * 4] * m[0] + em[r * 4 + 1] * m[1] + em[r * 4 + 2] * m[2] + em[r * 4 + 3];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
             cp[r] = em[12 + r * 4] * m[0] + em[12 + r * 4 + 1] * m[1] + em[12 + r * 4 + 2] * m[2] + em[12 + r * 4 + 3];
-        const float Wd = float(vc.width), Hd = float(vc.height);
-        const float fxp = 0.5f * Wd * vc.focal[0], fyp = 0.5f * Hd * vc.focal[1];
 
-        // opacity
-        glogit += g[5] * op * (1.f - op);
-
-        // colour -> SH coefficients and view direction
-        float campos[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            campos[k] = -(vc.view[k] * vc.view[3] + vc.view[4 + k] * vc.view[7] + vc.view[8 + k] * vc.view[11]);
-        const float d0 = m[0] - campos[0], d1 = m[1] - campos[1], d2 = m[2] - campos[2];
-        const float vlen = sqrtf(d0 * d0 + d1 * d1 + d2 * d2);
-        const float x = d0 / vlen, y = d1 / vlen, z = d2 / vlen;
-        const float col[3] = {sp_c.x, sp_c.y, sp_c.z};
-        float graw[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) graw[c] = col[c] > 0.f ? g[6 + c] : 0.f;
-        float gd0 = 0.f, gd1 = 0.f, gd2 = 0.f;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) gsh[c] += graw[c] * SH_C0;
-#pragma unroll
-        for (int k = 1; k <= 15; ++k) {
-            if (k > nf) break;
-            float b, b0, b1, b2;
-            sh_basis(k, x, y, z, b, b0, b1, b2);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const int slot = 3 + c * 15 + (k - 1);
-                if (k == 12 && compat) {
-                    gsh[slot] += graw[c];
-                    gd0 += graw[c] * b0;
-                    gd1 += graw[c] * b1;
-                    gd2 += graw[c] * b2;
-                } else {
-                    const float coef = rec[12 + slot];
-                    gsh[slot] += graw[c] * b;
-                    gd0 += graw[c] * coef * b0;
-                    gd1 += graw[c] * coef * b1;
-                    gd2 += graw[c] * coef * b2;
-                }
-            }
-        }
-        const float dd = x * gd0 + y * gd1 + z * gd2;
-        gm[0] += (gd0 - x * dd) / vlen;
-        gm[1] += (gd1 - y * dd) / vlen;
-        gm[2] += (gd2 - z * dd) / vlen;
+        glogit += gop * op * (1.f - op);
 
         // pixel position -> clip -> mean
-        const float w = cp[3];
-        const float gcp[4] = {g[0] * Wd / (2.f * w), g[1] * Hd / (2.f * w), 0.f,
-                              -(g[0] * Wd * cp[0] + g[1] * Hd * cp[1]) / (2.f * w * w)};
+        const float iw = 1.0f / cp[3];
+        const float gc0 = gpx * Wd * (0.5f * iw), gc1 = gpy * Hd * (0.5f * iw);
+        const float gc3 = -(gc0 * cp[0] + gc1 * cp[1]) * iw;
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
-            gm[d] += em[12 + 0 * 4 + d] * gcp[0] + em[12 + 1 * 4 + d] * gcp[1] + em[12 + 3 * 4 + d] * gcp[3];
+        for (int d = 0; d < 3; ++d) gm[d] += em[12 + 0 * 4 + d] * gc0 + em[12 + 1 * 4 + d] * gc1 + em[12 + 3 * 4 + d] * gc3;
 
         // 2D covariance
-        const float vz = vp[2];
-        const float J0 = fxp / vz, J2 = -fxp * vp[0] / (vz * vz), J4 = fyp / vz, J5 = -fyp * vp[1] / (vz * vz);
-        const float* V = vc.view;
+        const float ivz = 1.0f / vp[2];
+        const float J0 = fxp * ivz, J4 = fyp * ivz, J2 = -J0 * vp[0] * ivz, J5 = -J4 * vp[1] * ivz;
         float Tm[6];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -206,16 +261,19 @@ __global__ void __launch_bounds__(kBwdThreads) preprocess_backward_kernel(Prepro
         const float cc = TS[3] * Tm[3] + TS[4] * Tm[4] + TS[5] * Tm[5] + 0.3f;
         const float det = ca * cc - cb * cb;
         const float idet2 = 1.f / (det * det);
-        const float gA = g[2], gB = g[3], gC = g[4];
         const float ga = (-gA * cc * cc + gB * cb * cc - gC * cb * cb) * idet2;
         const float gb = (2.f * gA * cb * cc - gB * (ca * cc + cb * cb) + 2.f * gC * ca * cb) * idet2;
         const float gc = (-gA * cb * cb + gB * ca * cb - gC * ca * ca) * idet2;
         // G = [[ga, 0], [gb, gc]]: dL/dSig = T^T G T, dL/dT = (G + G^T) T Sig
+        {
+            int k = 0;
 #pragma unroll
-        for (int r = 0; r < 3; ++r)
+            for (int r = 0; r < 3; ++r)
 #pragma unroll
-            for (int c = 0; c < 3; ++c)
-                gSigAcc[r * 3 + c] += Tm[r] * (ga * Tm[c]) + Tm[3 + r] * (gb * Tm[c] + gc * Tm[3 + c]);
+                for (int c = r; c < 3; ++c, ++k)
+                    gsig[k] += 2.f * ga * Tm[r] * Tm[c] + 2.f * gc * Tm[3 + r] * Tm[3 + c] +
+                               gb * (Tm[3 + r] * Tm[c] + Tm[3 + c] * Tm[r]);
+        }
         float gT[6];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -223,80 +281,114 @@ __global__ void __launch_bounds__(kBwdThreads) preprocess_backward_kernel(Prepro
             gT[3 + c] = gb * TS[c] + 2.f * gc * TS[3 + c];
         }
         // T = J W: dL/dJ = dL/dT W^T (only J0, J2, J4, J5 are non-zero functions of vp)
-        float gJ[6];
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                gJ[r * 3 + c] = gT[r * 3 + 0] * V[c * 4 + 0] + gT[r * 3 + 1] * V[c * 4 + 1] + gT[r * 3 + 2] * V[c * 4 + 2];
-        const float ivz2 = 1.f / (vz * vz), ivz3 = ivz2 / vz;
-        const float gvp0 = gJ[2] * (-fxp * ivz2);
-        const float gvp1 = gJ[5] * (-fyp * ivz2);
-        const float gvp2 = gJ[0] * (-fxp * ivz2) + gJ[2] * (2.f * fxp * vp[0] * ivz3) + gJ[4] * (-fyp * ivz2) +
-                           gJ[5] * (2.f * fyp * vp[1] * ivz3);
+        const float gJ0 = gT[0] * V[0] + gT[1] * V[1] + gT[2] * V[2];
+        const float gJ2 = gT[0] * V[8] + gT[1] * V[9] + gT[2] * V[10];
+        const float gJ4 = gT[3] * V[4] + gT[4] * V[5] + gT[5] * V[6];
+        const float gJ5 = gT[3] * V[8] + gT[4] * V[9] + gT[5] * V[10];
+        // J0 = fx / z, J2 = -fx x / z^2, J4 = fy / z, J5 = -fy y / z^2
+        const float gvp0 = -gJ2 * J0 * ivz;
+        const float gvp1 = -gJ5 * J4 * ivz;
+        const float gvp2 = -(gJ0 * J0 + 2.f * gJ2 * J2 + gJ4 * J4 + 2.f * gJ5 * J5) * ivz;
 #pragma unroll
         for (int d = 0; d < 3; ++d) gm[d] += em[0 * 4 + d] * gvp0 + em[1 * 4 + d] * gvp1 + em[2 * 4 + d] * gvp2;
-    }
+    });
+}
 
-    // Sigma = M M^T, M = R S
-    float gM[9];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            gM[r * 3 + c] = (gSigAcc[r * 3 + 0] + gSigAcc[0 * 3 + r]) * M[0 * 3 + c] +
-                            (gSigAcc[r * 3 + 1] + gSigAcc[1 * 3 + r]) * M[1 * 3 + c] +
-                            (gSigAcc[r * 3 + 2] + gSigAcc[2 * 3 + r]) * M[2 * 3 + c];
-    float gR[9];
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) gR[r * 3 + c] = gM[r * 3 + c] * s[c];
-    float gq[4], glsv[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) glsv[c] = (gM[0 * 3 + c] * R[0 * 3 + c] + gM[1 * 3 + c] * R[1 * 3 + c] + gM[2 * 3 + c] * R[2 * 3 + c]) * s[c];
-    gq[0] = gR[1] * 2.f * qy + gR[2] * 2.f * qz + gR[3] * 2.f * qy + gR[4] * (-4.f * qx) + gR[5] * (-2.f * qw) +
-            gR[6] * 2.f * qz + gR[7] * 2.f * qw + gR[8] * (-4.f * qx);
-    gq[1] = gR[0] * (-4.f * qy) + gR[1] * 2.f * qx + gR[2] * 2.f * qw + gR[3] * 2.f * qx + gR[5] * 2.f * qz +
-            gR[6] * (-2.f * qw) + gR[7] * 2.f * qz + gR[8] * (-4.f * qy);
-    gq[2] = gR[0] * (-4.f * qz) + gR[1] * (-2.f * qw) + gR[2] * 2.f * qx + gR[3] * 2.f * qw + gR[4] * (-4.f * qz) +
-            gR[5] * 2.f * qy + gR[6] * 2.f * qx + gR[7] * 2.f * qy;
-    gq[3] = gR[1] * (-2.f * qz) + gR[2] * 2.f * qy + gR[3] * 2.f * qz + gR[5] * (-2.f * qx) + gR[6] * (-2.f * qy) +
-            gR[7] * 2.f * qx;
-    if (active) {
-        float* gls = a.g_log_scales + size_t(i) * 3;
-        gls[0] = glsv[0];
-        gls[1] = glsv[1];
-        gls[2] = glsv[2];
-        if ((reinterpret_cast<uintptr_t>(a.g_quats) & 15u) == 0) {
-            reinterpret_cast<float4*>(a.g_quats)[i] = make_float4(gq[0], gq[1], gq[2], gq[3]);
-        } else {
-            float* gqo = a.g_quats + size_t(i) * 4;
-            gqo[0] = gq[0];
-            gqo[1] = gq[1];
-            gqo[2] = gq[2];
-            gqo[3] = gq[3];
-        }
+// A barrier of the whole CTA that its two halves reach in their own code (a
+// barrier resource of its own: bar.sync counts arrivals, wherever they come from).
+__device__ __forceinline__ void records_done() {
+    asm volatile("bar.sync 1, %0;" ::"n"(2 * kBwdThreads) : "memory");
+}
+
+// A CTA of 256 threads for 128 Gaussians: the first four warps take the colour
+// half of each, the other four the shape half. One thread for both held 168
+// registers, three CTAs of four warps per SM, and waited on its own chains
+// (issue on 40% of the cycles). 8 views of 500,000: 276 -> 184 us, of 1.5M of
+// which few are in a view 655 -> 527. Three CTAs per SM spill (222 us).
+// Its records are staged into shared memory with coalesced 16-byte loads (a
+// record is 240 B, so thread-per-record loads would stride), and its SH
+// gradients leave through the same buffer as coalesced 16-byte stores.
+__global__ void __launch_bounds__(2 * kBwdThreads, 2) preprocess_backward_kernel(PreprocessBackwardArgs a) {
+    __shared__ __align__(16) float srec[kBwdThreads * kRecordFloats];  // 30 KB; reused for the SH gradients
+    __shared__ float sgm[3][kBwdThreads];                              // the colour half's mean gradients
+    pdl_wait();  // launched as a dependent of the stream's previous kernel: its output is read below
+    pdl_trigger();
+    const uint32_t base = blockIdx.x * kBwdThreads;
+    const uint32_t cnt = min(kBwdThreads, a.n - base);
+    {
+        const float4* src = reinterpret_cast<const float4*>(a.recs + size_t(base) * kRecordFloats);
+        float4* dst = reinterpret_cast<float4*>(srec);
+        for (uint32_t k = threadIdx.x; k < cnt * (kRecordFloats / 4); k += 2 * kBwdThreads) dst[k] = src[k];
     }
-    __syncthreads();  // every thread is done with the staged records
-    if (active) {
-        float* gmo = a.g_means + size_t(i) * 3;
-        gmo[0] = gm[0];
-        gmo[1] = gm[1];
-        gmo[2] = gm[2];
-        a.g_logits[i] = glogit;
-        float4* mine = reinterpret_cast<float4*>(srec + threadIdx.x * 48);
+    __syncthreads();
+    const uint32_t t = threadIdx.x % kBwdThreads, i = base + t;
+    const bool active = t < cnt;
+    const Item it{a, i, (a.ent_idx && active) ? a.ent_idx[i] : 0u, active, srec + (active ? t : 0u) * kRecordFloats};
+    if (threadIdx.x < kBwdThreads) {
+        float gsh[48], gm[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-        for (int k = 0; k < 12; ++k) mine[k] = make_float4(gsh[4 * k], gsh[4 * k + 1], gsh[4 * k + 2], gsh[4 * k + 3]);
+        for (int k = 0; k < 48; ++k) gsh[k] = 0.f;
+        colour_adjoint(it, gsh, gm);
+        sgm[0][t] = gm[0];
+        sgm[1][t] = gm[1];
+        sgm[2][t] = gm[2];
+        records_done();
+        if (active) {
+            float4* mine = reinterpret_cast<float4*>(srec + t * 48);
+#pragma unroll
+            for (int k = 0; k < 12; ++k) mine[k] = make_float4(gsh[4 * k], gsh[4 * k + 1], gsh[4 * k + 2], gsh[4 * k + 3]);
+        }
+    } else {
+        float glogit = 0.f, gm[3] = {0.f, 0.f, 0.f}, gsig[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        shape_adjoint(it, glogit, gm, gsig);
+        // Sigma = M M^T, M = R S
+        const float4 q = it.f4(1);
+        float R[9], s[3], M[9], gM[9], gR[9];
+        rotation_scale(q, it.f4(2), R, s, M);
+        const float gS[9] = {gsig[0], gsig[1], gsig[2], gsig[1], gsig[3], gsig[4], gsig[2], gsig[4], gsig[5]};
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                gM[r * 3 + c] = gS[r * 3 + 0] * M[0 * 3 + c] + gS[r * 3 + 1] * M[1 * 3 + c] + gS[r * 3 + 2] * M[2 * 3 + c];
+                gR[r * 3 + c] = gM[r * 3 + c] * s[c];
+            }
+        const float qx = q.x, qy = q.y, qz = q.z, qw = q.w;
+        float gq[4], gls[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) gls[c] = (gM[0 * 3 + c] * R[0 * 3 + c] + gM[1 * 3 + c] * R[1 * 3 + c] + gM[2 * 3 + c] * R[2 * 3 + c]) * s[c];
+        gq[0] = gR[1] * 2.f * qy + gR[2] * 2.f * qz + gR[3] * 2.f * qy + gR[4] * (-4.f * qx) + gR[5] * (-2.f * qw) +
+                gR[6] * 2.f * qz + gR[7] * 2.f * qw + gR[8] * (-4.f * qx);
+        gq[1] = gR[0] * (-4.f * qy) + gR[1] * 2.f * qx + gR[2] * 2.f * qw + gR[3] * 2.f * qx + gR[5] * 2.f * qz +
+                gR[6] * (-2.f * qw) + gR[7] * 2.f * qz + gR[8] * (-4.f * qy);
+        gq[2] = gR[0] * (-4.f * qz) + gR[1] * (-2.f * qw) + gR[2] * 2.f * qx + gR[3] * 2.f * qw + gR[4] * (-4.f * qz) +
+                gR[5] * 2.f * qy + gR[6] * 2.f * qx + gR[7] * 2.f * qy;
+        gq[3] = gR[1] * (-2.f * qz) + gR[2] * 2.f * qy + gR[3] * 2.f * qz + gR[5] * (-2.f * qx) + gR[6] * (-2.f * qy) +
+                gR[7] * 2.f * qx;
+        records_done();
+        if (active) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                a.g_means[size_t(i) * 3 + c] = gm[c] + sgm[c][t];
+                a.g_log_scales[size_t(i) * 3 + c] = gls[c];
+            }
+            if ((reinterpret_cast<uintptr_t>(a.g_quats) & 15u) == 0) {
+                reinterpret_cast<float4*>(a.g_quats)[i] = make_float4(gq[0], gq[1], gq[2], gq[3]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) a.g_quats[size_t(i) * 4 + c] = gq[c];
+            }
+            a.g_logits[i] = glogit;
+        }
     }
     __syncthreads();
     if ((reinterpret_cast<uintptr_t>(a.g_sh) & 15u) == 0) {
         float4* gs = reinterpret_cast<float4*>(a.g_sh + size_t(base) * 48);
         const float4* from = reinterpret_cast<const float4*>(srec);
-        for (uint32_t k = threadIdx.x; k < cnt * 12; k += kBwdThreads) gs[k] = from[k];
+        for (uint32_t k = threadIdx.x; k < cnt * 12; k += 2 * kBwdThreads) gs[k] = from[k];
     } else {  // a caller's buffer that is not 16-byte aligned
         float* gs = a.g_sh + size_t(base) * 48;
-        for (uint32_t k = threadIdx.x; k < cnt * 48; k += kBwdThreads) gs[k] = srec[k];
+        for (uint32_t k = threadIdx.x; k < cnt * 48; k += 2 * kBwdThreads) gs[k] = srec[k];
     }
 }
 
@@ -304,8 +396,8 @@ __global__ void __launch_bounds__(kBwdThreads) preprocess_backward_kernel(Prepro
 
 void launch_preprocess_backward(const PreprocessBackwardArgs& a, cudaStream_t s) {
     if (a.n == 0) return;
-    launch_dependent(preprocess_backward_kernel, dim3((a.n + kBwdThreads - 1) / kBwdThreads), dim3(kBwdThreads), 0,
-                     s, a);
+    launch_dependent(preprocess_backward_kernel, dim3((a.n + kBwdThreads - 1) / kBwdThreads), dim3(2 * kBwdThreads),
+                     0, s, a);
 }
 
 }  // namespace tpd
