@@ -29,6 +29,20 @@ def test_sort_pairs(cuda, n, bits):
     np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), vals[order])
 
 
+@pytest.mark.parametrize("n", [1 << 17, (1 << 17) + 1, 3 << 17, (3 << 17) + 1])
+def test_sort_pairs_where_the_partitions_grow(cuda, n):
+    """Sizes at which a radix pass takes more keys per thread."""
+    torch = cuda
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, 1 << 45, size=n, dtype=np.uint64)
+    keys[rng.random(n) < 0.5] &= np.uint64(0xFF)
+    vals = np.arange(n, dtype=np.uint32)
+    order = np.argsort(keys, kind="stable")
+    k, v = T.sort_pairs(torch.from_numpy(keys.view(np.int64)).cuda(), torch.from_numpy(vals.view(np.int32)).cuda(), 45)
+    np.testing.assert_array_equal(k.cpu().numpy().view(np.uint64), keys[order])
+    np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), vals[order])
+
+
 @pytest.mark.parametrize("n,views", [(1, 1), (1025, 1), (12288, 1), (12289, 1), (3072, 4), (2000, 5)])
 def test_frames(cuda, n, views):
     rec = configs.scene("cfg0", n).records.copy()

@@ -419,7 +419,10 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     dp.ticket_base = kTicketDepthSortBase;
     dp.tag_base = kTagDepthSort;
     dp.ctas_per_sm = int(e->settings.sort_ctas_per_sm);
-    dp.items = e->settings.depth_sort_items == 4 || e->settings.depth_sort_items == 8 ? e->settings.depth_sort_items : 16;
+    dp.items = e->settings.depth_sort_items == 4 || e->settings.depth_sort_items == 8 ||
+                       e->settings.depth_sort_items == 16
+                   ? e->settings.depth_sort_items
+                   : sort_items_for(items);
     dp.threads = e->settings.depth_sort_threads == 512 ? 512 : 256;
     dp.fixed_count = items;
     dp.compact_culled = true;  // culled items leave in the first pass; the rest sort ctl->depth_count
@@ -1349,7 +1352,7 @@ void* tpd_get_stream(const tpd_engine* e) { return e ? static_cast<void*>(e->str
 // ---- stage entry points
 
 size_t tpd_sort_workspace_size(uint32_t n) {
-    return 256 * ((sizeof(FrameCtl) + 255) / 256) + sort_desc_entries(n) * 8;
+    return 256 * ((sizeof(FrameCtl) + 255) / 256) + sort_desc_entries(n, sort_items_for(n)) * 8;
 }
 
 int tpd_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, uint32_t n,
@@ -1371,7 +1374,7 @@ int tpd_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t*
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaMemsetAsync(desc, 0, sort_desc_entries(n) * 8, s) != cudaSuccess) return TPD_ERR_DEVICE;
+    if (cudaMemsetAsync(desc, 0, sort_desc_entries(n, sort_items_for(n)) * 8, s) != cudaSuccess) return TPD_ERR_DEVICE;
     launch_sort_begin(ctl, n, s);
     SortPlan plan;
     plan.first_bit = 0;
@@ -1384,6 +1387,7 @@ int tpd_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t*
     // histogram kernel included) and than the counted passes that serve the
     // frame's 32-bit key sort
     plan.threads = 256;
+    plan.items = sort_items_for(n);
     plan.ctas_per_sm = 2;
     const bool alt = launch_sort(keys, vals, keys_alt, vals_alt, n, plan, desc, ctl, kDefaultSpin, sms, s);
     *result_in_alt = alt ? 1 : 0;

@@ -139,6 +139,9 @@ void launch_materialize_keys(const uint32_t* tiles, const uint32_t* vals, const 
 // for an even pass count, else in (keys_alt, vals_alt); returns true for *_alt.
 // desc: sort_desc_entries(capacity, items) descriptors (tagged, never cleared).
 size_t sort_desc_entries(uint32_t capacity, uint32_t items = 16);
+// Keys per thread of the 256-thread onesweep passes over n 64-bit pairs, 4, 8
+// or 16: fewer where 4096-key partitions would leave SMs idle.
+uint32_t sort_items_for(uint32_t n);
 uint32_t sort_pass_count(uint32_t key_bits);
 struct SortPlan {
     uint32_t first_bit = 0;
