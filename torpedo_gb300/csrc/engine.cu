@@ -107,7 +107,8 @@ struct tpd_engine {
     uint32_t total_tiles = 0;
     uint64_t total_pixels = 0;
     uint32_t* d_tile_view = nullptr;
-    uint32_t* d_tile_order = nullptr;  // tiles by decreasing list length, for the blend adjoint
+    uint32_t* d_tile_len = nullptr;    // per tile, list entries up to its last contributor (frames keeping the adjoint's inputs)
+    uint32_t* d_tile_order = nullptr;  // tiles by decreasing d_tile_len, for the blend adjoint
     uint64_t* d_image_offset = nullptr;
 
     // frame buffers
@@ -499,6 +500,7 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     ba.image_offset = e->n_views > 1 ? e->d_image_offset : nullptr;
     ba.final_T = state ? e->d_final_T : nullptr;
     ba.n_contrib = state ? e->d_n_contrib : nullptr;
+    ba.tile_len = e->d_tile_len;
     ba.rgba = rgba;
     launch_blend(ba, blend_launch(e), s);
     mark(6);
@@ -628,6 +630,7 @@ int set_views_internal(tpd_engine* e, const tpd_view* views, uint32_t nv) {
         TPD_CUDA(e, dalloc(e->d_ranges, uint64_t(tiles) * 2));
         TPD_CUDA(e, dalloc(e->d_tile_view, tiles));
         TPD_CUDA(e, dalloc(e->d_tile_order, tiles));
+        TPD_CUDA(e, dalloc(e->d_tile_len, tiles));
         e->tile_cap = tiles;
     }
     if (!e->d_image_offset) TPD_CUDA(e, dalloc(e->d_image_offset, kMaxViews));
@@ -814,6 +817,7 @@ void tpd_destroy(tpd_engine* e) {
     dfree(e->d_views);
     dfree(e->d_tile_view);
     dfree(e->d_tile_order);
+    dfree(e->d_tile_len);
     dfree(e->d_image_offset);
     dfree(e->d_splats);
     dfree(e->d_offsets);
@@ -1189,8 +1193,8 @@ void enqueue_backward(tpd_engine* e, const float* dL_dimage, const BackwardOut& 
     bb.dL_dimage = dL_dimage;
     bb.g2d = e->d_g2d;
     bb.g2d_view_stride = uint64_t(e->n) * kG2DStride;
-    // longest tile lists first: the adjoint's cost per tile varies more than the forward's
-    launch_tile_order(e->d_ranges, e->total_tiles, e->d_ctl, uint32_t(e->capacity), e->d_tile_order, e->stream);
+    // longest walks first: the adjoint's cost per tile varies more than the forward's
+    launch_tile_order(e->d_tile_len, e->total_tiles, e->d_ctl, e->d_tile_order, e->stream);
     bb.tile_order = e->d_tile_order;
     mark(TPD_STAGE_BACKWARD_SETUP + 1);
     launch_blend_backward(bb, blend_launch(e), e->stream);

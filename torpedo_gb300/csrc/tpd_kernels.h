@@ -26,7 +26,10 @@ struct FrameCtl {
     // key (the order stays in the pass's input buffer): when odd, the later
     // passes swap their buffers and the sorted items are in the other one
     uint32_t depth_skips;
-    uint32_t pad[2];
+    uint32_t tile_order_done;  // CTAs of the tile order that have finished (reset by the last)
+    uint32_t pad;
+    uint32_t tile_hist[128];    // tiles by class of their walk length (tile_class), counted by the blend
+    uint32_t tile_cursor[128];  // tiles of each class that the tile order has placed (0 at rest)
 };
 
 // Entity matrices: rows 0..2 of view*model and rows 0..3 of projview*model.
@@ -213,6 +216,9 @@ struct BlendArgs {
     // contributor (the adjoint's inputs); both null: not tracked
     float* final_T;
     uint32_t* n_contrib;
+    // with them: per tile, the list entries up to its last contributor, whose
+    // classes are counted in ctl->tile_hist (for launch_tile_order)
+    uint32_t* tile_len;
     // nullable: the image also as RGBA8 UNORM (alpha 255), packed like image
     // (launch_pack_rgba8's conversion), written with it
     uint32_t* rgba;
@@ -253,13 +259,12 @@ struct BlendBackwardArgs {
 };
 void launch_blend_backward(const BlendBackwardArgs& a, const BlendLaunch& l, cudaStream_t s);
 
-// order[0 .. n_tiles): the tiles by decreasing list length (in classes of
-// equal floor(log2(length + 1)); any order within a class), so the longest
-// lists start first and no SM is left with one at the end. ranges as the
-// blend leaves them (empty tiles (0, 0)); lengths are clipped at
-// min(ctl->total_keys, capacity). Also resets the adjoint's tile queue.
-void launch_tile_order(const uint32_t* ranges, uint32_t n_tiles, FrameCtl* ctl, uint32_t capacity,
-                       uint32_t* order, cudaStream_t s);
+// order[0 .. n_tiles): the tiles by decreasing walk length (classes of a
+// quarter octave; any order within a class), so the longest walks of the
+// adjoint start first and no SM is left with one at the end. tile_len and
+// ctl->tile_hist as the last blend that kept the adjoint's inputs left them.
+// Also resets the adjoint's tile queue.
+void launch_tile_order(const uint32_t* tile_len, uint32_t n_tiles, FrameCtl* ctl, uint32_t* order, cudaStream_t s);
 
 // Per-splat gradient record of the blend adjoint: 9 used floats padded to 12
 // (48 B), so it is accumulated with three 16-byte vector atomics.
