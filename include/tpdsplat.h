@@ -116,7 +116,7 @@ typedef struct tpd_frame_stats {
     uint32_t visible;       /* (view, Gaussian) pairs with a non-empty tile rect */
     uint32_t tiles;         /* 16x16 tiles over all views */
     uint32_t key_bits;      /* low key bits sorted: getHigherMSB(tiles) + 32 */
-    uint32_t sort_passes;   /* 8-bit radix passes */
+    uint32_t sort_passes;   /* 8-bit digits of the tile ids (the sort may take them in fewer, 9-bit passes) */
     uint32_t status;        /* device status bits (0 = clean) */
     uint32_t retries;       /* frames re-run after growing the key buffers */
     uint32_t views;         /* views rendered */

@@ -1282,8 +1282,9 @@ int tpd_step_async(tpd_engine* e, const float* dL_dimage, float* g_means, float*
 namespace {
 
 // The sorted (tile | depth) keys of the last frame, for read-back: the frame
-// itself sorts tile ids only (their depth order comes from the presort), and
-// a key's depth is that of its value's splat, so the keys are rebuilt here
+// itself sorts tile ids only (their depth order comes from the presort) and
+// ends with their ranges, and a key's depth is that of its value's splat, so
+// the keys are rebuilt here
 // into a buffer of their own, allocated on first use. Waits for the stream.
 int rebuild_keys(tpd_engine* e) {
     cudaSetDevice(e->device);
@@ -1294,8 +1295,9 @@ int rebuild_keys(tpd_engine* e) {
         e->keys64_cap = e->capacity;
     }
     const int b = e->sorted_in_alt ? 1 : 0;
-    launch_materialize_keys(e->d_tiles[b], e->d_vals[b], e->d_splats, e->n, e->n_views > 1 ? e->d_tile_view : nullptr,
-                            e->total_tiles, uint32_t(e->capacity), e->d_ctl, e->d_keys64, e->stream);
+    launch_materialize_keys(e->d_ranges, e->total_tiles, e->d_vals[b], e->d_splats, e->n,
+                            e->n_views > 1 ? e->d_tile_view : nullptr, uint32_t(e->capacity), e->d_ctl, e->d_keys64,
+                            e->stream);
     TPD_CUDA(e, cudaGetLastError());
     return wait_stream(e);
 }

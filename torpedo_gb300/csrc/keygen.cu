@@ -205,13 +205,16 @@ constexpr uint32_t kExpandThreads = 256;
 constexpr uint32_t kExpandSlots = kCountedTile / kExpandThreads;
 constexpr uint32_t kTileDigitsMax = 4;
 
-template <bool kCounted>
+// kDig: digits of the counted first pass (256 or 512), 0 for the look-back form.
+template <uint32_t kDig>
 __global__ void __launch_bounds__(kExpandThreads)
     expand_keys_kernel(const uint4* __restrict__ item_info, const uint32_t* __restrict__ part_first,
                        uint32_t* __restrict__ tiles, uint32_t* __restrict__ vals, uint32_t n_items, uint32_t capacity, uint32_t max_parts,
                        uint32_t tile_bits, uint32_t* __restrict__ work, FrameCtl* ctl) {
     __shared__ __align__(16) uint16_t owner[kCountedTile];  // item of each slot, from the partition's first
-    __shared__ uint32_t digits[kCounted ? 1 : kTileDigitsMax][256];
+    constexpr bool kCounted = kDig != 0;
+    constexpr uint32_t kRows = kCounted ? 1u : kTileDigitsMax, kWidth = kCounted ? kDig : 256u;
+    __shared__ uint32_t digits[kRows][kWidth];
     __shared__ uint32_t wmax[kExpandThreads / 32], wsum[kExpandThreads / 32];
     __shared__ bool s_last;
     pdl_wait();
@@ -230,7 +233,7 @@ __global__ void __launch_bounds__(kExpandThreads)
     uint4* own4 = reinterpret_cast<uint4*>(owner);
     own4[2 * tid] = own4[2 * tid + 1] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-    for (uint32_t p = 0; p < (kCounted ? 1u : kTileDigitsMax); ++p) digits[p][tid] = 0;
+    for (uint32_t p = 0; p < kRows * kWidth / kExpandThreads; ++p) (&digits[0][0])[p * kExpandThreads + tid] = 0;
     __syncthreads();
     for (uint32_t k = tid + 1u; k < m; k += kExpandThreads) {  // (item 0 owns slot 0: the map's zeros)
         const uint32_t slot = item_info[first + k].z - base;
@@ -312,8 +315,8 @@ __global__ void __launch_bounds__(kExpandThreads)
             for (uint32_t u = 0; u < 4; ++u) {
                 if (!kFull && slot + u >= cnt) continue;
 #pragma unroll
-                for (uint32_t p = 0; p < (kCounted ? 1u : kTileDigitsMax); ++p)
-                    if (p < ndig) atomicAdd(&digits[p][(t[u] >> (8u * p)) & 255u], 1u);
+                for (uint32_t p = 0; p < kRows; ++p)
+                    if (p < ndig) atomicAdd(&digits[p][(t[u] >> (8u * p)) & (kWidth - 1u)], 1u);
             }
         }
     };
@@ -323,7 +326,11 @@ __global__ void __launch_bounds__(kExpandThreads)
         expand(std::false_type{});
     __syncthreads();
     if constexpr (kCounted) {
-        counted_finish(CountedWork(work, max_parts), nparts, part, digits[0][tid], wsum, s_last);
+        constexpr uint32_t kPer = kWidth / kExpandThreads;
+        RowDigits<kPer> count;
+#pragma unroll
+        for (uint32_t p = 0; p < kPer; ++p) count.v[p] = digits[0][kPer * tid + p];
+        counted_finish<kWidth>(CountedWork<kWidth>(work, max_parts), nparts, part, count, wsum, s_last);
     } else {
         for (uint32_t p = 0; p < ndig; ++p)
             if (digits[p][tid]) atomicAdd(&ctl->sort_hist[p][tid], digits[p][tid]);
@@ -348,21 +355,26 @@ void launch_keygen(const KeygenArgs& a, int num_sms, cudaStream_t s) {
                      a.items_other, a.n_items, a.n, a.views, a.offsets, a.item_info, a.part_first, a.capacity,
                      a.ranges, a.n_tiles, a.desc, a.ctl, a.spin_limit, a.never_publish);
     const uint32_t max_parts = std::max(1u, uint32_t((uint64_t(a.capacity) + kCountedTile - 1) / kCountedTile));
-    launch_dependent(a.counted_work ? expand_keys_kernel<true> : expand_keys_kernel<false>, dim3(max_parts),
+    const auto expand = !a.counted_work                                ? expand_keys_kernel<0>
+                        : counted_digit_bits(a.tile_bits) > 8 ? expand_keys_kernel<512>
+                                                              : expand_keys_kernel<256>;
+    launch_dependent(expand, dim3(max_parts),
                      dim3(kExpandThreads), 0, s, static_cast<const uint4*>(a.item_info),
                      static_cast<const uint32_t*>(a.part_first), a.tiles, a.vals, a.n_items, a.capacity, max_parts, a.tile_bits, a.counted_work, a.ctl);
 }
 
 namespace {
 
-__global__ void materialize_keys_kernel(const uint32_t* __restrict__ tiles, const uint32_t* __restrict__ vals,
+// One CTA per tile: the tile's range of values, with the tile and each value's
+// depth. (A tile without keys has the range (0, 0) or (0xFFFFFFFF, 0).)
+__global__ void materialize_keys_kernel(const uint32_t* __restrict__ ranges, const uint32_t* __restrict__ vals,
                                         const Splat* __restrict__ splats, uint32_t n,
-                                        const uint32_t* __restrict__ tile_view, uint32_t n_tiles, uint32_t capacity,
+                                        const uint32_t* __restrict__ tile_view, uint32_t capacity,
                                         const FrameCtl* __restrict__ ctl, uint64_t* __restrict__ keys) {
-    const uint32_t K = min(ctl->total_keys, capacity);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < K; i += gridDim.x * blockDim.x) {
-        const uint32_t t = tiles[i], g = vals[i];
-        const uint32_t v = tile_view && t < n_tiles ? tile_view[t] : 0u;
+    const uint32_t t = blockIdx.x, v = tile_view ? tile_view[t] : 0u;
+    const uint32_t K = min(ctl->total_keys, capacity), end = min(ranges[2 * t + 1], K);
+    for (uint32_t i = ranges[2 * t] + threadIdx.x; i < end; i += blockDim.x) {
+        const uint32_t g = vals[i];
         const uint32_t depth = g < n ? __float_as_uint(reinterpret_cast<const float4*>(splats + size_t(v) * n + g)[1].z)
                                      : 0xFFFFFFFFu;
         keys[i] = (uint64_t(t) << 32) | depth;
@@ -371,12 +383,11 @@ __global__ void materialize_keys_kernel(const uint32_t* __restrict__ tiles, cons
 
 }  // namespace
 
-void launch_materialize_keys(const uint32_t* tiles, const uint32_t* vals, const Splat* splats, uint32_t n,
-                             const uint32_t* tile_view, uint32_t n_tiles, uint32_t capacity, const FrameCtl* ctl,
+void launch_materialize_keys(const uint32_t* ranges, uint32_t n_tiles, const uint32_t* vals, const Splat* splats,
+                             uint32_t n, const uint32_t* tile_view, uint32_t capacity, const FrameCtl* ctl,
                              uint64_t* keys, cudaStream_t s) {
-    if (capacity == 0) return;
-    const uint32_t blocks = std::min<uint32_t>((capacity + 255) / 256, 4096u);
-    materialize_keys_kernel<<<blocks, 256, 0, s>>>(tiles, vals, splats, n, tile_view, n_tiles, capacity, ctl, keys);
+    if (capacity == 0 || n_tiles == 0) return;
+    materialize_keys_kernel<<<n_tiles, 128, 0, s>>>(ranges, vals, splats, n, tile_view, capacity, ctl, keys);
 }
 
 }  // namespace tpd

@@ -127,11 +127,12 @@ struct KeygenArgs {
 };
 void launch_keygen(const KeygenArgs& a, int num_sms, cudaStream_t s);
 
-// keys[i] = tiles[i] << 32 | bits(viewZ of splat vals[i] in the tile's view),
-// i < min(ctl->total_keys, capacity): the 64-bit (tile | depth) keys of a
-// frame, from its sorted tile ids and values (read-back only).
-void launch_materialize_keys(const uint32_t* tiles, const uint32_t* vals, const Splat* splats, uint32_t n,
-                             const uint32_t* tile_view, uint32_t n_tiles, uint32_t capacity, const FrameCtl* ctl,
+// keys[i] = tile << 32 | bits(viewZ of splat vals[i] in the tile's view) for
+// the slots i < min(ctl->total_keys, capacity) of every tile's range: the
+// 64-bit (tile | depth) keys of a frame, from its tile ranges and sorted values
+// (read-back only).
+void launch_materialize_keys(const uint32_t* ranges, uint32_t n_tiles, const uint32_t* vals, const Splat* splats,
+                             uint32_t n, const uint32_t* tile_view, uint32_t capacity, const FrameCtl* ctl,
                              uint64_t* keys, cudaStream_t s);
 
 // Onesweep LSD radix sort of (key, val) pairs on key bits [first_bit, key_bits),
@@ -170,7 +171,8 @@ struct SortPlan {
     // non-null, 32-bit keys: counted passes (every partition's digit offsets
     // counted and scanned beforehand, no look-back; plain pass kinds only) using this work
     // area of sort_counted_work_words(capacity) u32, zeroed once (every launch
-    // leaves its arrival counts at zero)
+    // leaves its arrival counts at zero). With ranges, the last pass writes
+    // them and the values, not the keys
     uint32_t* counted_work = nullptr;
     // counted passes: the first pass's digit offsets are already in
     // counted_work, put there by the kernel that wrote the keys right before
@@ -178,6 +180,9 @@ struct SortPlan {
     bool precounted = false;
 };
 size_t sort_counted_work_words(uint32_t capacity);
+// Digit width of the counted passes over keys of key_bits bits: 9 where that
+// takes fewer passes than 8.
+uint32_t counted_digit_bits(uint32_t key_bits);
 bool launch_sort(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, uint32_t capacity,
                  const SortPlan& plan, uint64_t* desc, FrameCtl* ctl, uint32_t spin_limit, int num_sms,
                  cudaStream_t s);
