@@ -199,15 +199,16 @@ __global__ void __launch_bounds__(kScanItemsThreads)
 // (look-back passes): every digit of the tile ids is added to ctl->sort_hist.
 // Bound by latency and issue; the stores are 8 bytes a key. With one key per
 // thread and step (35 instructions a key, two dependent loads) 1M Gaussians at
-// 1080p took 67 us with the scan, 8 views of 500,000 at 720p 216; now 57 and
-// 171.
+// 1080p took 67 us with the scan, 8 views of 500,000 at 720p 216; now 55 and
+// 162, with registers for four CTAs per SM (71 registers, three CTAs: 59 and
+// 171; five: 57 and 164).
 constexpr uint32_t kExpandThreads = 256;
 constexpr uint32_t kExpandSlots = kCountedTile / kExpandThreads;
 constexpr uint32_t kTileDigitsMax = 4;
 
 // kDig: digits of the counted first pass (256 or 512), 0 for the look-back form.
 template <uint32_t kDig>
-__global__ void __launch_bounds__(kExpandThreads)
+__global__ void __launch_bounds__(kExpandThreads, 4)
     expand_keys_kernel(const uint4* __restrict__ item_info, const uint32_t* __restrict__ part_first,
                        uint32_t* __restrict__ tiles, uint32_t* __restrict__ vals, uint32_t n_items, uint32_t capacity, uint32_t max_parts,
                        uint32_t tile_bits, uint32_t* __restrict__ work, FrameCtl* ctl) {

@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 // The permutation is the same stable one.
 // Digits have 8 bits, or 9 (kDig = 512) where that takes a pass less.
 template <int kItems, uint32_t kDig, typename KeyT>
-__global__ void __launch_bounds__(256) partition_count_kernel(const KeyT* __restrict__ keys, uint32_t capacity,
+__global__ void __launch_bounds__(256, 6) partition_count_kernel(const KeyT* __restrict__ keys, uint32_t capacity,
                                                               uint32_t shift, uint32_t bits, uint32_t fixed_count,
                                                               uint32_t max_parts, uint32_t* __restrict__ work,
                                                               FrameCtl* ctl, uint32_t abort_mask) {
@@ -534,13 +534,13 @@ __global__ void __launch_bounds__(256) partition_count_kernel(const KeyT* __rest
     counted_finish<kDig>(CountedWork<kDig>(work, max_parts), nparts, part, total, wsum, last);
 }
 
-template <uint32_t kDig, typename KeyT>
+// A partition of a scatter: its pairs reordered by digit, each in one 8-byte
+// slot (one store and one load per pair), one pad slot per 16 (pad16).
+template <uint32_t kDig>
 struct ScatterSmem {
-    KeyT keys[4096 + 4096 / 16];
-    uint32_t vals[4096 + 4096 / 16];
-    uint32_t whist[8][kDig];
-    uint32_t lstart[kDig];  // partition-local digit start
-    uint32_t gmap[kDig];    // global position of local index 0 of each digit
+    uint2 pairs[4096 + 4096 / 16];  // key, value
+    uint32_t whist[8][kDig];        // per-warp digit counts, then the first slot of the warp's keys of each digit
+    uint32_t gmap[kDig];            // global position of local index 0 of each digit
     uint32_t wsum[8];
 };
 
@@ -555,6 +555,11 @@ struct ScatterSmem {
 // give the range whatever the order (range.slang:18-35). Against writing the
 // keys too and comparing both neighbours of every key: 1M Gaussians at 1080p 57
 // -> 51 us, 3M at 2160p 573 -> 501.
+// What bounds it: the shared-memory pipe (75% busy with keys and values in
+// arrays of their own and the digit and warp offsets looked up apart) and the
+// integer pipe (63%: ballots). Pairs in one slot and merged offsets took both
+// passes and the count from 120 to 108 us at 1M Gaussians and 1080p; 64
+// registers for a fourth CTA per SM spill (118).
 template <int kMinBlocks, int kBits, bool kLast, typename KeyT>
 __global__ void __launch_bounds__(256, kMinBlocks)
     scatter_kernel(const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, KeyT* __restrict__ keys_out,
@@ -564,7 +569,8 @@ __global__ void __launch_bounds__(256, kMinBlocks)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr uint32_t kItems = 16, kSortTile = 4096, kWarps = 8;
     constexpr uint32_t kDig = kBits > 8 ? 512 : 256, kPer = kDig / 256;
-    ScatterSmem<kDig, KeyT>& S = *reinterpret_cast<ScatterSmem<kDig, KeyT>*>(smem_raw);
+    static_assert(sizeof(KeyT) == 4, "a pair is 8 bytes");
+    ScatterSmem<kDig>& S = *reinterpret_cast<ScatterSmem<kDig>*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     // the keys and values come from the kernel before the counting one, so they
     // are loaded while that one finishes; or (keys_just_written) from the
@@ -603,7 +609,7 @@ __global__ void __launch_bounds__(256, kMinBlocks)
             reinterpret_cast<uint4*>(&S.whist[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
         // stable rank within the warp (warp-striped order)
-        uint32_t dr[kItems];
+        uint32_t rank[kItems / 2];  // two 16-bit ranks each
         const uint32_t lt = lanemask_lt();
 #pragma unroll
         for (uint32_t i = 0; i < kItems; ++i) {
@@ -628,49 +634,52 @@ __global__ void __launch_bounds__(256, kMinBlocks)
                 S.whist[warp][d] = prev + __popc(peers);
             }
             prev = __shfl_sync(0xFFFFFFFFu, prev, leader);
-            dr[i] = d | ((prev + __popc(peers & lt)) << 10);
+            const uint32_t r = prev + __popc(peers & lt);
+            rank[i / 2] = i & 1u ? rank[i / 2] | r << 16 : r;
             __syncwarp();
         }
         __syncthreads();
-        RowDigits<kPer> count = {};
+        RowDigits<kPer> c[kWarps], count = {};
 #pragma unroll
         for (uint32_t w = 0; w < kWarps; ++w)
 #pragma unroll
             for (uint32_t p = 0; p < kPer; ++p) {
-                const uint32_t c = S.whist[w][kPer * tid + p];
-                S.whist[w][kPer * tid + p] = count.v[p];
-                count.v[p] += c;
+                c[w].v[p] = S.whist[w][kPer * tid + p];
+                count.v[p] += c[w].v[p];
             }
-        const RowDigits<kPer> lstart = scan_digits<kPer>(count, S.wsum);  // (its barriers cover whist)
+        RowDigits<kPer> slot = scan_digits<kPer>(count, S.wsum);  // the digits' first slots
 #pragma unroll
-        for (uint32_t p = 0; p < kPer; ++p) {
-            S.lstart[kPer * tid + p] = lstart.v[p];
-            S.gmap[kPer * tid + p] = goff.v[p] - lstart.v[p];
-        }
+        for (uint32_t p = 0; p < kPer; ++p) S.gmap[kPer * tid + p] = goff.v[p] - slot.v[p];
+#pragma unroll
+        for (uint32_t w = 0; w < kWarps; ++w)
+#pragma unroll
+            for (uint32_t p = 0; p < kPer; ++p) {
+                S.whist[w][kPer * tid + p] = slot.v[p];
+                slot.v[p] += c[w].v[p];
+            }
         __syncthreads();
 #pragma unroll
         for (uint32_t i = 0; i < kItems; ++i) {
-            const uint32_t d = dr[i] & 1023u;
-            if (kFull || d < kDig) {
-                const uint32_t pos = S.lstart[d] + S.whist[warp][d] + (dr[i] >> 10);
-                if (TPD_INBOUNDS(ctl, 20, pos, cnt)) {
-                    S.keys[pad16(pos)] = k[i];
-                    S.vals[pad16(pos)] = vr[i];
-                }
+            const uint32_t idx = warp * (kItems * 32) + i * 32 + lane;
+            if (kFull || idx < cnt) {
+                const uint32_t pos =
+                    S.whist[warp][(k[i] >> shift) & mask] + (i & 1u ? rank[i / 2] >> 16 : rank[i / 2] & 0xFFFFu);
+                if (TPD_INBOUNDS(ctl, 20, pos, cnt)) S.pairs[pad16(pos)] = make_uint2(k[i], vr[i]);
             }
         }
         __syncthreads();
         // (g < K <= capacity: the bound check covers the buffer's end)
         auto write_out = [&](uint32_t j) {
-            const KeyT key = S.keys[pad16(j)];
-            const uint32_t g = S.gmap[uint32_t(key >> shift) & mask] + j;
+            const uint2 pair = S.pairs[pad16(j)];
+            const KeyT key = pair.x;
+            const uint32_t g = S.gmap[(key >> shift) & mask] + j;
             if (!TPD_INBOUNDS(ctl, 22, g, K)) return;
-            vals_out[g] = S.vals[pad16(j)];
+            vals_out[g] = pair.y;
             if constexpr (!kLast) {
                 keys_out[g] = key;
             } else {
                 if (!TPD_INBOUNDS(ctl, 18, key, n_tiles)) return;
-                const KeyT before = j ? S.keys[pad16(j - 1)] : KeyT(~KeyT(0));
+                const KeyT before = j ? S.pairs[pad16(j - 1)].x : KeyT(~KeyT(0));
                 if (before != key) {
                     atomicMin(&ranges[2 * key], g);
                     if (j && TPD_INBOUNDS(ctl, 18, before, n_tiles))
@@ -750,7 +759,7 @@ void launch_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout, uint32_
 template <int kMinBlocks, int kBits, bool kLast, typename KeyT>
 int scatter_setup() {
     cudaFuncSetAttribute(scatter_kernel<kMinBlocks, kBits, kLast, KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(sizeof(ScatterSmem<(kBits > 8 ? 512 : 256), KeyT>)));
+                         int(sizeof(ScatterSmem<(kBits > 8 ? 512 : 256)>)));
     return 1;
 }
 
@@ -758,7 +767,7 @@ int scatter_setup() {
 // a scatter launch, one CTA per 4096-key partition each. work: the counted
 // work area (counted_work_words(max partitions) u32, its arrival counts zero
 // at rest). The scatter ranks with as many ballots as the pass has bits (the
-// 3-CTA variant; the 2-CTA one with 8 or 9).
+// default variant; the 2-CTA one with 8 or 9).
 template <int kMinBlocks, typename KeyT>
 void launch_counted_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout, uint32_t capacity,
                            const SortPlan& plan, uint32_t* work, FrameCtl* ctl, cudaStream_t s) {
@@ -778,12 +787,12 @@ void launch_counted_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout,
             constexpr bool kLast = decltype(last_tag)::value;
             device_once(scatter_setup<kMinBlocks, kBits, kLast, KeyT>);
             launch_dependent(scatter_kernel<kMinBlocks, kBits, kLast, KeyT>, dim3(max_parts), dim3(256),
-                             sizeof(ScatterSmem<(kBits > 8 ? 512 : 256), KeyT>), s, kin, vin, kout, vout, capacity,
+                             sizeof(ScatterSmem<(kBits > 8 ? 512 : 256)>), s, kin, vin, kout, vout, capacity,
                              shift, bits, plan.fixed_count, max_parts, work, ctl, plan.ranges, plan.n_tiles, abort,
                              counted);
         };
         auto either = [&](auto bits_tag) { last ? scatter(bits_tag, std::true_type{}) : scatter(bits_tag, std::false_type{}); };
-        if (kMinBlocks != 3 && bits <= 8) {
+        if (kMinBlocks == 2 && bits <= 8) {
             either(std::integral_constant<int, 8>{});
         } else {
             switch (bits) {
