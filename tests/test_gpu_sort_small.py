@@ -29,7 +29,7 @@ def test_sort_pairs(cuda, n, bits):
     np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), vals[order])
 
 
-@pytest.mark.parametrize("n", [1 << 17, (1 << 17) + 1, 3 << 17, (3 << 17) + 1])
+@pytest.mark.parametrize("n", [1 << 17, (1 << 17) + 1, 1 << 19, (1 << 19) + 1])
 def test_sort_pairs_where_the_partitions_grow(cuda, n):
     """Sizes at which a radix pass takes more keys per thread."""
     torch = cuda

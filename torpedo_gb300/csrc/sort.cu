@@ -704,7 +704,8 @@ __global__ void __launch_bounds__(256, kMinBlocks)
 // Residencies: the 256-thread, 16-key variant is compiled for 2 CTAs per SM
 // (128 registers, no spills; the default) or 3 (80 registers); the 512-thread,
 // 8-key variant for 2 (32 warps per SM); the 8- and 4-key 256-thread variants
-// (shorter partitions, for small sorts) for 4 and 5.
+// (shorter partitions, for small sorts) for 3 and 4 (registers for 4 and 5 spill
+// and measured 4 to 8% slower).
 // Shared-memory opt-in of every pass kind of a variant and its resident CTAs
 // per SM, once per device.
 template <int kItems, int kThreads, int kMinBlocks, typename KeyT>
@@ -831,10 +832,10 @@ size_t sort_desc_entries(uint32_t capacity, uint32_t items) {
     return (size_t(capacity) + tile - 1) / tile * kRadix + kRadix;
 }
 
-// Measured on the depth sort (4 passes, us): 30,000 items 44 / 36 / 32 with 16
-// / 8 / 4 keys a thread, 120,000 49 / 41 / 40, 250,000 52 / 47 / 48, 500,000
-// 58 / 58 / 66, 1M 69 / 77 / 90.
-uint32_t sort_items_for(uint32_t n) { return n <= (1u << 17) ? 4u : n <= 3u << 17 ? 8u : 16u; }
+// Measured on the depth sort (4 passes, us): 30,000 items 44 / 35 / 30 with 16
+// / 8 / 4 keys a thread, 120,000 49 / 40 / 38, 250,000 52 / 45 / 48, 500,000
+// 58 / 56 / 66, 1M 69 / 71 / 90.
+uint32_t sort_items_for(uint32_t n) { return n <= (1u << 17) ? 4u : n <= (1u << 19) ? 8u : 16u; }
 
 void launch_sort_begin(FrameCtl* ctl, uint32_t total, cudaStream_t s) { sort_begin_kernel<<<1, 256, 0, s>>>(ctl, total); }
 
@@ -868,10 +869,10 @@ bool launch_sort_t(KeyT* keys, uint32_t* vals, KeyT* keys_alt, uint32_t* vals_al
         launch_passes<8, 512, 2>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan, hist, desc, ctl, spin_limit,
                                  sms, s);
     else if (plan.items == 8)
-        launch_passes<8, 256, 4>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan, hist, desc, ctl, spin_limit,
+        launch_passes<8, 256, 3>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan, hist, desc, ctl, spin_limit,
                                  sms, s);
     else if (plan.items == 4)
-        launch_passes<4, 256, 5>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan, hist, desc, ctl, spin_limit,
+        launch_passes<4, 256, 4>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan, hist, desc, ctl, spin_limit,
                                  sms, s);
     else if (plan.ctas_per_sm == 3)
         launch_passes<16, 256, 3>(keys, vals, keys_alt, vals_alt, capacity, p0, p1, plan, hist, desc, ctl, spin_limit,
