@@ -1412,12 +1412,8 @@ int tpd_scan_tiles(const void* splats, uint32_t n, uint32_t* offsets, uint32_t* 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     FrameCtl* ctl = static_cast<FrameCtl*>(workspace);
     uint64_t* desc = reinterpret_cast<uint64_t*>(static_cast<char*>(workspace) + 256 * ((sizeof(FrameCtl) + 255) / 256));
-    const size_t entries = size_t(n) / kScanTileStandalone + 2;
-    if (cudaMemsetAsync(desc, 0, entries * 8, s) != cudaSuccess) return TPD_ERR_DEVICE;
-    launch_sort_begin(ctl, 0, s);
-    launch_scan_tiles(static_cast<const Splat*>(splats), n, offsets, desc, ctl, kDefaultSpin,
+    launch_scan_tiles(static_cast<const Splat*>(splats), n, offsets, total, desc, ctl, &ctl->status, kDefaultSpin,
                       test_never_publish_standalone(), s);
-    if (cudaMemcpyAsync(total, &ctl->total_keys, 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return TPD_ERR_DEVICE;
     return cudaGetLastError() == cudaSuccess ? TPD_OK : TPD_ERR_DEVICE;
 }
 

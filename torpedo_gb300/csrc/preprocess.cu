@@ -413,36 +413,53 @@ __global__ void __launch_bounds__(kPreThreads, kCtas) preprocess_kernel(Preproce
             if (S.hist[p][d]) atomicAdd(&a.ctl->depth_hist[p][d], S.hist[p][d]);
 }
 
-// Exclusive scan of Splat.tiles over partitions of 256 threads x 4 items
-// (prefix.slang:40-158), partitions taken by atomic ticket. Total ->
-// ctl->total_keys, non-empty count -> ctl->visible. (The frame scans its
-// counts in depth order, scan_items_kernel.)
+// Exclusive scan of Splat.tiles (prefix.slang:40-158) over partitions of 256
+// threads x kScanItems items taken by atomic ticket, a warp's items in chunks
+// of 32, one per lane (a splat is 48 bytes, so a chunk's counts lie in 12 lines;
+// four consecutive items per lane touched four times as many, 18 us for 1M
+// splats). 16 items per lane take 8 us (36 MB of sectors and offsets, 5 at copy
+// speed), 8 items 11, 4 items 13: fewer partitions shorten the look-back's
+// chain. Total -> *total. (The frame scans its counts in depth order,
+// scan_items_kernel.)
 constexpr uint32_t kScanThreads = 256;
-constexpr uint32_t kScanItems = 4;
+constexpr uint32_t kScanItems = 16;
+
+// Clears what the scan starts from: the look-back descriptors, the ticket,
+// the status and the total (of no splats).
+__global__ void scan_begin_kernel(uint64_t* desc, uint32_t entries, FrameCtl* ctl, uint32_t* status, uint32_t* total) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < entries) desc[i] = 0;
+    if (i == 0) {
+        ctl->ticket[kTicketScan] = 0;
+        ctl->tag = 0;
+        *status = 0;
+        *total = 0;
+    }
+}
 
 __global__ void __launch_bounds__(kScanThreads)
     scan_tiles_kernel(const Splat* splats, uint32_t n, uint32_t* offsets, uint64_t* desc, FrameCtl* ctl,
-                      uint32_t spin_limit, uint32_t never_publish) {
+                      uint32_t* status, uint32_t* total_out, uint32_t spin_limit, uint32_t never_publish) {
     constexpr uint32_t kScanTile = kScanThreads * kScanItems;
+    constexpr uint32_t kTag = 1;  // (a cleared descriptor has tag 0)
     __shared__ uint32_t s_part, s_excl;
     __shared__ uint32_t s_warp[kScanThreads / 32];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    pdl_wait();  // launched as a dependent of scan_begin_kernel
     if (tid == 0) s_part = atomicAdd(&ctl->ticket[kTicketScan], 1u);
     __syncthreads();
     const uint32_t part = s_part;
-    if (part * kScanTile >= n) return;  // (uniform) past the items; nothing waits on it
-    const uint32_t base = part * kScanTile + tid * kScanItems;
-    uint32_t v[kScanItems], sum = 0, vis = 0;
+    const uint64_t base = uint64_t(part) * kScanTile + warp * (32u * kScanItems) + lane;
+    if (uint64_t(part) * kScanTile >= n) return;  // (uniform) past the items; nothing waits on it
+    uint32_t v[kScanItems], incl[kScanItems], sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kScanItems; ++k) v[k] = base + 32u * k < n ? splats[base + 32u * k].tiles : 0u;
 #pragma unroll
     for (uint32_t k = 0; k < kScanItems; ++k) {
-        v[k] = base + k < n ? splats[base + k].tiles : 0u;
-        sum += v[k];
-        vis += v[k] ? 1u : 0u;
+        incl[k] = sum + warp_inclusive_scan(v[k]);
+        sum = __shfl_sync(0xFFFFFFFFu, incl[k], 31);
     }
-    const uint32_t incl = warp_inclusive_scan(sum);
-    if (lane == 31) s_warp[warp] = incl;
-    vis = warp_sum(vis);
-    if (lane == 0 && vis) atomicAdd(&ctl->visible, vis);
+    if (lane == 0) s_warp[warp] = sum;
     __syncthreads();
     uint32_t wbase = 0, total = 0;
 #pragma unroll
@@ -452,21 +469,17 @@ __global__ void __launch_bounds__(kScanThreads)
         total += sw;
     }
     if (warp == 0) {
-        const uint32_t ex = warp_lookback(desc, part, total, ctl->tag * 32u + kTagScan, &ctl->status, spin_limit,
-                                          never_publish != 0);
+        const uint32_t ex = warp_lookback(desc, part, total, kTag, status, spin_limit, never_publish != 0);
         if (lane == 0) {
             s_excl = ex;
-            const uint32_t nparts = (n + kScanTile - 1) / kScanTile;
-            if (part == nparts - 1) ctl->total_keys = ex + total;
+            if (part == (n - 1u) / kScanTile) *total_out = ex + total;
         }
     }
     __syncthreads();
-    uint32_t run = s_excl + wbase + incl - sum;
+    const uint32_t first = s_excl + wbase;
 #pragma unroll
-    for (uint32_t k = 0; k < kScanItems; ++k) {
-        if (base + k < n) offsets[base + k] = run;
-        run += v[k];
-    }
+    for (uint32_t k = 0; k < kScanItems; ++k)
+        if (base + 32u * k < n) offsets[base + 32u * k] = first + incl[k] - v[k];
 }
 
 // Raw parameters -> records (activation as in GaussianGeometry.cpp:112-115:
@@ -533,11 +546,13 @@ void launch_preprocess(const PreprocessArgs& a, int num_sms, cudaStream_t s) {
         launch_preprocess_t<4>(a, num_sms, s);
 }
 
-void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint64_t* desc, FrameCtl* ctl,
-                       uint32_t spin_limit, uint32_t never_publish, cudaStream_t s) {
+void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint32_t* total, uint64_t* desc,
+                       FrameCtl* ctl, uint32_t* status, uint32_t spin_limit, uint32_t never_publish, cudaStream_t s) {
+    const uint32_t parts = uint32_t((uint64_t(n) + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems));
+    scan_begin_kernel<<<parts / 256 + 1, 256, 0, s>>>(desc, parts, ctl, status, total);
     if (n == 0) return;
-    const uint32_t blocks = (n + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems);
-    scan_tiles_kernel<<<blocks, kScanThreads, 0, s>>>(splats, n, offsets, desc, ctl, spin_limit, never_publish);
+    launch_dependent(scan_tiles_kernel, dim3(parts), dim3(kScanThreads), 0, s, splats, n, offsets, desc, ctl, status,
+                     total, spin_limit, never_publish);
 }
 
 void launch_pack_records(const float* means, const float* log_scales, const float* quats, const float* logits,

@@ -79,14 +79,8 @@ int tpd_scan_tiles_static(const void* splats, uint32_t n, uint32_t* offsets, uin
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     FrameCtl* ctl = reinterpret_cast<FrameCtl*>(scratch);
     uint64_t* desc = reinterpret_cast<uint64_t*>(scratch + kCtlBytes);
-    const size_t entries = size_t(n) / kStaticScanTile + 2;
-    if (cudaMemsetAsync(desc, 0, entries * sizeof(uint64_t), s) != cudaSuccess) return TPD_ERR_DEVICE;
-    launch_sort_begin(ctl, 0, s);
-    launch_scan_tiles(static_cast<const Splat*>(splats), n, offsets, desc, ctl, kStaticSpin,
-                      test_never_publish_standalone(), s);
-    if (cudaMemcpyAsync(total, &ctl->total_keys, 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return TPD_ERR_DEVICE;
-    if (status && cudaMemcpyAsync(status, &ctl->status, 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-        return TPD_ERR_DEVICE;
+    launch_scan_tiles(static_cast<const Splat*>(splats), n, offsets, total, desc, ctl, status ? status : &ctl->status,
+                      kStaticSpin, test_never_publish_standalone(), s);
     return cudaGetLastError() == cudaSuccess ? TPD_OK : TPD_ERR_DEVICE;
 }
 

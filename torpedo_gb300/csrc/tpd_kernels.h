@@ -82,9 +82,11 @@ void launch_frame_begin(FrameCtl* ctl, const float* transforms, uint32_t n_ent, 
                         uint32_t n_views, float* ent_mats, cudaStream_t s);
 void launch_preprocess(const PreprocessArgs& a, int num_sms, cudaStream_t s);
 
-// Standalone exclusive scan of Splat.tiles (prefix.slang); total -> ctl->total_keys.
-void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint64_t* desc, FrameCtl* ctl,
-                       uint32_t spin_limit, uint32_t never_publish, cudaStream_t s);
+// Standalone exclusive scan of Splat.tiles (prefix.slang) into offsets, total
+// into *total, device status into *status. Clears everything it starts from:
+// desc (ceil(n / 4096) descriptors) and ctl's ticket.
+void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint32_t* total, uint64_t* desc,
+                       FrameCtl* ctl, uint32_t* status, uint32_t spin_limit, uint32_t never_publish, cudaStream_t s);
 
 // Items (view, Gaussian) in depth order per partition of the depth-order
 // scan: its look-back descriptors number n_items / kKeygenPart + 2.
