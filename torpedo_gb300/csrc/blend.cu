@@ -639,25 +639,29 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
     float* g2d_view = a.g2d + size_t(vi) * a.g2d_view_stride;
 
     // A round's entries, kPer per thread (with fewer entries than threads the
-    // warps take turns): loaded before the previous round is walked and staged
-    // after it, so the gathers' latency hides behind the walk. Slot k of the
+    // warps take turns): their indices loaded two rounds before they are
+    // walked, their splats one, and staged after that round's walk, so both
+    // latencies hide behind walks. Slot k of the
     // round whose list positions end at r_end holds position r_end - 1 - k.
     constexpr uint32_t kPer = kBwdRound > kAdjThreads ? kBwdRound / kAdjThreads : 1u;
-    uint32_t pf_idx[kPer];
+    uint32_t pf_idx[kPer], nx_idx[kPer];  // of the round being loaded, and of the one after it
     float4 pf_c[kPer], pf_tex[kPer], pf_co[kPer];
-    auto load_round = [&](uint32_t r_end, uint32_t turn) {
+    auto load_indices = [&](uint32_t r_end, uint32_t turn) {
 #pragma unroll
         for (uint32_t u = 0; u < kPer; ++u) {
             const uint32_t k = (tid ^ turn) + u * kAdjThreads;
-            pf_idx[u] = 0xFFFFFFFFu;
-            if (k < min(kBwdRound, r_end)) {
-                pf_idx[u] = a.vals[start + r_end - 1u - k];
-                if (pf_idx[u] < a.n) {
-                    const float4* p = reinterpret_cast<const float4*>(vsplats + pf_idx[u]);
-                    pf_c[u] = __ldg(p + 0);
-                    pf_tex[u] = __ldg(p + 1);
-                    pf_co[u] = __ldg(p + 2);
-                }
+            nx_idx[u] = k < min(kBwdRound, r_end) ? a.vals[start + r_end - 1u - k] : 0xFFFFFFFFu;
+        }
+    };
+    auto load_round = [&]() {
+#pragma unroll
+        for (uint32_t u = 0; u < kPer; ++u) {
+            pf_idx[u] = nx_idx[u];
+            if (pf_idx[u] < a.n) {
+                const float4* p = reinterpret_cast<const float4*>(vsplats + pf_idx[u]);
+                pf_c[u] = __ldg(p + 0);
+                pf_tex[u] = __ldg(p + 1);
+                pf_co[u] = __ldg(p + 2);
             }
         }
     };
@@ -678,14 +682,19 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
     };
     const float2 one = f2(1.0f, 1.0f), mone = f2(-1.0f, -1.0f);
     const uint32_t block = 4u * warp + (lane >> 3), j = lane & 7u;
-    load_round(max_last, 0u);
+    load_indices(max_last, 0u);
+    load_round();
+    load_indices(max_last > kBwdRound ? max_last - kBwdRound : 0u, 32u);
     store_round(max_last, 0u);
     __syncthreads();
     uint32_t turn = 0;
     for (uint32_t r_end = max_last; r_end > 0;) {
         const uint32_t n = min(kBwdRound, r_end), next_end = r_end - n;
         turn ^= 32u;
-        if (next_end) load_round(next_end, turn);
+        if (next_end) {
+            load_round();
+            load_indices(next_end > kBwdRound ? next_end - kBwdRound : 0u, turn ^ 32u);
+        }
         const uint32_t steps = build_block_lists<kBwdRound>(SM.lists, warp, lane, n, [&](uint32_t e) {
             uint32_t m = uint32_t(SM.mask[e]) >> (4u * warp);
 #pragma unroll
