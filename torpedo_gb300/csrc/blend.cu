@@ -392,6 +392,17 @@ __device__ __forceinline__ bool next_tile(FrameCtl* ctl, uint32_t slot, const ui
     return true;
 }
 
+// Item i of the tiles in class order (buckets as launch_list_classes fills
+// them): the class whose tiles item i falls among, by a scan of their counts.
+__device__ __forceinline__ uint32_t class_tile(const FrameCtl* ctl, const uint32_t* buckets, uint32_t n_tiles, uint32_t i) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t incl = warp_inclusive_scan(lane < kListClasses ? __ldcg(&ctl->list_class[lane]) : 0u);
+    const uint32_t after = __ballot_sync(0xFFFFFFFFu, incl > i);  // classes that end past item i
+    const uint32_t c = after ? uint32_t(__ffs(after) - 1) : 0u;
+    const uint32_t before = c ? __shfl_sync(0xFFFFFFFFu, incl, c - 1u) : 0u;
+    return after ? __ldcg(buckets + size_t(c) * n_tiles + (i - before)) : i;
+}
+
 // One CTA per tile, or (kPersistent) one CTA per resident slot taking tiles
 // from the queue.
 template <uint32_t kRound, bool kPersistent, bool kState>
@@ -403,9 +414,11 @@ __global__ void __launch_bounds__(kFwdThreads, fwd_min_blocks<kRound>()) blend_k
     if (a.ctl->status & (kStatusFatal | kStatusKeyOverflow)) return;
     if constexpr (kPersistent) {
         uint32_t tile;
-        while (next_tile(a.ctl, kTicketBlend, nullptr, a.n_tiles, tile)) blend_tile<kRound, kState>(a, tile, S);
+        while (next_tile(a.ctl, kTicketBlend, nullptr, a.n_tiles, tile))
+            blend_tile<kRound, kState>(a, a.list_buckets ? class_tile(a.ctl, a.list_buckets, a.n_tiles, tile) : tile, S);
     } else {
-        blend_tile<kRound, kState>(a, blockIdx.x, S);
+        blend_tile<kRound, kState>(
+            a, a.list_buckets ? class_tile(a.ctl, a.list_buckets, a.n_tiles, blockIdx.x) : blockIdx.x, S);
     }
 }
 
@@ -799,14 +812,49 @@ __global__ void __launch_bounds__(kAdjThreads, bwd_min_blocks<kBwdRound>())
     }
 }
 
+// The blend's order: tiles by octave of their list length, each class in a
+// bucket of its own that a CTA's 1024 tiles fill from a cursor, so one launch
+// is enough.
+constexpr uint32_t kOrderThreads = 256;
+constexpr uint32_t kOrderTiles = 1024;
+
+__global__ void __launch_bounds__(kOrderThreads)
+    list_classes_kernel(const uint32_t* __restrict__ ranges, uint32_t n_tiles, FrameCtl* __restrict__ ctl,
+                        uint32_t* __restrict__ buckets) {
+    __shared__ uint32_t count[kListClasses], base[kListClasses];
+    pdl_wait();     // launched as a dependent of the key sort's last pass: its ranges
+    pdl_trigger();  // the blend may be scheduled; it waits for this grid
+    const uint32_t tid = threadIdx.x;
+    if (tid < kListClasses) count[tid] = 0;
+    __syncthreads();
+    constexpr uint32_t kPer = kOrderTiles / kOrderThreads;
+    uint32_t cls[kPer], rank[kPer];
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u) {
+        const uint32_t t = blockIdx.x * kOrderTiles + u * kOrderThreads + tid;
+        cls[u] = rank[u] = 0;
+        if (t < n_tiles) {
+            const uint2 r = reinterpret_cast<const uint2*>(ranges)[t];
+            const uint32_t len = r.y > r.x ? r.y - r.x : 0u;
+            cls[u] = kListClasses - 1u - min(kListClasses - 1u, 32u - uint32_t(__clz(len)));
+            rank[u] = atomicAdd(&count[cls[u]], 1u);
+        }
+    }
+    __syncthreads();
+    if (tid < kListClasses && count[tid]) base[tid] = atomicAdd(&ctl->list_class[tid], count[tid]);
+    __syncthreads();
+#pragma unroll
+    for (uint32_t u = 0; u < kPer; ++u) {
+        const uint32_t t = blockIdx.x * kOrderTiles + u * kOrderThreads + tid;
+        if (t < n_tiles) buckets[size_t(cls[u]) * n_tiles + base[cls[u]] + rank[u]] = t;
+    }
+}
+
 // The tiles in class order, the classes counted by the blend: a CTA counts
 // its 1024 tiles per class, takes that many places of each class at once, and
 // its tiles fill them. (One CTA counting list lengths for all tiles took 182 us
 // for the 259,000 tiles of 8 views of 2160p; and a list's length
 // says little about a walk that stops early.)
-constexpr uint32_t kOrderThreads = 256;
-constexpr uint32_t kOrderTiles = 1024;
-
 __global__ void __launch_bounds__(kOrderThreads)
     tile_order_kernel(const uint32_t* __restrict__ tile_len, uint32_t n_tiles, FrameCtl* __restrict__ ctl,
                       uint32_t* __restrict__ order) {
@@ -858,6 +906,23 @@ __global__ void __launch_bounds__(kOrderThreads)
 }
 
 }  // namespace
+
+// Between one and five waves of CTAs (8 per SM). In one wave every tile starts
+// at once; in many, the end of the launch is short beside it and the order's
+// own launch (3 us) is lost: blend with and without the order, its launch
+// included, 120,000 Gaussians at 801x603 60 and 71 us, 500,000 at 720p 90 and
+// 99, at 1080p (8160 tiles) 144 and 150, but 1M spread evenly at 720p 147 and
+// 145, at 1080p 254 and 250, 3M at 2160p 763 and 751.
+bool blend_takes_list_order(uint32_t n_tiles, int num_sms) {
+    const uint32_t wave = 8u * uint32_t(num_sms > 0 ? num_sms : 148);
+    return n_tiles > wave && n_tiles <= 5u * wave;
+}
+
+void launch_list_classes(const uint32_t* ranges, uint32_t n_tiles, FrameCtl* ctl, uint32_t* buckets, cudaStream_t s) {
+    if (n_tiles == 0) return;
+    launch_dependent(list_classes_kernel, dim3((n_tiles + kOrderTiles - 1) / kOrderTiles), dim3(kOrderThreads), 0, s,
+                     ranges, n_tiles, ctl, buckets);
+}
 
 void launch_tile_order(const uint32_t* tile_len, uint32_t n_tiles, FrameCtl* ctl, uint32_t* order, cudaStream_t s) {
     if (n_tiles == 0) return;

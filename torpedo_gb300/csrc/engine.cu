@@ -108,6 +108,8 @@ struct tpd_engine {
     uint64_t total_pixels = 0;
     uint32_t* d_tile_view = nullptr;
     uint32_t* d_tile_len = nullptr;    // per tile, list entries up to its last contributor (frames keeping the adjoint's inputs)
+    uint32_t* d_list_buckets = nullptr;  // tiles by class of their list length, for the blend
+    uint64_t list_bucket_cap = 0;
     uint32_t* d_tile_order = nullptr;  // tiles by decreasing d_tile_len, for the blend adjoint
     uint64_t* d_image_offset = nullptr;
 
@@ -496,6 +498,10 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     ba.views = e->d_views;
     ba.tile_view = e->n_views > 1 ? e->d_tile_view : nullptr;
     ba.n_tiles = e->total_tiles;
+    if (blend_takes_list_order(e->total_tiles, e->num_sms)) {
+        launch_list_classes(e->d_ranges, e->total_tiles, e->d_ctl, e->d_list_buckets, s);
+        ba.list_buckets = e->d_list_buckets;
+    }
     ba.image = e->d_image;
     ba.image_offset = e->n_views > 1 ? e->d_image_offset : nullptr;
     ba.final_T = state ? e->d_final_T : nullptr;
@@ -632,6 +638,10 @@ int set_views_internal(tpd_engine* e, const tpd_view* views, uint32_t nv) {
         TPD_CUDA(e, dalloc(e->d_tile_order, tiles));
         TPD_CUDA(e, dalloc(e->d_tile_len, tiles));
         e->tile_cap = tiles;
+    }
+    if (blend_takes_list_order(tiles, e->num_sms) && uint64_t(tiles) * kListClasses > e->list_bucket_cap) {
+        TPD_CUDA(e, dalloc(e->d_list_buckets, uint64_t(tiles) * kListClasses));
+        e->list_bucket_cap = uint64_t(tiles) * kListClasses;
     }
     if (!e->d_image_offset) TPD_CUDA(e, dalloc(e->d_image_offset, kMaxViews));
     TPD_CUDA(e, cudaMemcpy(e->d_tile_view, tile_view.data(), tiles * 4ull, cudaMemcpyHostToDevice));
@@ -818,6 +828,7 @@ void tpd_destroy(tpd_engine* e) {
     dfree(e->d_tile_view);
     dfree(e->d_tile_order);
     dfree(e->d_tile_len);
+    dfree(e->d_list_buckets);
     dfree(e->d_image_offset);
     dfree(e->d_splats);
     dfree(e->d_offsets);

@@ -74,6 +74,7 @@ __global__ void frame_begin_kernel(FrameCtl* ctl, const float* transforms, uint3
     const uint32_t t = threadIdx.x;
     for (uint32_t i = t; i < 32; i += blockDim.x) ctl->ticket[i] = 0;
     for (uint32_t i = t; i < 128; i += blockDim.x) ctl->tile_hist[i] = 0;
+    for (uint32_t i = t; i < 32; i += blockDim.x) ctl->list_class[i] = 0;
     for (uint32_t i = t; i < 8 * 256; i += blockDim.x) {
         (&ctl->sort_hist[0][0])[i] = 0;
         (&ctl->depth_hist[0][0])[i] = 0;

@@ -30,7 +30,9 @@ struct FrameCtl {
     uint32_t pad;
     uint32_t tile_hist[128];    // tiles by class of their walk length (tile_class), counted by the blend
     uint32_t tile_cursor[128];  // tiles of each class that the tile order has placed (0 at rest)
+    uint32_t list_class[32];    // tiles by class of their list length, as launch_list_classes places them
 };
+constexpr uint32_t kListClasses = 16;
 
 // Entity matrices: rows 0..2 of view*model and rows 0..3 of projview*model.
 constexpr int kEntityMatFloats = 28;
@@ -207,6 +209,12 @@ void launch_small_sort(const uint64_t* keys, const uint32_t* vals, uint64_t* key
 void launch_sort_begin(FrameCtl* ctl, uint32_t total, cudaStream_t s);
 
 
+// The tiles by class of their list length (octaves, longest first), for the
+// blend: class c's tiles fill buckets[c n_tiles ..), ctl->list_class[c] of them.
+void launch_list_classes(const uint32_t* ranges, uint32_t n_tiles, FrameCtl* ctl, uint32_t* buckets, cudaStream_t s);
+// Whether a frame of n_tiles blends in that order.
+bool blend_takes_list_order(uint32_t n_tiles, int num_sms);
+
 struct BlendArgs {
     const Splat* splats;      // n_views x n (view-major)
     uint32_t n;               // Gaussians per view
@@ -217,6 +225,7 @@ struct BlendArgs {
     const ViewConst* views;   // device, n_views entries
     const uint32_t* tile_view;  // per global tile: view index (nullptr: single view 0)
     uint32_t n_tiles;
+    const uint32_t* list_buckets;  // nullable: CTAs take the tiles in launch_list_classes' order
     float* image;             // HWC float3 per view, packed per view at image_offset[view]
     const uint64_t* image_offset;  // per view pixel offset (nullptr: 0)
     // per pixel: final transmittance and list entries up to the last
