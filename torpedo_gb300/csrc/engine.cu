@@ -133,6 +133,8 @@ struct tpd_engine {
     uint32_t* d_vals[2] = {nullptr, nullptr};
     uint64_t* d_desc_sort = nullptr;
     uint32_t* d_sort_work = nullptr;  // counted key-sort passes: partition counts and offsets
+    uint32_t* d_strip_starts = nullptr;  // first key slot of every strip (frames that take strips)
+    uint64_t strip_cap = 0;
     uint32_t* d_part_first = nullptr;  // first item of every 4096-key partition
     uint32_t* d_ranges = nullptr;
     uint64_t pixel_cap = 0, tile_cap = 0;
@@ -276,6 +278,19 @@ int ensure_splat_buffers(tpd_engine* e) {
     return TPD_OK;
 }
 
+// The strips' buffer, for the current views and key capacity. Without the
+// memory for it the frame's keys are sorted as they are.
+void ensure_strips(tpd_engine* e) {
+    if (e->n_views == 0 || e->strip_cap >= e->capacity) return;
+    if (!takes_strips(e->n_views, grid_x(e->vw[0]), grid_y(e->vh[0]))) return;
+    invalidate_graph(e);
+    e->strip_cap = 0;
+    if (dalloc(e->d_strip_starts, e->capacity) == cudaSuccess)
+        e->strip_cap = e->capacity;
+    else
+        cudaGetLastError();
+}
+
 int ensure_key_capacity(tpd_engine* e, uint64_t want) {
     if (want <= e->capacity) return TPD_OK;
     if (want > 0x7FFFFFFFull) return fail(e, TPD_ERR_CAPACITY, "key count exceeds 2^31-1");
@@ -292,6 +307,7 @@ int ensure_key_capacity(tpd_engine* e, uint64_t want) {
     TPD_CUDA(e, cudaMemset(e->d_sort_work, 0, words * 4));
     TPD_CUDA(e, dalloc(e->d_part_first, want / 4096 + 1));
     e->capacity = want;
+    ensure_strips(e);
     return TPD_OK;
 }
 
@@ -460,6 +476,13 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
     ka.tile_bits = e->key_bits - 32;
     ka.desc = e->d_desc_pre;
     ka.counted_work = counted ? e->d_sort_work : nullptr;
+    // strips, with buffers and look-back descriptors for them (settings that
+    // ask for another form of the passes keep the keys)
+    const bool strips = counted && e->settings.sort_ctas_per_sm != 2 && e->strip_cap >= e->capacity &&
+                        takes_strips(e->n_views, grid_x(e->vw[0]), grid_y(e->vh[0])) &&
+                        (items + kKeygenPart - 1) / kKeygenPart <= sort_desc_entries(cap);
+    ka.strips = strips;
+    ka.strip_desc = e->d_desc_sort;
     ka.ctl = e->d_ctl;
     ka.spin_limit = spin;
     ka.never_publish = e->settings.test_never_publish;
@@ -483,8 +506,15 @@ void enqueue_frame(tpd_engine* e, bool io = true, bool state = true, uint32_t* r
         kp.precounted = true;  // keygen counted the first pass
         kp.ctas_per_sm = e->settings.sort_ctas_per_sm == 2 ? 2 : 3;
     }
-    e->sorted_in_alt = launch_sort(e->d_tiles[0], e->d_vals[0], e->d_tiles[1], e->d_vals[1], cap, kp, e->d_desc_sort,
-                                   e->d_ctl, spin, e->num_sms, s);
+    if (strips) {
+        StripSort ss{e->d_tiles[0], e->d_vals[0], e->d_tiles[1], e->d_vals[1], e->d_strip_starts, e->d_part_first, cap,
+                     e->d_sort_work, e->d_ranges, e->total_tiles, grid_x(e->vw[0]), e->d_ctl};
+        launch_strip_sort(ss, s);
+        e->sorted_in_alt = false;
+    } else {
+        e->sorted_in_alt = launch_sort(e->d_tiles[0], e->d_vals[0], e->d_tiles[1], e->d_vals[1], cap, kp,
+                                       e->d_desc_sort, e->d_ctl, spin, e->num_sms, s);
+    }
     mark(4);
     const int b = e->sorted_in_alt ? 1 : 0;
     mark(5);  // (tile ranges come out of the key sort's last pass)
@@ -646,6 +676,7 @@ int set_views_internal(tpd_engine* e, const tpd_view* views, uint32_t nv) {
     if (!e->d_image_offset) TPD_CUDA(e, dalloc(e->d_image_offset, kMaxViews));
     TPD_CUDA(e, cudaMemcpy(e->d_tile_view, tile_view.data(), tiles * 4ull, cudaMemcpyHostToDevice));
     TPD_CUDA(e, cudaMemcpy(e->d_image_offset, img_off.data(), nv * 8ull, cudaMemcpyHostToDevice));
+    ensure_strips(e);
     return ensure_splat_buffers(e);
 }
 
@@ -844,6 +875,7 @@ void tpd_destroy(tpd_engine* e) {
     dfree(e->d_desc_sort);
     dfree(e->d_sort_work);
     dfree(e->d_part_first);
+    dfree(e->d_strip_starts);
     dfree(e->d_keys64);
     dfree(e->d_ranges);
     dfree(e->d_image);

@@ -30,6 +30,7 @@
 #include "tpd_counted.cuh"
 #include "tpd_kernels.h"
 #include "tpd_scan.cuh"
+#include "tpd_slots.cuh"
 
 namespace tpd {
 namespace {
@@ -46,8 +47,15 @@ struct ItemRect {
     uint32_t t0, wgx, cnt, gi;
 };
 
+// For the strips of an item: its rectangle's first column, first row and height
+// packed as a strip's key (strip_key), and its width (its strips).
+struct ItemStrips {
+    uint32_t key, w;
+};
+
 __device__ __forceinline__ ItemRect item_rect(uint32_t item, bool valid, float4 texel, uint32_t n_items, uint32_t n,
-                                              const ViewConst* __restrict__ views, FrameCtl* ctl) {
+                                              const ViewConst* __restrict__ views, FrameCtl* ctl, ItemStrips& strips) {
+    strips = ItemStrips{0u, 0u};
     uint32_t w = 1, h = 0, gx = 1, gi = 0, t0 = 0;
     if (valid && TPD_INBOUNDS(ctl, 21, item, n_items)) {
         const uint32_t v = n_items == n ? 0u : item / n;  // one view: no division
@@ -61,6 +69,7 @@ __device__ __forceinline__ ItemRect item_rect(uint32_t item, bool valid, float4 
                 w = x1 - x0;
                 h = y1 - y0;
                 t0 = vc.tile_base + y0 * gx + x0;
+                strips = ItemStrips{strip_key(x0, y0, h), w};
             }
         }
     }
@@ -86,17 +95,24 @@ __device__ __forceinline__ ItemRect item_rect(uint32_t item, bool valid, float4 
 // publishes its aggregate soon. Bound by the gathers (32 bytes of every
 // 48-byte splat in depth order) and the look-back's latency.
 struct ScanItemsSmem {
-    uint32_t wtot[kScanItemsWarps];  // key counts of the warps' items
-    uint32_t ticket;                 // the partition being worked on
-    uint32_t excl;                   // the partition's exclusive prefix
+    uint32_t wtot[2][kScanItemsWarps];  // key counts of the warps' items; strip counts
+    uint32_t ticket;                    // the partition being worked on
+    uint32_t excl[2];                   // the partition's exclusive prefixes
 };
 
-__global__ void __launch_bounds__(kScanItemsThreads)
+// kStrips: the items' strips (one per column of the rectangle) are scanned as
+// well, by a second look-back beside the first, and item_info and part_first
+// are those of the strip slots. (Registers for six CTAs per SM, as without: 48 ->
+// 45 us with the expansion, 1M Gaussians at 1080p.)
+template <bool kStrips>
+__global__ void __launch_bounds__(kScanItemsThreads, 6)
     scan_items_kernel(const Splat* __restrict__ splats, const uint32_t* __restrict__ items,
                       const uint32_t* __restrict__ items_other, uint32_t n_items, uint32_t n,
                       const ViewConst* __restrict__ views, uint32_t* __restrict__ offsets,
                       uint4* __restrict__ item_info, uint32_t* __restrict__ part_first, uint32_t capacity,
-                      uint32_t* __restrict__ ranges, uint32_t n_tiles, uint64_t* desc, FrameCtl* ctl, uint32_t spin_limit, uint32_t never_publish) {
+                      uint32_t* __restrict__ ranges, uint32_t n_tiles, uint64_t* desc, uint64_t* strip_desc, FrameCtl* ctl, uint32_t spin_limit,
+                      uint32_t never_publish) {
+    constexpr uint32_t kSums = kStrips ? 2u : 1u;
     __shared__ ScanItemsSmem S;
     pdl_wait();     // launched as a dependent of the depth sort's last pass: its order is read below
     pdl_trigger();  // expand_keys_kernel may be scheduled (it waits for this grid)
@@ -129,52 +145,69 @@ __global__ void __launch_bounds__(kScanItemsThreads)
             texel[c] = item[c] < n_items ? reinterpret_cast<const float4*>(splats + item[c])[1]
                                          : make_float4(0.f, 0.f, 0.f, 0.f);
         ItemRect rect[kScanItemsChunks];
-        uint32_t incl[kScanItemsChunks], ctot[kScanItemsChunks], wtotal = 0, vis = 0;
+        ItemStrips strips[kScanItemsChunks];
+        // [0]: keys, [1]: strips
+        uint32_t incl[kSums][kScanItemsChunks], ctot[kSums][kScanItemsChunks], wtotal[kSums] = {}, vis = 0;
 #pragma unroll
         for (uint32_t c = 0; c < kScanItemsChunks; ++c) {
-            rect[c] = item_rect(item[c], r0 + 32u * c < count, texel[c], n_items, n, views, ctl);
-            incl[c] = warp_inclusive_scan(rect[c].cnt);
-            ctot[c] = __shfl_sync(0xFFFFFFFFu, incl[c], 31);
-            wtotal += ctot[c];
+            rect[c] = item_rect(item[c], r0 + 32u * c < count, texel[c], n_items, n, views, ctl, strips[c]);
+#pragma unroll
+            for (uint32_t u = 0; u < kSums; ++u) {
+                incl[u][c] = warp_inclusive_scan(u ? strips[c].w : rect[c].cnt);
+                ctot[u][c] = __shfl_sync(0xFFFFFFFFu, incl[u][c], 31);
+                wtotal[u] += ctot[u][c];
+            }
             vis += rect[c].cnt ? 1u : 0u;
         }
         vis = warp_sum(vis);
         if (lane == 0) {
-            S.wtot[warp] = wtotal;
+#pragma unroll
+            for (uint32_t u = 0; u < kSums; ++u) S.wtot[u][warp] = wtotal[u];
             if (vis) atomicAdd(&ctl->visible, vis);
         }
         __syncthreads();
-        uint32_t wbase = 0, total = 0;
+        uint32_t wbase[kSums] = {}, total[kSums] = {};
 #pragma unroll
-        for (uint32_t w = 0; w < kScanItemsWarps; ++w) {
-            const uint32_t sw = S.wtot[w];
-            wbase += w < warp ? sw : 0u;
-            total += sw;
-        }
-        if (warp == 0) {
-            const uint32_t ex = warp_lookback(desc, part, total, tag, &ctl->status, spin_limit, never_publish != 0);
+        for (uint32_t u = 0; u < kSums; ++u)
+#pragma unroll
+            for (uint32_t w = 0; w < kScanItemsWarps; ++w) {
+                const uint32_t sw = S.wtot[u][w];
+                wbase[u] += w < warp ? sw : 0u;
+                total[u] += sw;
+            }
+        if (warp < kSums) {
+            const bool keys = warp == 0;
+            const uint32_t sum = keys ? total[0] : total[kSums - 1u];
+            const uint32_t ex = warp_lookback(keys ? desc : strip_desc, part, sum, tag, &ctl->status, spin_limit,
+                                              never_publish != 0);
             if (lane == 0) {
-                S.excl = ex;
+                S.excl[warp] = ex;
                 if (part == nparts - 1u) {
-                    ctl->total_keys = ex + total;
-                    if (ex + total > capacity) atomicOr(&ctl->status, kStatusKeyOverflow);
+                    (keys ? ctl->total_keys : ctl->total_strips) = ex + sum;
+                    if (keys && ex + sum > capacity) atomicOr(&ctl->status, kStatusKeyOverflow);
                 }
             }
         }
         __syncthreads();
-        uint32_t base = S.excl + wbase;
+        uint32_t base[kSums];
+#pragma unroll
+        for (uint32_t u = 0; u < kSums; ++u) base[u] = S.excl[u] + wbase[u];
 #pragma unroll
         for (uint32_t c = 0; c < kScanItemsChunks; ++c) {
-            const uint32_t r = r0 + 32u * c, first = base + incl[c] - rect[c].cnt;
+            const uint32_t r = r0 + 32u * c, first_key = base[0] + incl[0][c] - rect[c].cnt;
+            const uint32_t slots = kStrips ? strips[c].w : rect[c].cnt;
+            const uint32_t first = kStrips ? base[kSums - 1u] + incl[kSums - 1u][c] - slots : first_key;
             if (r < count) {
-                offsets[r] = first;
-                item_info[r] = make_uint4(rect[c].t0, rect[c].wgx, first, rect[c].gi);
-                // (keys past the capacity are not written: the frame is flagged)
-                const uint32_t end = min(first + rect[c].cnt, capacity);
+                offsets[r] = first_key;
+                item_info[r] = kStrips ? make_uint4(strips[c].key, 0u, first, rect[c].gi)
+                                       : make_uint4(rect[c].t0, rect[c].wgx, first, rect[c].gi);
+                // (slots past the capacity are not written: the frame is flagged)
+                const uint32_t end = min(first + slots, capacity);
                 for (uint32_t p = (first + kCountedTile - 1) / kCountedTile; p * kCountedTile < end; ++p)
                     part_first[p] = r;
             }
-            base += ctot[c];
+#pragma unroll
+            for (uint32_t u = 0; u < kSums; ++u) base[u] += ctot[u][c];
         }
         __syncthreads();  // S is rewritten for the next partition
     }
@@ -216,11 +249,11 @@ __global__ void __launch_bounds__(kExpandThreads, 4)
     constexpr bool kCounted = kDig != 0;
     constexpr uint32_t kRows = kCounted ? 1u : kTileDigitsMax, kWidth = kCounted ? kDig : 256u;
     __shared__ uint32_t digits[kRows][kWidth];
-    __shared__ uint32_t wmax[kExpandThreads / 32], wsum[kExpandThreads / 32];
+    __shared__ uint32_t wsum[kExpandThreads / 32];
     __shared__ bool s_last;
     pdl_wait();
     pdl_trigger();
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x;
     const uint32_t K = (ctl->status & (kStatusFatal | kStatusKeyOverflow)) ? 0u : min(ctl->total_keys, capacity);
     const uint32_t nparts = min((K + kCountedTile - 1) / kCountedTile, max_parts);
     const uint32_t part = blockIdx.x;
@@ -231,41 +264,9 @@ __global__ void __launch_bounds__(kExpandThreads, 4)
     const uint32_t last = part + 1u < nparts ? min(part_first[part + 1u], n_all - 1u) : n_all - 1u;
     // an item has at least one key: a partition holds at most kCountedTile items
     const uint32_t m = min(last - first + 1u, kCountedTile + 1u);
-    uint4* own4 = reinterpret_cast<uint4*>(owner);
-    own4[2 * tid] = own4[2 * tid + 1] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (uint32_t p = 0; p < kRows * kWidth / kExpandThreads; ++p) (&digits[0][0])[p * kExpandThreads + tid] = 0;
-    __syncthreads();
-    for (uint32_t k = tid + 1u; k < m; k += kExpandThreads) {  // (item 0 owns slot 0: the map's zeros)
-        const uint32_t slot = item_info[first + k].z - base;
-        if (slot < cnt) owner[slot] = uint16_t(k);
-    }
-    __syncthreads();
-    // prefix maximum over the map: 16 consecutive slots per thread
-    uint16_t o[kExpandSlots];
-    {
-        const uint4 a = own4[2 * tid], b = own4[2 * tid + 1];
-        *reinterpret_cast<uint4*>(o) = a;
-        *reinterpret_cast<uint4*>(o + 8) = b;
-    }
-#pragma unroll
-    for (uint32_t q = 1; q < kExpandSlots; ++q) o[q] = max(o[q], o[q - 1]);
-    uint32_t before = o[kExpandSlots - 1];
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, before, d);
-        if (lane >= d) before = max(before, x);
-    }
-    if (lane == 31) wmax[warp] = before;
-    before = __shfl_up_sync(0xFFFFFFFFu, before, 1);
-    if (lane == 0) before = 0;
-    __syncthreads();
-    for (uint32_t w = 0; w < warp; ++w) before = max(before, wmax[w]);
-#pragma unroll
-    for (uint32_t q = 0; q < kExpandSlots; ++q) o[q] = max(o[q], uint16_t(before));
-    own4[2 * tid] = *reinterpret_cast<const uint4*>(o);
-    own4[2 * tid + 1] = *reinterpret_cast<const uint4*>(o + 8);
-    __syncthreads();
+    slot_owners(owner, m, cnt, wsum, [&](uint32_t k) { return item_info[first + k].z - base; });
     const uint32_t ndig = kCounted ? 1u : min(kTileDigitsMax, (tile_bits + 7u) / 8u);
     // kFull: a whole partition (all but the last), without per-slot checks
     auto expand = [&](auto full_tag) {
@@ -338,9 +339,76 @@ __global__ void __launch_bounds__(kExpandThreads, 4)
     }
 }
 
+// The strips' form (see sort.cu): a slot is a strip, one column of its item's
+// rectangle. Its key is that column with the rectangle's rows (strip_key), its
+// value the Gaussian. Counted per partition and column: the strips and, as
+// digits 256 and up, their heights (the keys they hold). Bound by latency, as
+// the keys' form: 3M Gaussians at 2160p 67 us (242 for the keys), 1M at 1080p
+// 20 (35).
+__global__ void __launch_bounds__(kExpandThreads, 4)
+    expand_strips_kernel(const uint4* __restrict__ item_info, const uint32_t* __restrict__ part_first,
+                         uint32_t* __restrict__ strips, uint32_t* __restrict__ vals, uint32_t n_items,
+                         uint32_t capacity, uint32_t max_parts, uint32_t* __restrict__ work, FrameCtl* ctl) {
+    __shared__ __align__(16) uint16_t owner[kCountedTile];  // item of each slot, from the partition's first
+    __shared__ __align__(8) uint32_t sums[512];              // strips by column, heights by column
+    __shared__ uint32_t wsum[kExpandThreads / 32];
+    __shared__ bool s_last;
+    pdl_wait();
+    pdl_trigger();
+    const uint32_t tid = threadIdx.x;
+    const uint32_t K = (ctl->status & (kStatusFatal | kStatusKeyOverflow)) ? 0u : min(ctl->total_strips, capacity);
+    const uint32_t nparts = min((K + kCountedTile - 1) / kCountedTile, max_parts);
+    const uint32_t part = blockIdx.x;
+    if (part >= nparts) return;  // (uniform)
+    const uint32_t base = part * kCountedTile, cnt = min(kCountedTile, K - base);
+    const uint32_t n_all = min(ctl->depth_count, n_items);
+    const uint32_t first = min(part_first[part], n_all - 1u);
+    const uint32_t last = part + 1u < nparts ? min(part_first[part + 1u], n_all - 1u) : n_all - 1u;
+    const uint32_t m = min(last - first + 1u, kCountedTile + 1u);
+    sums[tid] = sums[tid + 256u] = 0u;
+    slot_owners(owner, m, cnt, wsum, [&](uint32_t k) { return item_info[first + k].z - base; });
+#pragma unroll
+    for (uint32_t q = 0; q < kExpandSlots / 4u; ++q) {
+        const uint32_t slot = q * (4u * kExpandThreads) + 4u * tid;
+        if (slot >= cnt) break;
+        const uint2 own = *reinterpret_cast<const uint2*>(owner + slot);  // four 16-bit owners
+        const uint32_t o[4] = {own.x & 0xFFFFu, own.x >> 16, own.y & 0xFFFFu, own.y >> 16};
+        uint32_t key[4], gi[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            const uint4 info = __ldg(item_info + first + o[u]);
+            key[u] = info.x + (base + slot + u - info.z);  // (the columns stay below 256)
+            gi[u] = info.w;
+        }
+        if (slot + 4u <= cnt) {
+            *reinterpret_cast<uint4*>(strips + base + slot) = make_uint4(key[0], key[1], key[2], key[3]);
+            *reinterpret_cast<uint4*>(vals + base + slot) = make_uint4(gi[0], gi[1], gi[2], gi[3]);
+        } else {
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u)
+                if (slot + u < cnt) {
+                    strips[base + slot + u] = key[u];
+                    vals[base + slot + u] = gi[u];
+                }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u)
+            if (slot + u < cnt) {
+                atomicAdd(&sums[strip_col(key[u])], 1u);
+                atomicAdd(&sums[256u + strip_col(key[u])], strip_height(key[u]));
+            }
+    }
+    __syncthreads();
+    RowDigits<2> count;
+    const uint2 c = reinterpret_cast<const uint2*>(sums)[tid];
+    count.v[0] = c.x;
+    count.v[1] = c.y;
+    counted_finish<512>(CountedWork<512>(work, max_parts), nparts, part, count, wsum, s_last);
+}
+
 int scan_items_setup() {
     int r = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, scan_items_kernel, kScanItemsThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, scan_items_kernel<false>, kScanItemsThreads, 0);
     return r > 0 ? r : 1;
 }
 
@@ -352,10 +420,16 @@ void launch_keygen(const KeygenArgs& a, int num_sms, cudaStream_t s) {
     const int per_sm = device_once(scan_items_setup);  // resident CTAs per SM
     const uint64_t cap = uint64_t(num_sms > 0 ? num_sms : 148) * uint64_t(per_sm);  // persistent
     const uint64_t blocks = parts < cap ? parts : cap;
-    launch_dependent(scan_items_kernel, dim3(unsigned(blocks)), dim3(kScanItemsThreads), 0, s, a.splats, a.items,
+    launch_dependent(a.strips ? scan_items_kernel<true> : scan_items_kernel<false>, dim3(unsigned(blocks)), dim3(kScanItemsThreads), 0, s, a.splats, a.items,
                      a.items_other, a.n_items, a.n, a.views, a.offsets, a.item_info, a.part_first, a.capacity,
-                     a.ranges, a.n_tiles, a.desc, a.ctl, a.spin_limit, a.never_publish);
+                     a.ranges, a.n_tiles, a.desc, a.strip_desc, a.ctl, a.spin_limit, a.never_publish);
     const uint32_t max_parts = std::max(1u, uint32_t((uint64_t(a.capacity) + kCountedTile - 1) / kCountedTile));
+    if (a.strips) {
+        launch_dependent(expand_strips_kernel, dim3(max_parts), dim3(kExpandThreads), 0, s,
+                         static_cast<const uint4*>(a.item_info), static_cast<const uint32_t*>(a.part_first), a.tiles,
+                         a.vals, a.n_items, a.capacity, max_parts, a.counted_work, a.ctl);
+        return;
+    }
     const auto expand = !a.counted_work                                ? expand_keys_kernel<0>
                         : counted_digit_bits(a.tile_bits) > 8 ? expand_keys_kernel<512>
                                                               : expand_keys_kernel<256>;

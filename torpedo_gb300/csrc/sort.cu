@@ -36,6 +36,7 @@
 #include "tpd_counted.cuh"
 #include "tpd_kernels.h"
 #include "tpd_scan.cuh"
+#include "tpd_slots.cuh"
 
 namespace tpd {
 namespace {
@@ -534,14 +535,110 @@ __global__ void __launch_bounds__(256, 6) partition_count_kernel(const KeyT* __r
     counted_finish<kDig>(CountedWork<kDig>(work, max_parts), nparts, part, total, wsum, last);
 }
 
+// Strips. A rectangle of w x h tiles is w h keys but w column strips, and a key
+// is its strip's column and one of its rows. So a frame of one view sorts the
+// strips by column (a counted pass whose heights are counted too, which gives
+// each sorted strip its first key slot), and its last pass, by row, makes the
+// keys of 4096 consecutive slots from their strips instead of loading them:
+// (row, column, depth) order with the keys ranked and moved once, not twice.
+// 3M Gaussians at 2160p, us: expand 242 -> 67, counts 110 -> 52, first scatter
+// 412 -> 98 (of strips), last 476 -> 480 (now with the expansion).
+
+// What a scatter moves.
+constexpr int kScatterPairs = 0;    // keys and values
+constexpr int kScatterLast = 1;     // the last pass: values, and the tile ranges
+constexpr int kScatterColumns = 2;  // strips, by column; also each strip's first key slot
+constexpr int kScatterRows = 3;     // the keys of column-sorted strips, by row: the last pass
+
+// Column-sorted strips (kScatterColumns writes them, kScatterRows expands them).
+struct StripList {
+    uint32_t *keys, *vals, *starts;  // strip_key, Gaussian, first key slot
+    uint32_t* part_first;            // the strip that holds the first slot of every 4096-key partition
+    uint32_t gx;                     // the image's tile columns
+};
+
+// The rows of every 4096-key partition of column-sorted strips: a strip covers
+// consecutive rows, so it adds one where its slots of the partition begin and
+// takes one where they end, and a prefix sum gives the counts (two shared
+// atomics per strip, none per key). kParts partitions per CTA: latency is all
+// it spends, of the loads and of the arrivals (keygen + key sort with 1 / 2 / 4
+// / 8 of them: 817 / 798 / 789 / 816 us for 3M Gaussians at 2160p, 150 / 148 /
+// 151 / 154 for 1M at 1080p, 98 / 101 / 102 / 106 for 2M seen from inside).
+template <uint32_t kParts>
+__global__ void __launch_bounds__(256, 6) strip_rows_kernel(StripList strips, uint32_t capacity, uint32_t max_parts,
+                                                            uint32_t* __restrict__ work, FrameCtl* ctl,
+                                                            uint32_t abort_mask) {
+    constexpr uint32_t kTile = 4096, kGroup = 256 / kParts;  // threads per partition
+    __shared__ __align__(16) uint32_t edges[kParts][260];
+    __shared__ uint32_t wsum[8];
+    __shared__ bool s_last;
+    pdl_wait();
+    pdl_trigger();
+    const uint32_t tid = threadIdx.x, at = tid % kGroup, group = tid / kGroup;
+    const bool off = ctl->status & abort_mask;
+    const uint32_t K = off ? 0u : min(ctl->total_keys, capacity), n_strips = min(ctl->total_strips, capacity);
+    const uint32_t nparts = min((K + kTile - 1) / kTile, max_parts);
+    const uint32_t part0 = blockIdx.x * kParts, part = part0 + group;
+    if (part0 >= nparts) return;  // (uniform)
+    const CountedWork<256> W(work, max_parts);
+    for (uint32_t k = tid; k < kParts * 260; k += 256) (&edges[0][0])[k] = 0;
+    uint32_t* edge = edges[group];
+    const uint32_t base = part * kTile, end = part < nparts ? base + min(kTile, K - base) : base;
+    uint32_t first = 1, last = 0;
+    if (part < nparts) {
+        first = min(strips.part_first[part], n_strips - 1u);
+        last = part + 1u < nparts ? min(strips.part_first[part + 1u], n_strips - 1u) : n_strips - 1u;
+    }
+    __syncthreads();
+    for (uint32_t q0 = first; q0 <= last; q0 += 4 * kGroup) {
+        uint32_t strip[4], start[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            const uint32_t q = q0 + kGroup * u + at;
+            strip[u] = q <= last ? strips.keys[q] : 0u;  // (no height: nothing is added)
+            start[u] = q <= last ? strips.starts[q] : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            const uint32_t lo = max(start[u], base), hi = min(start[u] + strip_height(strip[u]), end);
+            const uint32_t row = strip_row(strip[u]) + lo - start[u];
+            if (lo < hi && TPD_INBOUNDS(ctl, 23, row + hi - lo, 257)) {
+                atomicAdd(&edge[row], 1u);
+                atomicSub(&edge[row + hi - lo], 1u);
+            }
+        }
+    }
+    __syncthreads();
+    if (at < 32 && part < nparts) {  // a warp: rows 8 at .. 8 at + 7
+        uint32_t v[8], sum = 0;
+        *reinterpret_cast<uint4*>(v) = reinterpret_cast<const uint4*>(edge)[2 * at];
+        *reinterpret_cast<uint4*>(v + 4) = reinterpret_cast<const uint4*>(edge)[2 * at + 1];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) sum = v[k] += sum;
+        const uint32_t before = warp_inclusive_scan(sum) - sum;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) v[k] += before;
+        uint4* row = reinterpret_cast<uint4*>(W.rows + size_t(part) * 256);
+        row[2 * at] = *reinterpret_cast<const uint4*>(v);
+        row[2 * at + 1] = *reinterpret_cast<const uint4*>(v + 4);
+    }
+    counted_arrive<256, kParts>(W, nparts, part0, wsum, s_last);
+}
+constexpr uint32_t kStripParts = 2;
+
 // A partition of a scatter: its pairs reordered by digit, each in one 8-byte
 // slot (one store and one load per pair), one pad slot per 16 (pad16).
-template <uint32_t kDig>
+template <uint32_t kDig, int kMode>
 struct ScatterSmem {
     uint2 pairs[4096 + 4096 / 16];  // key, value
     uint32_t whist[8][kDig];        // per-warp digit counts, then the first slot of the warp's keys of each digit
     uint32_t gmap[kDig];            // global position of local index 0 of each digit
     uint32_t wsum[8];
+    uint32_t match[kMode >= kScatterColumns ? 8 : 1][kDig];  // strips: per warp and digit, the lanes that have it (0 at rest)
+    // columns: the local prefix of the heights, and the columns' offsets (strips,
+    // heights), then the key slot of local height 0 of each column
+    uint32_t hpre[kMode == kScatterColumns ? 4096 + 4096 / 16 : 1];
+    uint32_t hmap[kMode == kScatterColumns ? 512 : 2];
 };
 
 // kBits: the pass's digit width (1..9); the lanes with the same digit are
@@ -555,28 +652,38 @@ struct ScatterSmem {
 // give the range whatever the order (range.slang:18-35). Against writing the
 // keys too and comparing both neighbours of every key: 1M Gaussians at 1080p 57
 // -> 51 us, 3M at 2160p 573 -> 501.
+// Strips (kScatterColumns, kScatterRows; see above): the lanes of one digit are
+// found by an atomic OR into a word per (warp, digit), as 32 strips or keys in
+// a row seldom share one: 855 -> 816 us (keygen + key sort, 3M Gaussians at
+// 2160p). With keys, whose last pass has most of a warp on one digit, ballots
+// are faster (251 and 284 us for 8 views of 500,000). A CTA's strips are staged
+// in shared memory while their slots are marked: 798 -> 699 us against two
+// gathers per key.
 // What bounds it: the shared-memory pipe (75% busy with keys and values in
 // arrays of their own and the digit and warp offsets looked up apart) and the
 // integer pipe (63%: ballots). Pairs in one slot and merged offsets took both
 // passes and the count from 120 to 108 us at 1M Gaussians and 1080p; 64
 // registers for a fourth CTA per SM spill (118).
-template <int kMinBlocks, int kBits, bool kLast, typename KeyT>
+template <int kMinBlocks, int kBits, int kMode, typename KeyT>
 __global__ void __launch_bounds__(256, kMinBlocks)
     scatter_kernel(const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, KeyT* __restrict__ keys_out,
                    uint32_t* __restrict__ vals_out, uint32_t capacity, uint32_t shift, uint32_t bits,
                    uint32_t fixed_count, uint32_t max_parts, uint32_t* __restrict__ work, FrameCtl* ctl,
-                   uint32_t* __restrict__ ranges, uint32_t n_tiles, uint32_t abort_mask, bool keys_just_written) {
+                   uint32_t* __restrict__ ranges, uint32_t n_tiles, uint32_t abort_mask, bool keys_just_written, StripList strips) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr bool kLast = kMode == kScatterLast || kMode == kScatterRows;
+    constexpr bool kMatch = kMode >= kScatterColumns;  // lanes of one digit by shared atomics, not by ballots
     constexpr uint32_t kItems = 16, kSortTile = 4096, kWarps = 8;
     constexpr uint32_t kDig = kBits > 8 ? 512 : 256, kPer = kDig / 256;
     static_assert(sizeof(KeyT) == 4, "a pair is 8 bytes");
-    ScatterSmem<kDig>& S = *reinterpret_cast<ScatterSmem<kDig>*>(smem_raw);
+    ScatterSmem<kDig, kMode>& S = *reinterpret_cast<ScatterSmem<kDig, kMode>*>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     // the keys and values come from the kernel before the counting one, so they
     // are loaded while that one finishes; or (keys_just_written) from the
     // kernel right before this one, which counted them as it wrote them
     if (keys_just_written) pdl_wait();
-    const uint32_t K = (ctl->status & abort_mask) ? 0u : min(fixed_count ? fixed_count : ctl->total_keys, capacity);
+    const uint32_t total = kMode == kScatterColumns ? ctl->total_strips : ctl->total_keys;
+    const uint32_t K = (ctl->status & abort_mask) ? 0u : min(fixed_count ? fixed_count : total, capacity);
     const uint32_t nparts = min((K + kSortTile - 1) / kSortTile, max_parts);
     const uint32_t part = blockIdx.x;
     if (part >= nparts) return;  // (uniform)
@@ -586,12 +693,38 @@ __global__ void __launch_bounds__(256, kMinBlocks)
     // checks and with a fixed write-out loop
     auto partition = [&](auto full_tag) {
         constexpr bool kFull = decltype(full_tag)::value;
-        KeyT k[kItems];
+        KeyT k[kMode == kScatterRows ? kItems / 2 : kItems];  // (rows: 16-bit keys, two to a register)
         uint32_t vr[kItems];
+        auto key_at = [&](uint32_t i) -> KeyT {
+            return kMode == kScatterRows ? (i & 1u ? k[i / 2] >> 16 : k[i / 2] & 0xFFFFu) : k[i];
+        };
+        // the strips of the partition's slots: the keys are column << 8 | row
+        [[maybe_unused]] uint16_t* owner = reinterpret_cast<uint16_t*>(&S.whist[0][0]);
+        [[maybe_unused]] uint32_t first = 0, col0 = 0;
+        [[maybe_unused]] bool one_column = false;
+        if constexpr (kMode == kScatterRows) {
+            const uint32_t n_strips = min(ctl->total_strips, capacity);
+            first = min(strips.part_first[part], n_strips - 1u);
+            const uint32_t last = part + 1u < nparts ? min(strips.part_first[part + 1u], n_strips - 1u) : n_strips - 1u;
+            const uint32_t m = min(last - first + 1u, kSortTile + 1u);
+            // a strip's column << 8 | the row that it would have at the partition's slot 0, and its value
+            slot_owners(owner, m, cnt, S.wsum, [&](uint32_t q) {
+                const uint32_t strip = strips.keys[first + q], slot = strips.starts[first + q] - base;
+                S.pairs[q] = make_uint2(strip_col(strip) << 8 | ((strip_row(strip) - slot) & 0xFFu), strips.vals[first + q]);
+                return slot;
+            });
+            col0 = S.pairs[0].x >> 8;
+            one_column = S.pairs[owner[cnt - 1]].x >> 8 == col0;
+        }
 #pragma unroll
         for (uint32_t i = 0; i < kItems; ++i) {
             const uint32_t idx = warp * (kItems * 32) + i * 32 + lane;
-            if (kFull || idx < cnt) {
+            if constexpr (kMode == kScatterRows) {
+                const uint2 strip = S.pairs[owner[idx]];  // (past cnt: the last strip)
+                const uint32_t key = (strip.x & 0xFF00u) | ((strip.x + idx) & 0xFFu);
+                k[i / 2] = i & 1u ? k[i / 2] | key << 16 : key;
+                vr[i] = strip.y;
+            } else if (kFull || idx < cnt) {
                 k[i] = keys_in[base + idx];
                 vr[i] = vals_in[base + idx];
             } else {
@@ -599,14 +732,31 @@ __global__ void __launch_bounds__(256, kMinBlocks)
                 vr[i] = 0u;
             }
         }
+        if constexpr (kMode == kScatterRows) __syncthreads();  // (the owners are read: their words are cleared next)
         // this partition's digit offsets, written by the counting kernel (this
         // kernel may have started while it ran)
         pdl_wait();
         pdl_trigger();  // the next kernel (the next counting kernel, or the blend) may be scheduled; it waits for this grid
-        const RowDigits<kPer> goff = counted_offset<kDig>(CountedWork<kDig>(work, max_parts), nparts, part, S.wsum);
+        RowDigits<kPer> goff;
+        [[maybe_unused]] uint32_t hoff = 0;
+        if constexpr (kMode == kScatterColumns) {
+            // 512 digits were counted: the heights' offsets start after all the strips
+            const RowDigits<2> both = counted_offset<512>(CountedWork<512>(work, max_parts), nparts, part, S.wsum);
+            S.hmap[2 * tid] = both.v[0];
+            S.hmap[2 * tid + 1] = both.v[1];
+            __syncthreads();
+            goff.v[0] = S.hmap[tid];
+            hoff = S.hmap[256 + tid] - K;
+        } else {
+            goff = counted_offset<kDig>(CountedWork<kDig>(work, max_parts), nparts, part, S.wsum);
+        }
 #pragma unroll
         for (uint32_t i = tid; i < kWarps * kDig / 4; i += 256)
             reinterpret_cast<uint4*>(&S.whist[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (kMatch)
+#pragma unroll
+            for (uint32_t i = tid; i < kWarps * kDig / 4; i += 256)
+                reinterpret_cast<uint4*>(&S.match[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
         __syncthreads();
         // stable rank within the warp (warp-striped order)
         uint32_t rank[kItems / 2];  // two 16-bit ranks each
@@ -614,8 +764,13 @@ __global__ void __launch_bounds__(256, kMinBlocks)
 #pragma unroll
         for (uint32_t i = 0; i < kItems; ++i) {
             const uint32_t idx = warp * (kItems * 32) + i * 32 + lane;
-            const uint32_t d = kFull || idx < cnt ? (uint32_t(k[i] >> shift) & mask) : kDig;
+            const uint32_t d = kFull || idx < cnt ? (uint32_t(key_at(i) >> shift) & mask) : kDig;
             uint32_t peers = 0xFFFFFFFFu;
+            if constexpr (kMatch) {
+                if (kFull || d < kDig) atomicOr(&S.match[warp][d], 1u << lane);
+                __syncwarp();
+                if (kFull || d < kDig) peers = S.match[warp][d];
+            } else {
 #pragma unroll
             for (int b = 0; b < kBits; ++b) {
                 const bool on = (d >> b) & 1u;
@@ -627,12 +782,15 @@ __global__ void __launch_bounds__(256, kMinBlocks)
                 const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
                 peers &= on ? bal : ~bal;
             }
+            }
             const uint32_t leader = __ffs(peers) - 1;
             uint32_t prev = 0;
             if (lane == leader && (kFull || d < kDig)) {
                 prev = S.whist[warp][d];
                 S.whist[warp][d] = prev + __popc(peers);
             }
+            __syncwarp();
+            if (kMatch && lane == leader && (kFull || d < kDig)) S.match[warp][d] = 0u;
             prev = __shfl_sync(0xFFFFFFFFu, prev, leader);
             const uint32_t r = prev + __popc(peers & lt);
             rank[i / 2] = i & 1u ? rank[i / 2] | r << 16 : r;
@@ -650,6 +808,16 @@ __global__ void __launch_bounds__(256, kMinBlocks)
         RowDigits<kPer> slot = scan_digits<kPer>(count, S.wsum);  // the digits' first slots
 #pragma unroll
         for (uint32_t p = 0; p < kPer; ++p) S.gmap[kPer * tid + p] = goff.v[p] - slot.v[p];
+        [[maybe_unused]] const uint32_t slot0 = slot.v[0];
+        // rows of one column (most partitions of a large frame): each is one
+        // tile's keys, and no key has to be compared with the one before it
+        if (kMode == kScatterRows && one_column && count.v[0]) {
+            const uint32_t tile = tid * strips.gx + col0;
+            if (TPD_INBOUNDS(ctl, 18, tile, n_tiles)) {
+                atomicMin(&ranges[2 * tile], goff.v[0]);
+                atomicMax(&ranges[2 * tile + 1], goff.v[0] + count.v[0]);
+            }
+        }
 #pragma unroll
         for (uint32_t w = 0; w < kWarps; ++w)
 #pragma unroll
@@ -663,11 +831,29 @@ __global__ void __launch_bounds__(256, kMinBlocks)
             const uint32_t idx = warp * (kItems * 32) + i * 32 + lane;
             if (kFull || idx < cnt) {
                 const uint32_t pos =
-                    S.whist[warp][(k[i] >> shift) & mask] + (i & 1u ? rank[i / 2] >> 16 : rank[i / 2] & 0xFFFFu);
-                if (TPD_INBOUNDS(ctl, 20, pos, cnt)) S.pairs[pad16(pos)] = make_uint2(k[i], vr[i]);
+                    S.whist[warp][(key_at(i) >> shift) & mask] + (i & 1u ? rank[i / 2] >> 16 : rank[i / 2] & 0xFFFFu);
+                if (TPD_INBOUNDS(ctl, 20, pos, cnt)) S.pairs[pad16(pos)] = make_uint2(key_at(i), vr[i]);
             }
         }
         __syncthreads();
+        if constexpr (kMode == kScatterColumns) {  // the key slots of the sorted strips: a prefix of their heights
+            uint32_t h[kItems], sum = 0;
+#pragma unroll
+            for (uint32_t q = 0; q < kItems; ++q) {
+                const uint32_t j = kItems * tid + q;
+                h[q] = kFull || j < cnt ? strip_height(S.pairs[pad16(j)].x) : 0u;
+                sum += h[q];
+            }
+            uint32_t before = block_exclusive_scan<kWarps>(sum, S.wsum);
+#pragma unroll
+            for (uint32_t q = 0; q < kItems; ++q) {
+                S.hpre[pad16(kItems * tid + q)] = before;
+                before += h[q];
+            }
+            __syncthreads();
+            if (count.v[0]) S.hmap[tid] = hoff - S.hpre[pad16(slot0)];
+            __syncthreads();
+        }
         // (g < K <= capacity: the bound check covers the buffer's end)
         auto write_out = [&](uint32_t j) {
             const uint2 pair = S.pairs[pad16(j)];
@@ -675,17 +861,26 @@ __global__ void __launch_bounds__(256, kMinBlocks)
             const uint32_t g = S.gmap[(key >> shift) & mask] + j;
             if (!TPD_INBOUNDS(ctl, 22, g, K)) return;
             vals_out[g] = pair.y;
+            if (kMode == kScatterRows && one_column) return;
             if constexpr (!kLast) {
                 keys_out[g] = key;
+                if constexpr (kMode == kScatterColumns) {
+                    const uint32_t start = S.hmap[strip_col(key)] + S.hpre[pad16(j)];
+                    strips.starts[g] = start;
+                    const uint32_t p = (start + kSortTile - 1) / kSortTile;  // (a strip holds at most 256 slots)
+                    if (p * kSortTile < start + strip_height(key) && p < max_parts) strips.part_first[p] = g;
+                }
             } else {
-                if (!TPD_INBOUNDS(ctl, 18, key, n_tiles)) return;
+                auto tile_of = [&](KeyT q) { return kMode == kScatterRows ? (q & 0xFFu) * strips.gx + (q >> 8) : q; };
+                const uint32_t tile = tile_of(key);
+                if (!TPD_INBOUNDS(ctl, 18, tile, n_tiles)) return;
                 const KeyT before = j ? S.pairs[pad16(j - 1)].x : KeyT(~KeyT(0));
                 if (before != key) {
-                    atomicMin(&ranges[2 * key], g);
-                    if (j && TPD_INBOUNDS(ctl, 18, before, n_tiles))
-                        atomicMax(&ranges[2 * before + 1], S.gmap[uint32_t(before >> shift) & mask] + j);
+                    atomicMin(&ranges[2 * tile], g);
+                    if (j && TPD_INBOUNDS(ctl, 18, tile_of(before), n_tiles))
+                        atomicMax(&ranges[2 * tile_of(before) + 1], S.gmap[uint32_t(before >> shift) & mask] + j);
                 }
-                if (j + 1 == cnt) atomicMax(&ranges[2 * key + 1], g + 1);
+                if (j + 1 == cnt) atomicMax(&ranges[2 * tile + 1], g + 1);
             }
         };
         if constexpr (kFull) {
@@ -757,10 +952,10 @@ void launch_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout, uint32_
     }
 }
 
-template <int kMinBlocks, int kBits, bool kLast, typename KeyT>
+template <int kMinBlocks, int kBits, int kMode, typename KeyT>
 int scatter_setup() {
-    cudaFuncSetAttribute(scatter_kernel<kMinBlocks, kBits, kLast, KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(sizeof(ScatterSmem<(kBits > 8 ? 512 : 256)>)));
+    cudaFuncSetAttribute(scatter_kernel<kMinBlocks, kBits, kMode, KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         int(sizeof(ScatterSmem<(kBits > 8 ? 512 : 256), kMode>)));
     return 1;
 }
 
@@ -785,12 +980,12 @@ void launch_counted_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout,
                              work, ctl, abort);
         auto scatter = [&](auto bits_tag, auto last_tag) {
             constexpr int kBits = decltype(bits_tag)::value;
-            constexpr bool kLast = decltype(last_tag)::value;
-            device_once(scatter_setup<kMinBlocks, kBits, kLast, KeyT>);
-            launch_dependent(scatter_kernel<kMinBlocks, kBits, kLast, KeyT>, dim3(max_parts), dim3(256),
-                             sizeof(ScatterSmem<(kBits > 8 ? 512 : 256)>), s, kin, vin, kout, vout, capacity,
+            constexpr int kMode = decltype(last_tag)::value ? kScatterLast : kScatterPairs;
+            device_once(scatter_setup<kMinBlocks, kBits, kMode, KeyT>);
+            launch_dependent(scatter_kernel<kMinBlocks, kBits, kMode, KeyT>, dim3(max_parts), dim3(256),
+                             sizeof(ScatterSmem<(kBits > 8 ? 512 : 256), kMode>), s, kin, vin, kout, vout, capacity,
                              shift, bits, plan.fixed_count, max_parts, work, ctl, plan.ranges, plan.n_tiles, abort,
-                             counted);
+                             counted, StripList{});
         };
         auto either = [&](auto bits_tag) { last ? scatter(bits_tag, std::true_type{}) : scatter(bits_tag, std::false_type{}); };
         if (kMinBlocks == 2 && bits <= 8) {
@@ -811,6 +1006,16 @@ void launch_counted_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout,
         std::swap(kin, kout);
         std::swap(vin, vout);
     }
+}
+
+template <int kBits, int kMode>
+void launch_strip_scatter(const StripSort& a, const StripList& strips, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
+                          uint32_t* vout, uint32_t bits, cudaStream_t s) {
+    device_once(scatter_setup<3, kBits, kMode, uint32_t>);
+    launch_dependent(scatter_kernel<3, kBits, kMode, uint32_t>, dim3(a.max_parts()), dim3(256),
+                     sizeof(ScatterSmem<256, kMode>), s, kin, vin, kout, vout, a.capacity, 0u, bits, 0u,
+                     a.max_parts(), a.work, a.ctl, a.ranges, a.n_tiles, kStatusFatal | kStatusKeyOverflow,
+                     kMode == kScatterColumns, strips);
 }
 
 }  // namespace
@@ -836,6 +1041,32 @@ size_t sort_desc_entries(uint32_t capacity, uint32_t items) {
 // / 8 / 4 keys a thread, 120,000 49 / 40 / 38, 250,000 52 / 45 / 48, 500,000
 // 58 / 56 / 66, 1M 69 / 71 / 90.
 uint32_t sort_items_for(uint32_t n) { return n <= (1u << 17) ? 4u : n <= (1u << 19) ? 8u : 16u; }
+
+// A strip's key has 8 bits for the column and 8 for the row, and the rows of
+// several views would need more. Measured (keygen + key sort, us, keys / strips):
+// 3M Gaussians at 2160p from the edge of the cloud 1106 / 699, from inside 207 /
+// 161; 1M at 1080p 163 / 130, 2M inside 89 / 87, 500,000 104 / 93; 200,000 at
+// 1440p 82 / 74. Smaller images have smaller rectangles, so fewer keys per
+// strip, and their sorts are a few waves, where the rows' longer CTAs count:
+// 300,000 at 720p (3600 tiles) 62 / 65, 120,000 at 801x603 51 / 54, 10,000 at
+// 256x256 30 / 43.
+bool takes_strips(uint32_t n_views, uint32_t gx, uint32_t gy) {
+    return n_views == 1 && gx <= 256 && gy <= 256 && gx * gy > 4096;
+}
+
+void launch_strip_sort(const StripSort& a, cudaStream_t s) {
+    const StripList strips{a.strips_alt, a.vals_alt, a.starts, a.part_first, a.gx};
+    if (a.gx <= 128)
+        launch_strip_scatter<7, kScatterColumns>(a, strips, a.strips, a.vals, a.strips_alt, a.vals_alt, 7, s);
+    else
+        launch_strip_scatter<8, kScatterColumns>(a, strips, a.strips, a.vals, a.strips_alt, a.vals_alt, 8, s);
+    launch_dependent(strip_rows_kernel<kStripParts>, dim3((a.max_parts() + kStripParts - 1) / kStripParts), dim3(256), 0, s, strips, a.capacity, a.max_parts(),
+                     a.work, a.ctl, kStatusFatal | kStatusKeyOverflow);
+    if (a.n_tiles <= 128 * a.gx)
+        launch_strip_scatter<7, kScatterRows>(a, strips, nullptr, nullptr, nullptr, a.vals, 7, s);
+    else
+        launch_strip_scatter<8, kScatterRows>(a, strips, nullptr, nullptr, nullptr, a.vals, 8, s);
+}
 
 void launch_sort_begin(FrameCtl* ctl, uint32_t total, cudaStream_t s) { sort_begin_kernel<<<1, 256, 0, s>>>(ctl, total); }
 

@@ -147,16 +147,17 @@ __device__ __forceinline__ bool last_to_arrive(uint32_t* count, uint32_t expecte
 // which counted_offset adds up itself: for the smallest frames the arrivals'
 // round trips were half of the counting kernel's time (10,000 Gaussians at
 // 256x256: 5.2 us of the frame with them, 2.4 without).
-template <uint32_t kDig>
-__device__ __forceinline__ void counted_finish(const CountedWork<kDig>& W, uint32_t nparts, uint32_t part,
-                                               const RowDigits<kDig / 256>& count, uint32_t* wsum, bool& s_last) {
+// counted_arrive is the same for a CTA that has stored the rows of kParts
+// consecutive partitions, from a multiple of kParts, the first being part.
+template <uint32_t kDig, uint32_t kParts = 1>
+__device__ __forceinline__ void counted_arrive(const CountedWork<kDig>& W, uint32_t nparts, uint32_t part,
+                                               uint32_t* wsum, bool& s_last) {
     constexpr uint32_t kPer = kDig / 256;
     const uint32_t tid = threadIdx.x;
-    store_row<kPer>(W.rows, part, tid, count);
     if (nparts <= kChunkParts) return;
     const uint32_t chunk = part / kChunkParts, nchunks = uint32_t(counted_div(nparts));
     const uint32_t first = chunk * kChunkParts, csize = min(kChunkParts, nparts - first);
-    if (!last_to_arrive(W.chunk_arrivals + chunk, csize, s_last)) return;
+    if (!last_to_arrive(W.chunk_arrivals + chunk, (csize + kParts - 1) / kParts, s_last)) return;
     scan_rows<kPer>(W.rows, first, csize, W.chunks, chunk, tid);
     const uint32_t group = chunk / kChunkParts, ngroups = uint32_t(counted_div(nchunks));
     const uint32_t gfirst = group * kChunkParts, gsize = min(kChunkParts, nchunks - gfirst);
@@ -177,6 +178,13 @@ __device__ __forceinline__ void counted_finish(const CountedWork<kDig>& W, uint3
 #pragma unroll
         for (uint32_t p = 0; p < kPer; ++p) run.v[p] += c.v[p];
     }
+}
+
+template <uint32_t kDig>
+__device__ __forceinline__ void counted_finish(const CountedWork<kDig>& W, uint32_t nparts, uint32_t part,
+                                               const RowDigits<kDig / 256>& count, uint32_t* wsum, bool& s_last) {
+    store_row<kDig / 256>(W.rows, part, threadIdx.x, count);
+    counted_arrive<kDig>(W, nparts, part, wsum, s_last);
 }
 
 // The global positions of the partition's first keys of the thread's digits

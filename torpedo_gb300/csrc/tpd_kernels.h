@@ -27,7 +27,7 @@ struct FrameCtl {
     // passes swap their buffers and the sorted items are in the other one
     uint32_t depth_skips;
     uint32_t tile_order_done;  // CTAs of the tile order that have finished (reset by the last)
-    uint32_t pad;
+    uint32_t total_strips;     // column strips of the visible items, written by the tile-count scan
     uint32_t tile_hist[128];    // tiles by class of their walk length (tile_class), counted by the blend
     uint32_t tile_cursor[128];  // tiles of each class that the tile order has placed (0 at rest)
     uint32_t list_class[32];    // tiles by class of their list length, as launch_list_classes places them
@@ -125,11 +125,36 @@ struct KeygenArgs {
     // offsets are ready afterwards (SortPlan.precounted); nullptr: the digit
     // counts of the tile ids go to ctl->sort_hist instead
     uint32_t* counted_work;
+    // strips (launch_strip_sort follows, see takes_strips): one view; column
+    // strips are written instead of keys, and their columns counted
+    bool strips;
+    uint64_t* strip_desc;         // look-back descriptors of the strip counts, as desc
     FrameCtl* ctl;
     uint32_t spin_limit;
     uint32_t never_publish;
 };
 void launch_keygen(const KeygenArgs& a, int num_sms, cudaStream_t s);
+
+// The key sort by strips. A frame's keys are the tiles of its rectangles; a
+// strip is one column of a rectangle, and there are several times fewer of them
+// than keys. launch_keygen (KeygenArgs.strips) writes them in depth order; here
+// they are sorted by column, then expanded into their keys while those are
+// sorted by row: the keys themselves are moved once. The sorted values are in
+// vals, and the ranges written, as by the last pass of launch_sort.
+struct StripSort {
+    uint32_t *strips, *vals, *strips_alt, *vals_alt;  // capacity each; the strips are in the first two
+    uint32_t* starts;      // capacity: scratch
+    uint32_t* part_first;  // ceil(capacity / 4096): scratch
+    uint32_t capacity;
+    uint32_t* work;        // the counted work area; the columns are counted
+    uint32_t* ranges;
+    uint32_t n_tiles;
+    uint32_t gx;           // the image's tile columns
+    FrameCtl* ctl;
+    uint32_t max_parts() const { return capacity > 4096u ? (capacity + 4095u) / 4096u : 1u; }
+};
+bool takes_strips(uint32_t n_views, uint32_t gx, uint32_t gy);  // whether a frame's key sort does (gx x gy tiles)
+void launch_strip_sort(const StripSort& a, cudaStream_t s);
 
 // keys[i] = tile << 32 | bits(viewZ of splat vals[i] in the tile's view) for
 // the slots i < min(ctl->total_keys, capacity) of every tile's range: the
