@@ -73,6 +73,8 @@ struct OnesweepSmem {
     KeyT keys[kTile + kTile / 16];
     uint32_t vals[kTile + kTile / 16];
     uint32_t whist[kThreads / 32][kRadix];
+    // per warp and digit (kInvalidDigit too), the lanes that have it (0 at rest)
+    uint32_t match[kThreads == 256 ? kThreads / 32 : 1][kRadix + 4];
     uint32_t gdig[kRadix];    // global exclusive digit offsets of this pass
     uint32_t lstart[kRadix];  // block-local digit start
     uint32_t gmap[kRadix];    // global position of local index 0 of each digit
@@ -289,6 +291,21 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
         }
     }
 
+    // How a warp finds its lanes of one digit: an atomic OR into a shared word
+    // per (warp, digit), where lanes that share a digit queue, or a ballot per
+    // digit bit, whatever the digits. The OR is faster unless a digit has more
+    // than a 24th of the keys, which the pass's histogram tells. 9M keys of 45
+    // bits, us, OR / ballots: random digits 495 / 540, 64 digits of each byte
+    // 548 / 551, 16 digits 663 / 573, 4 digits 634 / 535. With the choice (the
+    // ballots are a little slower beside the other loop): 499, 568, 595, 561;
+    // the depth sort of 3M 130 -> 124, of 500,000 in 8 views 220 -> 210.
+    constexpr bool kMayMatch = kThreads == 256;
+    bool by_match = false;
+    if constexpr (kMayMatch) {
+        for (uint32_t i = tid; i < kWarps * (kRadix + 4); i += kThreads) (&S.match[0][0])[i] = 0;
+        by_match = !__syncthreads_or(h > K / 24u);
+    }
+
     // Warp-striped items, loaded coalesced straight from global memory: warp w
     // owns [w*32*kItems, (w+1)*32*kItems), item i covers 32 consecutive keys.
     // Variants with registers to spare load the values with the keys. The
@@ -334,41 +351,60 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
         // key's rank among equal digits earlier in the warp (bits 9..31).
         uint32_t dr[kSortItems];
         const uint32_t lt = lanemask_lt();
+        auto rank = [&](auto match_tag) {
+            constexpr bool kMatch = decltype(match_tag)::value;
 #pragma unroll
-        for (uint32_t i = 0; i < kSortItems; ++i) {
-            const uint32_t idx = warp * (kSortItems * 32) + i * 32 + lane;
-            const uint32_t d = idx < cnt && !(kDrop && uint32_t(k[i]) == 0xFFFFFFFFu) ? (uint32_t(k[i] >> shift) & mask)
-                                                                                     : kInvalidDigit;
-            uint32_t peers;
-            if constexpr (kMatchRank) {
-                peers = __match_any_sync(0xFFFFFFFFu, d);
-            } else {
-                // lanes with the same digit: one ballot per digit bit (bits
-                // above the pass's width are zero in every valid lane and
-                // leave the mask as it is), and one for the past-the-end (or
-                // dropped) digit in the partitions that can have any
-                peers = 0xFFFFFFFFu;
+            for (uint32_t i = 0; i < kSortItems; ++i) {
+                const uint32_t idx = warp * (kSortItems * 32) + i * 32 + lane;
+                const uint32_t d = idx < cnt && !(kDrop && uint32_t(k[i]) == 0xFFFFFFFFu) ? (uint32_t(k[i] >> shift) & mask)
+                                                                                         : kInvalidDigit;
+                uint32_t peers;
+                if constexpr (kMatch) {
+                    atomicOr(&S.match[warp][d], 1u << lane);
+                    __syncwarp();
+                    peers = S.match[warp][d];
+                } else if constexpr (kMatchRank) {
+                    peers = __match_any_sync(0xFFFFFFFFu, d);
+                } else {
+                    // lanes with the same digit: one ballot per digit bit (bits
+                    // above the pass's width are zero in every valid lane and
+                    // leave the mask as it is), and one for the past-the-end (or
+                    // dropped) digit in the partitions that can have any
+                    peers = 0xFFFFFFFFu;
 #pragma unroll
-                for (uint32_t b = 0; b < kRadixBits; ++b) {
-                    const bool on = (d >> b) & 1u;
-                    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
-                    peers &= on ? bal : ~bal;
+                    for (uint32_t b = 0; b < kRadixBits; ++b) {
+                        const bool on = (d >> b) & 1u;
+                        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
+                        peers &= on ? bal : ~bal;
+                    }
+                    if (kDrop || cnt < kSortTile) {
+                        const bool on = d >= kRadix;
+                        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
+                        peers &= on ? bal : ~bal;
+                    }
                 }
-                if (kDrop || cnt < kSortTile) {
-                    const bool on = d >= kRadix;
-                    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
-                    peers &= on ? bal : ~bal;
+                const uint32_t leader = __ffs(peers) - 1;
+                uint32_t prev = 0;
+                if (lane == leader && d < kRadix) {
+                    prev = S.whist[warp][d];
+                    S.whist[warp][d] = prev + __popc(peers);
                 }
+                if constexpr (kMatch) {
+                    __syncwarp();  // (every lane has read its word)
+                    if (lane == leader) S.match[warp][d] = 0u;
+                }
+                prev = __shfl_sync(0xFFFFFFFFu, prev, leader);
+                dr[i] = d | ((prev + __popc(peers & lt)) << 9);
+                __syncwarp();
             }
-            const uint32_t leader = __ffs(peers) - 1;
-            uint32_t prev = 0;
-            if (lane == leader && d < kRadix) {
-                prev = S.whist[warp][d];
-                S.whist[warp][d] = prev + __popc(peers);
-            }
-            prev = __shfl_sync(0xFFFFFFFFu, prev, leader);
-            dr[i] = d | ((prev + __popc(peers & lt)) << 9);
-            __syncwarp();
+        };
+        if constexpr (kMayMatch) {
+            if (by_match)
+                rank(std::true_type{});
+            else
+                rank(std::false_type{});
+        } else {
+            rank(std::false_type{});
         }
         __syncthreads();
 
