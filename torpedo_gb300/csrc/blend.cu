@@ -758,7 +758,9 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
                 const float2 alpha =
                     f2(ca ? fminf(kAlphaMax, raw.x) : 0.0f, cb ? fminf(kAlphaMax, raw.y) : 0.0f);
                 const float2 om = __ffma2_rn(mone, alpha, one);  // 1 - alpha >= 0.01
-                T[h] = __fmul2_rn(T[h], f2(__fdividef(1.0f, om.x), __fdividef(1.0f, om.y)));  // in front of the entry
+                // in front of the entry (an approximate division takes a reciprocal as well, and
+                // scales around it: 1178 us for 8 views of 500,000, 1140 without)
+                T[h] = __fmul2_rn(T[h], f2(rcp_approx(om.x), rcp_approx(om.y)));
                 w[h] = __fmul2_rn(alpha, T[h]);
                 const float2 gc = __ffma2_rn(g2[h], bb, __ffma2_rn(g1[h], f2(rg.z, rg.w), __fmul2_rn(g0[h], f2(rg.x, rg.y))));
                 const float2 ad = __fmul2_rn(alpha, __fadd2_rn(gc, nA[h]));  // alpha (g.c - A)
