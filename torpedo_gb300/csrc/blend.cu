@@ -18,7 +18,7 @@
 // warp-reduced, then in shared memory, then with one global atomic per
 // (round, Gaussian, field).
 //
-// Every per-pixel operation (p2, alpha, the skip and stop tests) has the same
+// Every per-pixel operation (n2, alpha, the skip and stop tests) has the same
 // operations and explicit rounding in the forward and in the adjoint, so both
 // take identical decisions.
 //
@@ -48,22 +48,20 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
 // Per (pixel, entry) pair, with the conic pre-scaled at staging
-//   qa = -0.5 log2e cx, qb = -log2e cy, qc = -0.5 log2e cz,
+//   qa = 0.5 log2e cx, qb = log2e cy, qc = 0.5 log2e cz,
 //   dx = x - px, dy = y - py (rounded subtractions),
-//   p2 = fma(fma(qb, dy, qa dx), dx, (qc dy) dy) = log2(e) * power,
+//   n2 = fma(fma(qb, dy, qa dx), dx, (qc dy) dy) = -log2(e) * power,
 //   power = -0.5 * (cx*dx*dx + cz*dy*dy) - cy*dx*dy  (blend.slang:83-84),
-// five multiply/fma operations; exp(power) = 2^p2 is one ex2, and
-//   alpha = min(0.99, o * 2^p2) < 1/255  <=>  p2 < thr = log2(1 / (255 o))
-// is decided before the exponential.
-//
-// The forward holds the negated conic instead and computes n2 = -p2 by the same
-// operations (with (qc dy) dy a fused multiply-add onto +0, so that n2 is never
-// -0 unless its terms underflow): the pair counts when 0 <= n2 <= -thr, and as floats of that range ascend
-// as unsigned integers and negative ones lie above them, one integer comparison
-// of n2's bits with keep_limit decides both. 249 us with the two comparisons,
-// 239 with one, at 1M Gaussians and 1080p; 1621 and 1524 for 8 views of 1.5M at
-// 1080p. (The adjoint, with more to do per pair, gained nothing: 1178 and 1180
-// us for 8 views of 500,000, so it keeps the two.)
+// five multiply/fma operations; exp(power) = 2^-n2 is one ex2, and
+//   alpha = min(0.99, o * 2^-n2) < 1/255  <=>  n2 > -thr, thr = log2(1 / (255 o))
+// is decided before the exponential. The pair counts when power <= 0 and alpha
+// >= 1/255, i.e. 0 <= n2 <= -thr: floats of that range ascend as unsigned
+// integers and negative ones lie above them, so one integer comparison of n2's
+// bits with keep_limit decides both. ((qc dy) dy is taken as a fused
+// multiply-add onto +0, so that n2 is never -0 unless its terms underflow.)
+// With a comparison for each the blend of 1M Gaussians at 1080p took 249 us,
+// with one 239 (8 views of 1.5M: 1621 and 1525); the adjoint of 500,000 in 8
+// views 1140 and 1124.
 
 constexpr float kInf = __builtin_huge_valf();
 
@@ -85,9 +83,9 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // (pixel columns ox + 8c .. ox + 8c + 7), the block of warp 2k + c.
 //
 // With a = -qa, b = -qb / 2, c = -qc and d = centre - pixel, a pixel is kept
-// only when p2 >= thr, i.e. inside the ellipse a dx^2 + 2b dx dy + c dy^2 <= R
+// only when n2 <= -thr, i.e. inside the ellipse a dx^2 + 2b dx dy + c dy^2 <= R
 // for R = -thr. R is enlarged by 4e-3 (relative and absolute) plus 1e-5 ac/det
-// relative, which bounds the rounding of the per-pixel p2 even for thin
+// relative, which bounds the rounding of the per-pixel n2 even for thin
 // ellipses (its terms are at most 4 R ac / det in size there). For dy in a
 // slab, the ellipse spans dx in [(-b dy - s) / a, (-b dy + s) / a],
 // s = sqrt(a R - det dy^2); over the slab the extremes are +-hx (hx =
@@ -147,10 +145,7 @@ __device__ __forceinline__ uint32_t rgba8_unorm(float r, float g, float b) {
     return out;
 }
 
-// true when the pair is skipped (power > 0 or alpha < 1/255)
-__device__ __forceinline__ bool pair_skipped(float p2, float thr) { return p2 > 0.0f || p2 < thr; }
-
-// The forward's limit for the entry with the pre-scaled conic and threshold q:
+// The bits of n2 below which a pair counts, for q = (-qa, -qb, -qc, thr):
 // one above the bits of -thr, or 0 (no pair) when thr > 0. A conic that is not a
 // number (its covariance's determinant overflowed) gives n2 = NaN in every
 // pixel, which neither test skips: all bits are below the limit then. (No conic
@@ -182,7 +177,7 @@ __device__ __forceinline__ void load_view_tile(const ViewConst* views, const uin
 // (l & 7, (l >> 3) + 4) of that block. The two pixels of a lane share dx, and
 // the arithmetic of a (pixel, entry) pair runs on both pixels at once with
 // packed f32x2 operations: per pixel the operations, order and rounding
-// given above for p2, alpha and the tests, as in the adjoint. A staged entry
+// given above for n2, alpha and the tests, as in the adjoint. A staged entry
 // holds its values duplicated in register-pair order, so the packed operands
 // come straight out of five broadcast shared-memory loads.
 constexpr uint32_t kFwdThreads = 128;
@@ -317,22 +312,23 @@ __device__ __forceinline__ void blend_tile(const BlendArgs& a, uint32_t tile, Fw
                 return make_float2(__float_as_uint(n2.x) < limit ? fminf(kAlphaMax, ao.x) : 0.0f,
                                    __float_as_uint(n2.y) < limit ? fminf(kAlphaMax, ao.y) : 0.0f);
             };
-            // the pair's update, in list order. keep = 0 at the stop and after
-            // it (T = 0 gives tn = 0): the pair adds alpha T * 0 = 0 and T
-            // becomes 0; before the stop keep = 1 and both products are exact
-            // copies. With the adjoint's inputs, Tk keeps the transmittance at
+            // the pair's update, in list order. T becomes 0 at the stop and
+            // stays so after it (T = 0 gives tn = 0): the pair adds alpha * 0
+            // and leaves T = 0; before the stop the second product with 1 -
+            // alpha is tn again. With the adjoint's inputs, Tk keeps the transmittance at
             // the stop and the last entry that added is the last with w > 0
             // (alpha >= 1/255 times T >= 1e-4).
             auto apply = [&](float2 alpha, const PairStaged& E, uint32_t jj) {
                 const float4 rg = E.rg, bt = E.bt;
-                const float2 tn = __fmul2_rn(T, __ffma2_rn(mone, alpha, one));  // T (1 - alpha)
+                const float2 om = __ffma2_rn(mone, alpha, one);
+                const float2 tn = __fmul2_rn(T, om);  // T (1 - alpha)
                 const bool go_a = !(tn.x < kTMin), go_b = !(tn.y < kTMin);
-                const float2 keep = make_float2(go_a ? 1.0f : 0.0f, go_b ? 1.0f : 0.0f);
-                const float2 w = __fmul2_rn(__fmul2_rn(alpha, T), keep);
+                T = make_float2(go_a ? T.x : 0.0f, go_b ? T.y : 0.0f);
+                const float2 w = __fmul2_rn(alpha, T);
                 C0 = __ffma2_rn(make_float2(rg.x, rg.y), w, C0);
                 C1 = __ffma2_rn(make_float2(rg.z, rg.w), w, C1);
                 C2 = __ffma2_rn(make_float2(bt.x, bt.y), w, C2);
-                T = __fmul2_rn(tn, keep);
+                T = __fmul2_rn(T, om);
                 if constexpr (kState) {
                     Tk = make_float2(go_a ? tn.x : Tk.x, go_b ? tn.y : Tk.y);
                     last_a = w.x > 0.0f ? lbase + jj : last_a;
@@ -462,7 +458,7 @@ __global__ void pack_rgba8_kernel(const float* rgb, uint32_t* rgba, size_t pixel
 // one entry per block, and the four entries usually differ. The pixels of a
 // lane share dx, and their arithmetic runs two rows at a time in packed f32x2
 // operations, per pixel with the forward's operations, order and rounding for
-// p2, alpha and the tests. A staged entry holds the values that the packed
+// n2, alpha and the tests. A staged entry holds the values that the packed
 // operations take duplicated in register-pair order.
 //
 // Per pixel, with g = dL/dimage, and going from the back: T after an entry
@@ -471,7 +467,7 @@ __global__ void pack_rgba8_kernel(const float* rgb, uint32_t* rgba, size_t pixel
 // A <- A + alpha (g.c - A); then dL/dalpha = T_front (g.c - A). A skipped pair
 // has alpha = 0, which leaves T and A as they are (1 / (1 - 0) is exactly 1).
 //
-// Sums per (block, entry). With P = dL/dpower (power = p2 ln2) the record's
+// Sums per (block, entry). With P = dL/dpower (power = -n2 ln2) the record's
 // gradients follow from nine sums over pixels: P, P dx, P dy, P dx^2, P dx dy,
 // P dy^2 and w g (three). A lane's four pixels share dx, so it adds P, P dy
 // and P dy^2 over them first and multiplies by dx afterwards; eight of the
@@ -500,7 +496,7 @@ constexpr uint32_t kAdjThreads = 64;
 constexpr uint32_t kBlendBlocks = 8;  // 8x4 blocks of a tile
 
 struct BlockStaged {  // 80 bytes
-    float4 s;         // x, qa, thr, 0
+    float4 s;         // x, qa, keep_limit (bits), 0
     float4 yb;        // y, y, qb, qb
     float4 qco;       // qc, qc, opacity, opacity
     float4 rg;        // r, r, g, g
@@ -512,16 +508,16 @@ __device__ __forceinline__ void stage_block_values(float4 c, float4 tex, float4 
                                                    uint8_t& mask) {
     const float thr = co.w > 0.0f ? -__log2f(255.0f * co.w) : kInf;  // +inf: never blends
     const float4 q = make_float4(-0.5f * kLog2e * co.x, -kLog2e * co.y, -0.5f * kLog2e * co.z, thr);
-    d.s = make_float4(tex.x, q.x, thr, 0.0f);
-    d.yb = make_float4(tex.y, tex.y, q.y, q.y);
-    d.qco = make_float4(q.z, q.z, co.w, co.w);
+    d.s = make_float4(tex.x, -q.x, __uint_as_float(keep_limit(q)), 0.0f);
+    d.yb = make_float4(tex.y, tex.y, -q.y, -q.y);
+    d.qco = make_float4(-q.z, -q.z, co.w, co.w);
     d.rg = make_float4(c.x, c.x, c.y, c.y);
     d.b = make_float2(c.z, c.z);
     mask = uint8_t(block_mask<4>(tex.x, tex.y, q, ox, oy));
 }
 
 __device__ __forceinline__ void stage_block_empty(BlockStaged& d) {
-    d.s = make_float4(0.f, 0.f, kInf, 0.f);
+    d.s = make_float4(0.f, 0.f, 0.f, 0.f);
     d.yb = d.qco = d.rg = make_float4(0.f, 0.f, 0.f, 0.f);
     d.b = make_float2(0.f, 0.f);
 }
@@ -721,6 +717,10 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
     load_indices(max_last > kBwdRound ? max_last - kBwdRound : 0u, 32u);
     store_round(max_last, 0u);
     __syncthreads();
+    // the first entry of the round that a pixel counts (its last contributor; the round is back to front)
+    int from[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) from[q] = int(max_last - last[q]);
     uint32_t turn = 0;
     for (uint32_t r_end = max_last; r_end > 0;) {
         const uint32_t n = min(kBwdRound, r_end), next_end = r_end - n;
@@ -741,20 +741,20 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
         for (uint32_t i = 0; i < steps; ++i) {
             const uint32_t jj = list[i];
             const BlockStaged& E = SM.e[jj];
-            const uint32_t pos = r_end - 1u - jj;
             const float4 sc = E.s, yb = E.yb, qco = E.qco, rg = E.rg;
             const float2 bb = E.b;
             const float dx = __fadd_rn(sc.x, P.nx), qadx = __fmul_rn(sc.y, dx);
             float2 dpow[2], w[2], dy[2];
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
-                // p2 for both pixels, as in the forward
+                // n2 for both pixels, as in the forward
                 dy[h] = __fadd2_rn(f2(yb.x, yb.y), h ? P.ny1 : P.ny0);
                 const float2 t = __ffma2_rn(f2(yb.z, yb.w), dy[h], f2(qadx, qadx));
-                const float2 p2 = __ffma2_rn(t, f2(dx, dx), __fmul2_rn(__fmul2_rn(f2(qco.x, qco.y), dy[h]), dy[h]));
-                const bool ca = pos < last[2 * h] && !pair_skipped(p2.x, sc.z);
-                const bool cb = pos < last[2 * h + 1] && !pair_skipped(p2.y, sc.z);
-                const float2 raw = __fmul2_rn(f2(qco.z, qco.w), f2(ex2_approx(p2.x), ex2_approx(p2.y)));
+                const float2 qcdy = __fmul2_rn(f2(qco.x, qco.y), dy[h]);
+                const float2 n2 = __ffma2_rn(t, f2(dx, dx), __ffma2_rn(qcdy, dy[h], f2(0.0f, 0.0f)));
+                const bool ca = int(jj) >= from[2 * h] && __float_as_uint(n2.x) < __float_as_uint(sc.z);
+                const bool cb = int(jj) >= from[2 * h + 1] && __float_as_uint(n2.y) < __float_as_uint(sc.z);
+                const float2 raw = __fmul2_rn(f2(qco.z, qco.w), f2(ex2_approx(-n2.x), ex2_approx(-n2.y)));
                 const float2 alpha =
                     f2(ca ? fminf(kAlphaMax, raw.x) : 0.0f, cb ? fminf(kAlphaMax, raw.y) : 0.0f);
                 const float2 om = __ffma2_rn(mone, alpha, one);  // 1 - alpha >= 0.01
@@ -798,9 +798,9 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
             const BlockStaged& E = SM.e[k];
             float* rec = g2d_view + size_t(SM.idx[k]) * kG2DStride;
             if (warp == 0) {
-                // d power / d(dx, dy) = ln2 (2 qa dx + qb dy, 2 qc dy + qb dx)
+                // d power / d(dx, dy) = -ln2 (2 qa dx + qb dy, 2 qc dy + qb dx)
                 const float qa = E.s.y, qb = E.yb.z, qc = E.qco.x;
-                v = make_float4(kLn2 * (2.0f * qa * v.x + qb * v.y), kLn2 * (2.0f * qc * v.y + qb * v.x), -0.5f * v.z,
+                v = make_float4(-kLn2 * (2.0f * qa * v.x + qb * v.y), -kLn2 * (2.0f * qc * v.y + qb * v.x), -0.5f * v.z,
                                 -v.w);
             } else {
                 v = make_float4(-0.5f * v.x, __fdividef(v.y, E.qco.z), v.z, v.w);  // alpha = opacity exp(power)
@@ -813,6 +813,8 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
         if (next_end) store_round(next_end, turn);
         __syncthreads();
         r_end = next_end;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) from[q] -= int(n);
     }
 }
 
