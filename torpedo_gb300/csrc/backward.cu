@@ -241,9 +241,12 @@ __device__ __forceinline__ void shape_adjoint(const Item& it, float& glogit, flo
 #pragma unroll
         for (int d = 0; d < 3; ++d) gm[d] += em[12 + 0 * 4 + d] * gc0 + em[12 + 1 * 4 + d] * gc1 + em[12 + 3 * 4 + d] * gc3;
 
-        // 2D covariance
-        const float ivz = 1.0f / vp[2];
-        const float J0 = fxp * ivz, J4 = fyp * ivz, J2 = -J0 * vp[0] * ivz, J5 = -J4 * vp[1] * ivz;
+        // 2D covariance. J by divisions, each rounded once as in the forward: the
+        // conic's gradient amplifies J's error for thin splats (with one reciprocal
+        // and multiplications single gradients moved by up to 2e-3; 183 us instead
+        // of 187 for 8 views of 500,000)
+        const float vz = vp[2], ivz = 1.0f / vz;
+        const float J0 = fxp / vz, J2 = -fxp * vp[0] / (vz * vz), J4 = fyp / vz, J5 = -fyp * vp[1] / (vz * vz);
         float Tm[6];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -303,8 +306,8 @@ __device__ __forceinline__ void records_done() {
 // A CTA of 256 threads for 128 Gaussians: the first four warps take the colour
 // half of each, the other four the shape half. One thread for both held 168
 // registers, three CTAs of four warps per SM, and waited on its own chains
-// (issue on 40% of the cycles). 8 views of 500,000: 276 -> 184 us, of 1.5M of
-// which few are in a view 655 -> 527. Three CTAs per SM spill (222 us).
+// (issue on 40% of the cycles). 8 views of 500,000: 276 -> 187 us, of 1.5M of
+// which few are in a view 655 -> 540. Three CTAs per SM spill (222 us).
 // Its records are staged into shared memory with coalesced 16-byte loads (a
 // record is 240 B, so thread-per-record loads would stride), and its SH
 // gradients leave through the same buffer as coalesced 16-byte stores.
