@@ -246,9 +246,12 @@ def general_sort(eng, K, key_bits, stream, steps):
 def kernels_per_frame(views: int, tile_passes: int, counted: bool = True) -> int:
     """Kernel launches of one frame: frame_begin, preprocess, depth-sort passes
     (a pass whose digit is the same for every key launches and returns), the
-    depth-order scan fused with keygen, tile-id sort passes (counted passes: a
-    counting and a scatter kernel each; the last scatter also writes the tile
-    ranges), blend."""
+    depth-order scan, keygen (which counts the first tile-id pass), tile-id
+    sort passes (counted passes: a scatter kernel each and, but for the first,
+    a counting one; the last scatter also writes the tile ranges), blend. Column
+    strips take as many launches as two counted passes; onesweep passes are one
+    launch each, and the tile counts' scan and keygen are counted as one beside
+    them."""
     depth_passes = math.ceil((32 + (views - 1).bit_length()) / 8)
     return 4 + depth_passes + tile_passes * (2 if counted else 1)
 
@@ -541,13 +544,18 @@ def run_ours(args):
     # DRAM bytes per key of one pass, from the committed ncu capture of the
     # pass's kernels (read + write), times K
     counted = not settings.get("key_sort_lookback")
+    # one view this large sorts column strips and makes the keys in the last pass
+    gx, gy = (cam.width + 15) // 16, (cam.height + 15) // 16
+    strips = counted and settings.get("sort_ctas_per_sm", 0) != 2 and gx * gy > 4096 and max(gx, gy) <= 256
     traffic = None
     tfile = ROOT / "profiles" / "radix_pass_traffic.json"
-    if tfile.exists():
+    if tfile.exists() and not strips:
         t = json.loads(tfile.read_text())
         per_key = t.get("counted" if counted else "onesweep")
         traffic = int(per_key * K) if per_key else None
-    pass_kernel = ("partition_count_kernel (not in the first pass) + scatter_kernel "
+    pass_kernel = ("scatter_kernel by column over strips, strip_rows_kernel + scatter_kernel by row over the keys "
+                   "made from them (the key sort; one of its two passes on average)" if strips else
+                   "partition_count_kernel (not in the first pass) + scatter_kernel "
                    "(one counted 8-bit tile-id radix pass of the key sort)"
                    if counted else "onesweep_kernel (one 8-bit tile-id radix pass of the key sort)")
     general = general_sort(eng, K, key_bits, stream, args.steps) if not args.no_general_sort else None
@@ -613,14 +621,16 @@ def run_ours(args):
                      "bytes_per_launch": K * 24, "avg_launch_ms": round(pass_ms, 5),
                      "basis": "K * 24 B per 8-bit pass: the per-pass term of the fixed sort formula "
                               "K * (8 + 24 * ceil(B / 8)) for 64-bit keys and 32-bit values",
-                     "moved_bytes_per_launch": K * 16,
-                     "moved_GBps": round(K * 16 / (pass_ms / 1000.0) / 1e9, 1),
-                     "moved_frac": round(K * 16 / (pass_ms / 1000.0) / 1e9 / hbm, 4),
-                     "moved_note": "the pass itself reads and writes 32-bit tile ids and 32-bit values "
-                                   "(16 B per key); the depth half of the keys is ordered by the depth presort",
+                     "moved_bytes_per_launch": None if strips else K * 16,
+                     "moved_GBps": None if strips else round(K * 16 / (pass_ms / 1000.0) / 1e9, 1),
+                     "moved_frac": None if strips else round(K * 16 / (pass_ms / 1000.0) / 1e9 / hbm, 4),
+                     "moved_note": ("column strips (12 B each, several keys to a strip) are sorted, and the keys made "
+                                    "from them in the last pass, which writes 4 B per key; " if strips else
+                                    "the pass itself reads and writes 32-bit tile ids and 32-bit values (16 B per "
+                                    "key); ") + "the depth half of the keys is ordered by the depth presort",
                      "time_note": "avg_launch_ms = the key-sort stage / its passes; with counted passes the first "
-                                  "pass's digits are counted by expand_keys_kernel as it writes the keys (in the "
-                                  "keygen stage), so that pass has no counting launch"},
+                                  "pass's digits are counted as its keys (or strips) are written (in the keygen "
+                                  "stage), so that pass has no counting launch"},
         "frame_sort": {"keys": K, "key_bits": key_bits, "tile_passes": passes,
                        "depth_sort_ms": round(stage_avg["depth_sort"], 4), "key_sort_ms": round(stage_avg["key_sort"], 4),
                        "formula_GBps": round(sort_formula / ((stage_avg["depth_sort"] + stage_avg["key_sort"]) / 1000) / 1e9, 1),

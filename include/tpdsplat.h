@@ -87,7 +87,8 @@ typedef struct tpd_settings {
                                       queue (the adjoint's longest lists first); 0 (default): one CTA per tile */
     uint32_t key_sort_lookback;    /* 0 (default): the key sort's radix passes count every partition's digits first and
                                       scatter without waiting (counted passes, 3 CTAs per SM, or 2 with
-                                      sort_ctas_per_sm = 2); 1: onesweep passes with a decoupled look-back */
+                                      sort_ctas_per_sm = 2; a single large view sorts column strips unless that is
+                                      set); 1: onesweep passes with a decoupled look-back */
     uint32_t keep_backward_state;  /* whether frames keep the adjoint's inputs (per-pixel final transmittance and last
                                       contributor; tracking them costs the blend about 5%): 0 (default) once
                                       tpd_backward has been called on this engine; 1 always; 2 never. tpd_step_async
@@ -100,7 +101,7 @@ typedef struct tpd_settings {
 enum {
     TPD_STAGE_PREPROCESS = 0, /* camera upload, entity matrices, preprocess (splats + depth keys) */
     TPD_STAGE_DEPTH_SORT = 1, /* radix sort of the (view | depth) keys */
-    TPD_STAGE_KEYGEN = 2,     /* tile-count scan and key duplication in depth order (one kernel) */
+    TPD_STAGE_KEYGEN = 2,     /* tile-count scan and key (or strip) duplication in depth order */
     TPD_STAGE_KEY_SORT = 3,   /* radix sort of the (tile | depth) keys on their tile-id bits */
     TPD_STAGE_RANGES = 4,     /* empty: the key sort's last pass writes the tile ranges */
     TPD_STAGE_BLEND = 5,      /* alpha blend */

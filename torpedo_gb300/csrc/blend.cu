@@ -479,15 +479,15 @@ __global__ void pack_rgba8_kernel(const float* rgb, uint32_t* rgba, size_t pixel
 // the entry's conic, and adds them to the global record with vector atomics.
 //
 // Against one 8x8 block per warp with two pixels a lane and the nine gradients
-// of every pixel pair summed by shuffles and shared-memory atomics: 104M
+// of every pixel pair summed by shuffles and shared-memory atomics: 96M
 // instead of 185M warp instructions for 200,000 Gaussians at 800x800, 234 ->
-// 150 us; 8 views of 500,000 at 1280x720 1856 -> 1198 us; 5,003 at 201x151 90
-// -> 59 us; 8 views of 6M at 2160p 20.5 -> 13.5 ms. It issues on 54% of the
+// 131 us; 8 views of 500,000 at 1280x720 1856 -> 1119 us; 5,003 at 201x151 90
+// -> 58 us; 8 views of 6M at 2160p 20.5 -> 12.6 ms. It issues on 55% of the
 // cycles (16 warps per SM, by its registers and the blocks' sums; rounds of 32
 // with 20 warps measured 3% slower, rounds of 128 with 8 warps 38%), ALU and
-// FMA pipes at 47% and 41%; the last tiles leave 15% of the SM time idle.
-// The forward gains nothing from this layout (249 us at 1M Gaussians and
-// 1080p either way, and a mid-sized frame's longest tile takes 94 us on two
+// FMA pipes at 44% and 41%; the last tiles leave 15% of the SM time idle.
+// The forward gained nothing from this layout (249 us at 1M Gaussians and
+// 1080p either way, and a mid-sized frame's longest tile took 94 us on two
 // warps instead of 72 on four), so it keeps one 8x8 block per warp.
 //
 // List entries per round (an engine setting the autotuner picks): 64 by

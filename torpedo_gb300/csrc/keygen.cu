@@ -20,9 +20,11 @@
 // slots matters because depth order puts the nearest Gaussians, with the
 // largest rectangles, side by side: one kernel over 512-item partitions gave
 // the first CTA up to a million keys to write while the others were done
-// (1M Gaussians at 1080p from the edge of the cloud: 303 us, now 22 + 37;
-// 3M at 2160p: 1189 us, now 74 + 264; 10,000 at 256x256: 11 us with the scan of
-// the counts, now 6 + 5).
+// (1M Gaussians at 1080p from the edge of the cloud: 303 us, now 20 + 35;
+// 3M at 2160p: 1189 us, now 74 + 242; 10,000 at 256x256: 11 us with the scan of
+// the counts, now 6 + 5). In a large single view expand_strips_kernel takes the
+// second one's place and writes column strips, a few per item, for the key sort
+// to expand (sort.cu): 20 + 20 and 77 + 67 us for the first two.
 #include <algorithm>
 #include <type_traits>
 

@@ -10,12 +10,12 @@
 // passes instead of 23.
 //  1. In the frame the digit histograms come from earlier kernels (the
 //     preprocess counts the depth keys' digits, key duplication those of the
-//     tile ids); sort_histogram_kernel builds them for standalone sorts (one
+//     tile ids for look-back passes); sort_histogram_kernel builds them for standalone sorts (one
 //     read of the keys).
 //  2. onesweep_kernel, once per pass: a persistent CTA takes 4096-key
 //     partitions by atomic ticket, loads them with coalesced warp-striped
-//     loads, ranks keys per warp (bit ballots, or match-any in the 512-thread
-//     variant; stable within the warp-striped order), combines warps per
+//     loads, ranks keys per warp (shared atomics where the digits are spread,
+//     else bit ballots, or match-any in the 512-thread variant; stable within the warp-striped order), combines warps per
 //     digit, publishes its digit counts, reorders the partition in shared
 //     memory while predecessors publish, resolves each digit's global prefix
 //     by a decoupled look-back (one thread per digit, four predecessors per
@@ -1073,9 +1073,9 @@ size_t sort_desc_entries(uint32_t capacity, uint32_t items) {
     return (size_t(capacity) + tile - 1) / tile * kRadix + kRadix;
 }
 
-// Measured on the depth sort (4 passes, us): 30,000 items 44 / 35 / 30 with 16
-// / 8 / 4 keys a thread, 120,000 49 / 40 / 38, 250,000 52 / 45 / 48, 500,000
-// 58 / 56 / 66, 1M 69 / 71 / 90.
+// Measured on the depth sort (4 passes, us): 30,000 items 42 / 34 / 30 with 16
+// / 8 / 4 keys a thread, 120,000 47 / 39 / 38, 250,000 49 / 44 / 48, 500,000
+// 56 / 55 / 66, 1M 67 / 70 / 90 (4 keys from 250,000 up: with ballots only).
 uint32_t sort_items_for(uint32_t n) { return n <= (1u << 17) ? 4u : n <= (1u << 19) ? 8u : 16u; }
 
 // A strip's key has 8 bits for the column and 8 for the row, and the rows of
