@@ -600,8 +600,9 @@ struct StripList {
 // it spends, of the loads and of the arrivals (keygen + key sort with 1 / 2 / 4
 // / 8 of them: 817 / 798 / 789 / 816 us for 3M Gaussians at 2160p, 150 / 148 /
 // 151 / 154 for 1M at 1080p, 98 / 101 / 102 / 106 for 2M seen from inside).
+// (Registers for six CTAs per SM spill: 2 us more.)
 template <uint32_t kParts>
-__global__ void __launch_bounds__(256, 6) strip_rows_kernel(StripList strips, uint32_t capacity, uint32_t max_parts,
+__global__ void __launch_bounds__(256, 5) strip_rows_kernel(StripList strips, uint32_t capacity, uint32_t max_parts,
                                                             uint32_t* __restrict__ work, FrameCtl* ctl,
                                                             uint32_t abort_mask) {
     constexpr uint32_t kTile = 4096, kGroup = 256 / kParts;  // threads per partition
