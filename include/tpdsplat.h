@@ -242,7 +242,8 @@ TPD_API uint32_t tpd_key_bits_for_tiles(uint32_t tiles);
 /* Radix sort (radix-shuffle / prefixA / prefixB / mapping .slang): stable
  * sort of n (key, value) pairs on the low key_bits bits. Result in keys/vals
  * if *result_in_alt == 0, else in keys_alt/vals_alt. workspace: at least
- * tpd_sort_workspace_size(n) bytes of device memory, 16-byte aligned.
+ * tpd_sort_workspace_size(n) bytes of device memory, 16-byte aligned; the size
+ * never falls as n grows, so one made for the largest sort serves all.
  * The call enqueues its work on the stream and returns; once that work is
  * done, the uint32 at byte offset TPD_WORKSPACE_STATUS_OFFSET of the
  * workspace holds the device status (TPD_DEVSTAT_* bits): anything but 0

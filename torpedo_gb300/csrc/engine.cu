@@ -1400,8 +1400,16 @@ void* tpd_get_stream(const tpd_engine* e) { return e ? static_cast<void*>(e->str
 
 // ---- stage entry points
 
+// Enough for every sort of up to n pairs, so that one workspace serves them
+// all: a short sort's smaller partitions can take more descriptors than a long
+// sort's (sort_items_for).
 size_t tpd_sort_workspace_size(uint32_t n) {
-    return 256 * ((sizeof(FrameCtl) + 255) / 256) + sort_desc_entries(n, sort_items_for(n)) * 8;
+    size_t entries = sort_desc_entries(n, sort_items_for(n));
+    for (const uint32_t items : {4u, 8u}) {
+        const uint32_t most = std::min(n, sort_items_limit(items));
+        entries = std::max(entries, sort_desc_entries(most, items));
+    }
+    return 256 * ((sizeof(FrameCtl) + 255) / 256) + entries * 8;
 }
 
 int tpd_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t* vals_alt, uint32_t n,

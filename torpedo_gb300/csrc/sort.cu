@@ -1077,7 +1077,8 @@ size_t sort_desc_entries(uint32_t capacity, uint32_t items) {
 // Measured on the depth sort (4 passes, us): 30,000 items 42 / 34 / 30 with 16
 // / 8 / 4 keys a thread, 120,000 47 / 39 / 38, 250,000 49 / 44 / 48, 500,000
 // 56 / 55 / 66, 1M 67 / 70 / 90 (4 keys from 250,000 up: with ballots only).
-uint32_t sort_items_for(uint32_t n) { return n <= (1u << 17) ? 4u : n <= (1u << 19) ? 8u : 16u; }
+uint32_t sort_items_limit(uint32_t items) { return items == 4 ? 1u << 17 : items == 8 ? 1u << 19 : 0xFFFFFFFFu; }
+uint32_t sort_items_for(uint32_t n) { return n <= sort_items_limit(4) ? 4u : n <= sort_items_limit(8) ? 8u : 16u; }
 
 // A strip's key has 8 bits for the column and 8 for the row, and the rows of
 // several views would need more. Measured (keygen + key sort, us, keys / strips):

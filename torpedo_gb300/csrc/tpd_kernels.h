@@ -175,6 +175,7 @@ size_t sort_desc_entries(uint32_t capacity, uint32_t items = 16);
 // Keys per thread of the 256-thread onesweep passes over n 64-bit pairs, 4, 8
 // or 16: fewer where 4096-key partitions would leave SMs idle.
 uint32_t sort_items_for(uint32_t n);
+uint32_t sort_items_limit(uint32_t items);  // the most pairs sorted with that many
 uint32_t sort_pass_count(uint32_t key_bits);
 struct SortPlan {
     uint32_t first_bit = 0;
