@@ -167,7 +167,9 @@ TPD_API int tpd_compile(tpd_engine* e, const void* records, uint32_t n, const ui
 
 /* Training form: builds the records on the device from raw device parameters
  * (means n x 3, log_scales n x 3, quats n x 4 used as given, opacity_logits n,
- * sh n x 48): opacity = sigmoid(logit), scale = exp(log_scale), modifier 1. */
+ * sh n x 48): opacity = sigmoid(logit), scale = exp(log_scale), modifier 1.
+ * The parameters are read on the engine's stream before the call returns, so
+ * work that writes them has to be complete, as for tpd_backward's input. */
 TPD_API int tpd_compile_params_device(tpd_engine* e, const float* means, const float* log_scales, const float* quats,
                               const float* opacity_logits, const float* sh, uint32_t n);
 

@@ -21,7 +21,6 @@ class RasterizeGaussians(torch.autograd.Function):
     @staticmethod
     def forward(ctx, means, log_scales, quats, opacity_logits, sh, engine: GaussianEngine, cams: list):
         tensors = [t.detach().contiguous().float() for t in (means, log_scales, quats, opacity_logits, sh)]
-        torch.cuda.current_stream(means.device).synchronize()
         engine.compile_params(*tensors)
         if len(cams) == 1:
             engine.set_camera(cams[0])

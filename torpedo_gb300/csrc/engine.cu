@@ -689,9 +689,11 @@ int set_views_internal(tpd_engine* e, const tpd_view* views, uint32_t nv) {
 // -> 794 us (of these, 230 are the autograd call).
 int alloc_scene(tpd_engine* e, uint32_t n, uint32_t n_ent, bool entities) {
     if (n_ent == 0) n_ent = 1;
-    // work in flight may read the buffers that are written next, and the
-    // inputs may come from another stream (freeing memory waited for both)
-    TPD_CUDA(e, cudaDeviceSynchronize());
+    // work in flight may read the buffers that are written next. Only this
+    // engine's stream is waited for: another thread may be capturing a stream,
+    // and then a wait for the whole device fails and spoils that capture
+    const int rc = wait_stream(e);
+    if (rc != TPD_OK) return rc;
     const bool same_frame = e->compiled && e->n == n && n > 0 && e->n_ent == 1 && n_ent == 1 && !entities &&
                             !e->d_ent_idx && e->identity_transforms;
     if (!same_frame) invalidate_graph(e);

@@ -225,6 +225,7 @@ class GaussianEngine:
             if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
                 raise ValueError("parameters must be contiguous float32 CUDA tensors")
         n = means.shape[0]
+        torch.cuda.current_stream(means.device).synchronize()  # parameters written on torch's stream
         _check(L.load().tpd_compile_params_device(self._h, means.data_ptr(), log_scales.data_ptr(), quats.data_ptr(),
                                                   opacity_logits.data_ptr(), sh.data_ptr(), n), self._h)
         self.n = n
