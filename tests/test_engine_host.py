@@ -38,3 +38,7 @@ def run(tmp_path_factory):
 
 def test_compile_beside_another_threads_capture(run):
     run("engine_compile_capture")
+
+
+def test_failed_allocations_leave_nothing_stale(run):
+    run("engine_alloc_failures")

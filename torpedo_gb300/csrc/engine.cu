@@ -247,11 +247,16 @@ void invalidate_graph(tpd_engine* e) {
     invalidate_slot_graphs(e);
 }
 
+// The buffers below grow by being freed and allocated anew. Their capacity is
+// 0 meanwhile, so that after a failed allocation the next call allocates them
+// again instead of using a null pointer.
+
 // Views x n sized buffers.
 int ensure_splat_buffers(tpd_engine* e) {
     const uint64_t need = uint64_t(e->n) * e->n_views;
     if (need > e->splat_cap) {
         invalidate_graph(e);
+        e->splat_cap = 0;
         TPD_CUDA(e, dalloc(e->d_splats, need));
         TPD_CUDA(e, dalloc(e->d_offsets, need));
         TPD_CUDA(e, dalloc(e->d_dkeys[0], 2 * need));
@@ -265,6 +270,7 @@ int ensure_splat_buffers(tpd_engine* e) {
     const uint64_t parts = need / std::min(kScanTileStandalone, kKeygenPart) + 2;  // the frame's scan partitions
     if (parts > e->desc_pre_cap) {
         invalidate_graph(e);
+        e->desc_pre_cap = 0;
         TPD_CUDA(e, dalloc(e->d_desc_pre, parts));
         TPD_CUDA(e, cudaMemset(e->d_desc_pre, 0, parts * 8));
         e->desc_pre_cap = parts;
@@ -272,6 +278,7 @@ int ensure_splat_buffers(tpd_engine* e) {
     const uint64_t em = uint64_t(e->n_ent) * e->n_views * kEntityMatFloats;
     if (em > e->ent_mats_cap) {
         invalidate_graph(e);
+        e->ent_mats_cap = 0;
         TPD_CUDA(e, dalloc(e->d_ent_mats, em));
         e->ent_mats_cap = em;
     }
@@ -295,6 +302,7 @@ int ensure_key_capacity(tpd_engine* e, uint64_t want) {
     if (want <= e->capacity) return TPD_OK;
     if (want > 0x7FFFFFFFull) return fail(e, TPD_ERR_CAPACITY, "key count exceeds 2^31-1");
     invalidate_graph(e);
+    e->capacity = 0;
     for (int b = 0; b < 2; ++b) {
         TPD_CUDA(e, dalloc(e->d_tiles[b], want));
         TPD_CUDA(e, dalloc(e->d_vals[b], want));
@@ -607,6 +615,37 @@ void rerender_with_state(tpd_engine* e) {
     e->state_kept = true;
 }
 
+// The buffers of the engine's views; uploads each tile's view and each view's first pixel.
+int alloc_views(tpd_engine* e, const std::vector<uint32_t>& tile_view, const std::vector<uint64_t>& img_off) {
+    const uint64_t pixels = e->total_pixels, tiles = e->total_tiles;
+    if (pixels > e->pixel_cap) {
+        e->pixel_cap = 0;
+        TPD_CUDA(e, dalloc(e->d_image, pixels * 3));
+        TPD_CUDA(e, dalloc(e->d_final_T, pixels));
+        TPD_CUDA(e, dalloc(e->d_n_contrib, pixels));
+        TPD_CUDA(e, dalloc(e->d_rgba, pixels));
+        e->pixel_cap = pixels;
+    }
+    if (tiles > e->tile_cap) {
+        e->tile_cap = 0;
+        TPD_CUDA(e, dalloc(e->d_ranges, tiles * 2));
+        TPD_CUDA(e, dalloc(e->d_tile_view, tiles));
+        TPD_CUDA(e, dalloc(e->d_tile_order, tiles));
+        TPD_CUDA(e, dalloc(e->d_tile_len, tiles));
+        e->tile_cap = tiles;
+    }
+    if (blend_takes_list_order(uint32_t(tiles), e->num_sms) && tiles * kListClasses > e->list_bucket_cap) {
+        e->list_bucket_cap = 0;
+        TPD_CUDA(e, dalloc(e->d_list_buckets, tiles * kListClasses));
+        e->list_bucket_cap = tiles * kListClasses;
+    }
+    if (!e->d_image_offset) TPD_CUDA(e, dalloc(e->d_image_offset, kMaxViews));
+    TPD_CUDA(e, cudaMemcpy(e->d_tile_view, tile_view.data(), tiles * 4, cudaMemcpyHostToDevice));
+    TPD_CUDA(e, cudaMemcpy(e->d_image_offset, img_off.data(), img_off.size() * 8, cudaMemcpyHostToDevice));
+    ensure_strips(e);
+    return ensure_splat_buffers(e);
+}
+
 int set_views_internal(tpd_engine* e, const tpd_view* views, uint32_t nv) {
     if (nv == 0 || nv > kMaxViews) return fail(e, TPD_ERR_ARG, "view count must be in [1, 256]");
     bool shape_changed = nv != e->n_views;
@@ -655,29 +694,12 @@ int set_views_internal(tpd_engine* e, const tpd_view* views, uint32_t nv) {
         while ((1u << vb) < nv) ++vb;
         e->depth_key_bits = 32 + vb;
     }
-    if (pixels > e->pixel_cap) {
-        TPD_CUDA(e, dalloc(e->d_image, pixels * 3));
-        TPD_CUDA(e, dalloc(e->d_final_T, pixels));
-        TPD_CUDA(e, dalloc(e->d_n_contrib, pixels));
-        TPD_CUDA(e, dalloc(e->d_rgba, pixels));
-        e->pixel_cap = pixels;
+    const int rc = alloc_views(e, tile_view, img_off);
+    if (rc != TPD_OK) {  // no views: a call that sets them again allocates again
+        e->n_views = e->total_tiles = 0;
+        e->total_pixels = 0;
     }
-    if (tiles > e->tile_cap) {
-        TPD_CUDA(e, dalloc(e->d_ranges, uint64_t(tiles) * 2));
-        TPD_CUDA(e, dalloc(e->d_tile_view, tiles));
-        TPD_CUDA(e, dalloc(e->d_tile_order, tiles));
-        TPD_CUDA(e, dalloc(e->d_tile_len, tiles));
-        e->tile_cap = tiles;
-    }
-    if (blend_takes_list_order(tiles, e->num_sms) && uint64_t(tiles) * kListClasses > e->list_bucket_cap) {
-        TPD_CUDA(e, dalloc(e->d_list_buckets, uint64_t(tiles) * kListClasses));
-        e->list_bucket_cap = uint64_t(tiles) * kListClasses;
-    }
-    if (!e->d_image_offset) TPD_CUDA(e, dalloc(e->d_image_offset, kMaxViews));
-    TPD_CUDA(e, cudaMemcpy(e->d_tile_view, tile_view.data(), tiles * 4ull, cudaMemcpyHostToDevice));
-    TPD_CUDA(e, cudaMemcpy(e->d_image_offset, img_off.data(), nv * 8ull, cudaMemcpyHostToDevice));
-    ensure_strips(e);
-    return ensure_splat_buffers(e);
+    return rc;
 }
 
 // Buffers of a scene of n records and n_ent entities. An optimisation loop
@@ -705,7 +727,7 @@ int alloc_scene(tpd_engine* e, uint32_t n, uint32_t n_ent, bool entities) {
         TPD_CUDA(e, dalloc(e->d_recs, uint64_t(n) * kRecordFloats));
         e->recs_cap = n;
     }
-    if (!e->h_transforms || n_ent != e->n_ent) {
+    if (!e->h_transforms || !e->d_transforms || n_ent != e->n_ent) {
         e->n_ent = n_ent;
         if (e->h_transforms) cudaFreeHost(e->h_transforms);
         e->h_transforms = nullptr;
@@ -740,17 +762,22 @@ void fill_stats(tpd_engine* e, tpd_frame_stats* stats, uint32_t retries) {
 // Pinned ring slots and staging images of the pipelined renders, sized for
 // the current views and transforms (before any render is outstanding).
 int ensure_ring(tpd_engine* e) {
-    if (!e->copy_stream) {
-        TPD_CUDA(e, cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
-        for (int i = 0; i < tpd_engine::kRing; ++i) {
-            TPD_CUDA(e, cudaMallocHost(reinterpret_cast<void**>(&e->ring_views[i]), sizeof(ViewConst) * kMaxViews));
-            TPD_CUDA(e, cudaMallocHost(reinterpret_cast<void**>(&e->ring_stats[i]), sizeof(StatsHead)));
-            TPD_CUDA(e, cudaEventCreateWithFlags(&e->ring_ready[i], cudaEventDisableTiming));
-            TPD_CUDA(e, cudaEventCreateWithFlags(&e->ring_done[i], cudaEventDisableTiming));
-        }
+    if (!e->copy_stream) TPD_CUDA(e, cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking));
+    for (int i = 0; i < tpd_engine::kRing; ++i) {
+        auto pinned = [](auto*& p, size_t bytes) {
+            return p ? cudaSuccess : cudaMallocHost(reinterpret_cast<void**>(&p), bytes);
+        };
+        auto event = [](cudaEvent_t& ev) {
+            return ev ? cudaSuccess : cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        };
+        TPD_CUDA(e, pinned(e->ring_views[i], sizeof(ViewConst) * kMaxViews));
+        TPD_CUDA(e, pinned(e->ring_stats[i], sizeof(StatsHead)));
+        TPD_CUDA(e, event(e->ring_ready[i]));
+        TPD_CUDA(e, event(e->ring_done[i]));
     }
     if (!e->identity_transforms && e->n_ent > e->ring_transforms_cap) {
         invalidate_slot_graphs(e);  // they read the old buffers
+        e->ring_transforms_cap = 0;
         for (int i = 0; i < tpd_engine::kRing; ++i) {
             if (e->ring_transforms[i]) cudaFreeHost(e->ring_transforms[i]);
             e->ring_transforms[i] = nullptr;
@@ -761,6 +788,7 @@ int ensure_ring(tpd_engine* e) {
     const uint64_t bytes = e->total_pixels * 12;  // room for RGB32F
     if (bytes > e->ring_image_cap) {
         invalidate_slot_graphs(e);
+        e->ring_image_cap = 0;
         for (int i = 0; i < tpd_engine::kRing; ++i) TPD_CUDA(e, dalloc(e->ring_image[i], bytes));
         e->ring_image_cap = bytes;
     }
@@ -1191,12 +1219,14 @@ int prepare_backward(tpd_engine* e, BackwardOut& o) {
     const uint64_t g2d = uint64_t(e->n) * e->n_views * kG2DStride;
     if (g2d > e->g2d_cap) {
         invalidate_step_graph(e);
+        e->g2d_cap = 0;
         TPD_CUDA(e, dalloc(e->d_g2d, g2d));
         e->g2d_cap = g2d;
     }
     const uint64_t gs = uint64_t(e->n) * (3 + 3 + 4 + 1 + 48);
     if ((!o.means || !o.log_scales || !o.quats || !o.logits || !o.sh) && gs > e->gscratch_cap) {
         invalidate_step_graph(e);
+        e->gscratch_cap = 0;
         TPD_CUDA(e, dalloc(e->d_gscratch, gs));
         e->gscratch_cap = gs;
     }
