@@ -15,7 +15,7 @@ struct Splat;
 struct FrameCtl {
     uint32_t status;         // kStatus* bits, cleared at frame start
     uint32_t tag;            // launch tag, advanced once per frame / call
-    uint32_t total_keys;     // K, written by the tile-count scan
+    uint32_t total_keys;     // K, written by the tile-count scan (0xFFFFFFFF: 2^31 keys or more)
     uint32_t visible;        // (view, Gaussian) pairs with a non-empty tile rect
     uint32_t ticket[32];     // partition tickets, cleared at frame start
     uint32_t sort_hist[8][256];   // digit counts of the key sort, by 8-bit digit position
@@ -31,6 +31,7 @@ struct FrameCtl {
     uint32_t tile_hist[128];    // tiles by class of their walk length (tile_class), counted by the blend
     uint32_t tile_cursor[128];  // tiles of each class that the tile order has placed (0 at rest)
     uint32_t list_class[32];    // tiles by class of their list length, as launch_list_classes places them
+    unsigned long long keys_seen;  // key counts of the scan's partitions so far, in 64 bits
 };
 constexpr uint32_t kListClasses = 16;
 
@@ -101,8 +102,8 @@ constexpr uint32_t kKeygenPart = 1024;
 // items come in depth order, so only the tile id of each key is written
 // (tiles[], u32): the depth half of a key is the depth of its value's splat
 // (launch_materialize_keys). K goes to ctl->total_keys and the non-empty
-// count to ctl->visible; more keys than the capacity flag the frame
-// (kStatusKeyOverflow) and none are written. Also presets ranges (2 x n_tiles
+// count to ctl->visible; more keys than the capacity, or 2^31 of them, flag the
+// frame (kStatusKeyOverflow) and none are written. Also presets ranges (2 x n_tiles
 // u32) to (0xFFFFFFFF, 0) for the key sort's last pass.
 struct KeygenArgs {
     const Splat* splats;
