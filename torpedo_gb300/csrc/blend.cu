@@ -226,7 +226,7 @@ __device__ __forceinline__ void stage_pair_empty(PairStaged& d, uint8_t& mask) {
 
 // Class of a walk of len entries, longer walks first: quarter octaves of len + 1.
 __device__ __forceinline__ uint32_t tile_class(uint32_t len) {
-    const uint32_t o = 31u - __clz(len + 1u);  // len < 2^31
+    const uint32_t o = 31u - __clz(len + 1u);  // len < 2^31: the class is below 128
     const uint32_t quarter = o >= 2u ? ((len + 1u) >> (o - 2u)) & 3u : ((len + 1u) << (2u - o)) & 3u;
     return 127u - (4u * o + quarter);
 }
@@ -887,6 +887,10 @@ __global__ void __launch_bounds__(kOrderThreads)
     __shared__ uint32_t count[128], base[128], wsum[4];
     pdl_wait();  // launched as a dependent of the stream's previous kernel: its output is read below
     pdl_trigger();
+    // a frame that blended nothing has left no walk lengths (the buffer may
+    // never have been written, and a class past the last would be counted out
+    // of range); the adjoint does nothing either
+    if (ctl->status & (kStatusFatal | kStatusKeyOverflow)) return;  // (uniform)
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     if (tid < 128) count[tid] = 0;
     if (blockIdx.x == 0 && tid == 0) ctl->ticket[kTicketBlendBackward] = 0;  // the adjoint's tile queue starts again
