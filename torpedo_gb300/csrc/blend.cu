@@ -33,6 +33,7 @@
 // alpha below 1/255 and skips it, as the reference does; so the culling
 // changes which skipped pairs are visited, never a result.
 #include <algorithm>
+#include <type_traits>
 
 #include "tpd_common.cuh"
 #include "tpd_kernels.h"
@@ -494,6 +495,13 @@ __global__ void pack_rgba8_kernel(const float* rgb, uint32_t* rgba, size_t pixel
 // List entries per round (an engine setting the autotuner picks): 64 by
 // default, 32 or 128.
 constexpr uint32_t kAdjThreads = 64;
+// A tile with a larger gradient, an infinite one or one that is not a number is
+// walked with arithmetic that keeps it to the entries its pixel counts: g.c may
+// overflow, and 0 times an infinite g is no zero. There S, the colours behind an
+// entry, takes A's place, dL/dalpha = g.(T_front c - S / (1 - alpha)), and a pair
+// that does not count is selected away instead of multiplied by 0. (The usual
+// walk is as fast with it beside as without: a step of 16 views 5866 us.)
+constexpr float kHugeGradient = 1e18f;
 constexpr uint32_t kBlendBlocks = 8;  // 8x4 blocks of a tile
 
 struct BlockStaged {  // 80 bytes
@@ -647,11 +655,15 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
         }
         blk_last = max(blk_last, last[q]);
     }
-    float2 T[2], nA[2], g0[2], g1[2], g2[2];
+    float2 T[2], g0[2], g1[2], g2[2];
+    bool huge = false;  // a gradient beyond kHugeGradient, infinite or not a number
+#pragma unroll
+    for (uint32_t c = 0; c < 3; ++c)
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) huge |= !(fabsf(gp[c][q]) <= kHugeGradient);
 #pragma unroll
     for (uint32_t h = 0; h < 2; ++h) {
         T[h] = f2(Tp[2 * h], Tp[2 * h + 1]);
-        nA[h] = f2(0.f, 0.f);  // -A
         g0[h] = f2(gp[0][2 * h], gp[0][2 * h + 1]);
         g1[h] = f2(gp[1][2 * h], gp[1][2 * h + 1]);
         g2[h] = f2(gp[2][2 * h], gp[2][2 * h + 1]);
@@ -665,7 +677,7 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
     for (uint32_t g = 0; g < 4; ++g) bl[g] = __shfl_sync(0xFFFFFFFFu, blk_last, 8 * g);
     if (lane == 0) SM.wmax[warp] = max(max(bl[0], bl[1]), max(bl[2], bl[3]));
     if (tid == 0) stage_block_empty(SM.e[kBwdRound]);
-    __syncthreads();
+    const bool any_huge = __syncthreads_or(huge);
     const uint32_t max_last = max(SM.wmax[0], SM.wmax[1]);
     float* g2d_view = a.g2d + size_t(vi) * a.g2d_view_stride;
 
@@ -713,110 +725,143 @@ __device__ __forceinline__ void blend_backward_tile(const BlendBackwardArgs& a, 
     };
     const float2 one = f2(1.0f, 1.0f), mone = f2(-1.0f, -1.0f);
     const uint32_t block = 4u * warp + (lane >> 3), j = lane & 7u;
-    load_indices(max_last, 0u);
-    load_round();
-    load_indices(max_last > kBwdRound ? max_last - kBwdRound : 0u, 32u);
-    store_round(max_last, 0u);
-    __syncthreads();
-    // the first entry of the round that a pixel counts (its last contributor; the round is back to front)
-    int from[4];
+    auto walk_tile = [&](auto huge_tag) {
+        constexpr bool kHuge = decltype(huge_tag)::value;
+        float2 nA[2], S[3][2];  // -A; with huge gradients the colours behind, instead
 #pragma unroll
-    for (uint32_t q = 0; q < 4; ++q) from[q] = int(max_last - last[q]);
-    uint32_t turn = 0;
-    for (uint32_t r_end = max_last; r_end > 0;) {
-        const uint32_t n = min(kBwdRound, r_end), next_end = r_end - n;
-        turn ^= 32u;
-        if (next_end) {
-            load_round();
-            load_indices(next_end > kBwdRound ? next_end - kBwdRound : 0u, turn ^ 32u);
-        }
-        const uint32_t steps = build_block_lists<kBwdRound>(SM.lists, warp, lane, n, [&](uint32_t e) {
-            uint32_t m = uint32_t(SM.mask[e]) >> (4u * warp);
-#pragma unroll
-            for (uint32_t g = 0; g < 4; ++g)
-                if (e + bl[g] < r_end) m &= ~(1u << g);  // behind the block's last contributor
-            SM.met[warp][e] = uint8_t(m & 15u);
-            return m;
-        });
-        const uint16_t* list = SM.lists.e[block];
-        for (uint32_t i = 0; i < steps; ++i) {
-            const uint32_t jj = list[i];
-            const BlockStaged& E = SM.e[jj];
-            const float4 sc = E.s, yb = E.yb, qco = E.qco, rg = E.rg;
-            const float2 bb = E.b;
-            const float dx = __fadd_rn(sc.x, P.nx), qadx = __fmul_rn(sc.y, dx);
-            float2 dpow[2], w[2], dy[2];
-#pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-                // n2 for both pixels, as in the forward
-                dy[h] = __fadd2_rn(f2(yb.x, yb.y), h ? P.ny1 : P.ny0);
-                const float2 t = __ffma2_rn(f2(yb.z, yb.w), dy[h], f2(qadx, qadx));
-                const float2 qcdy = __fmul2_rn(f2(qco.x, qco.y), dy[h]);
-                const float2 n2 = __ffma2_rn(t, f2(dx, dx), __ffma2_rn(qcdy, dy[h], f2(0.0f, 0.0f)));
-                const bool ca = int(jj) >= from[2 * h] && __float_as_uint(n2.x) < __float_as_uint(sc.z);
-                const bool cb = int(jj) >= from[2 * h + 1] && __float_as_uint(n2.y) < __float_as_uint(sc.z);
-                const float2 raw = __fmul2_rn(f2(qco.z, qco.w), f2(ex2_approx(-n2.x), ex2_approx(-n2.y)));
-                const float2 alpha =
-                    f2(ca ? fminf(kAlphaMax, raw.x) : 0.0f, cb ? fminf(kAlphaMax, raw.y) : 0.0f);
-                const float2 om = __ffma2_rn(mone, alpha, one);  // 1 - alpha >= 0.01
-                // in front of the entry (an approximate division takes a reciprocal as well, and
-                // scales around it: 1178 us for 8 views of 500,000, 1140 without)
-                T[h] = __fmul2_rn(T[h], f2(rcp_approx(om.x), rcp_approx(om.y)));
-                w[h] = __fmul2_rn(alpha, T[h]);
-                const float2 gc = __ffma2_rn(g2[h], bb, __ffma2_rn(g1[h], f2(rg.z, rg.w), __fmul2_rn(g0[h], f2(rg.x, rg.y))));
-                const float2 ad = __fmul2_rn(alpha, __fadd2_rn(gc, nA[h]));  // alpha (g.c - A)
-                nA[h] = __ffma2_rn(mone, ad, nA[h]);
-                const float2 dp = __fmul2_rn(T[h], ad);  // alpha dL/dalpha = dL/dpower, unless alpha is clamped
-                dpow[h] = f2(raw.x <= kAlphaMax ? dp.x : 0.0f, raw.y <= kAlphaMax ? dp.y : 0.0f);
-            }
-            const float2 s0 = __fmul2_rn(dpow[0], dy[0]), s1 = __fmul2_rn(dpow[1], dy[1]);
-            const float p0 = hsum(__fadd2_rn(dpow[0], dpow[1])), py = hsum(__fadd2_rn(s0, s1));
-            const float pyy = hsum(__ffma2_rn(s1, dy[1], __fmul2_rn(s0, dy[0])));
-            const float px = p0 * dx;
-            const float v[8] = {px, py, px * dx, py * dx, pyy, p0,
-                                hsum(__ffma2_rn(g0[1], w[1], __fmul2_rn(g0[0], w[0]))),
-                                hsum(__ffma2_rn(g1[1], w[1], __fmul2_rn(g1[0], w[0])))};
-            float v9 = hsum(__ffma2_rn(g2[1], w[1], __fmul2_rn(g2[0], w[0])));
-            SM.sums[block][jj * 8u + j] = group_sum8_transposed(v, lane);
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) v9 += __shfl_xor_sync(0xFFFFFFFFu, v9, o);
-            if (j == 0) SM.sum9[block][jj] = v9;
-        }
-        __syncthreads();  // the round's sums are complete
-        // warp 0: the record's first 16 bytes; warp 1: the other 20
-        for (uint32_t k = lane; k < n; k += 32u) {
-            const uint32_t met = uint32_t(SM.met[0][k]) | uint32_t(SM.met[1][k]) << 4;
-            if (!met) continue;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            float v9 = 0.f;
-#pragma unroll
-            for (uint32_t b = 0; b < kBlendBlocks; ++b) {
-                if (!((met >> b) & 1u)) continue;
-                const float4 x = *reinterpret_cast<const float4*>(&SM.sums[b][k * 8u + 4u * warp]);
-                v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
-                if (warp) v9 += SM.sum9[b][k];
-            }
-            const BlockStaged& E = SM.e[k];
-            float* rec = g2d_view + size_t(SM.idx[k]) * kG2DStride;
-            if (warp == 0) {
-                // d power / d(dx, dy) = -ln2 (2 qa dx + qb dy, 2 qc dy + qb dx)
-                const float qa = E.s.y, qb = E.yb.z, qc = E.qco.x;
-                v = make_float4(-kLn2 * (2.0f * qa * v.x + qb * v.y), -kLn2 * (2.0f * qc * v.y + qb * v.x), -0.5f * v.z,
-                                -v.w);
-            } else {
-                v = make_float4(-0.5f * v.x, __fdividef(v.y, E.qco.z), v.z, v.w);  // alpha = opacity exp(power)
-                if (v9 != 0.0f) atomicAdd(rec + 8, v9);
-            }
-            if (v.x != 0.0f || v.y != 0.0f || v.z != 0.0f || v.w != 0.0f)
-                atomicAdd(reinterpret_cast<float4*>(rec) + warp, v);
-        }
-        __syncthreads();  // (the flush has read the entries that are staged over)
-        if (next_end) store_round(next_end, turn);
+        for (uint32_t h = 0; h < 2; ++h) nA[h] = S[0][h] = S[1][h] = S[2][h] = f2(0.f, 0.f);
+        load_indices(max_last, 0u);
+        load_round();
+        load_indices(max_last > kBwdRound ? max_last - kBwdRound : 0u, 32u);
+        store_round(max_last, 0u);
         __syncthreads();
-        r_end = next_end;
+        // the first entry of the round that a pixel counts (its last contributor; the round is back to front)
+        int from[4];
 #pragma unroll
-        for (uint32_t q = 0; q < 4; ++q) from[q] -= int(n);
-    }
+        for (uint32_t q = 0; q < 4; ++q) from[q] = int(max_last - last[q]);
+        uint32_t turn = 0;
+        for (uint32_t r_end = max_last; r_end > 0;) {
+            const uint32_t n = min(kBwdRound, r_end), next_end = r_end - n;
+            turn ^= 32u;
+            if (next_end) {
+                load_round();
+                load_indices(next_end > kBwdRound ? next_end - kBwdRound : 0u, turn ^ 32u);
+            }
+            const uint32_t steps = build_block_lists<kBwdRound>(SM.lists, warp, lane, n, [&](uint32_t e) {
+                uint32_t m = uint32_t(SM.mask[e]) >> (4u * warp);
+#pragma unroll
+                for (uint32_t g = 0; g < 4; ++g)
+                    if (e + bl[g] < r_end) m &= ~(1u << g);  // behind the block's last contributor
+                SM.met[warp][e] = uint8_t(m & 15u);
+                return m;
+            });
+            const uint16_t* list = SM.lists.e[block];
+            for (uint32_t i = 0; i < steps; ++i) {
+                const uint32_t jj = list[i];
+                const BlockStaged& E = SM.e[jj];
+                const float4 sc = E.s, yb = E.yb, qco = E.qco, rg = E.rg;
+                const float2 bb = E.b;
+                const float dx = __fadd_rn(sc.x, P.nx), qadx = __fmul_rn(sc.y, dx);
+                float2 dpow[2], w[2], dy[2];
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) {
+                    // n2 for both pixels, as in the forward
+                    dy[h] = __fadd2_rn(f2(yb.x, yb.y), h ? P.ny1 : P.ny0);
+                    const float2 t = __ffma2_rn(f2(yb.z, yb.w), dy[h], f2(qadx, qadx));
+                    const float2 qcdy = __fmul2_rn(f2(qco.x, qco.y), dy[h]);
+                    const float2 n2 = __ffma2_rn(t, f2(dx, dx), __ffma2_rn(qcdy, dy[h], f2(0.0f, 0.0f)));
+                    const bool ca = int(jj) >= from[2 * h] && __float_as_uint(n2.x) < __float_as_uint(sc.z);
+                    const bool cb = int(jj) >= from[2 * h + 1] && __float_as_uint(n2.y) < __float_as_uint(sc.z);
+                    const float2 raw = __fmul2_rn(f2(qco.z, qco.w), f2(ex2_approx(-n2.x), ex2_approx(-n2.y)));
+                    const float2 alpha =
+                        f2(ca ? fminf(kAlphaMax, raw.x) : 0.0f, cb ? fminf(kAlphaMax, raw.y) : 0.0f);
+                    const float2 om = __ffma2_rn(mone, alpha, one);  // 1 - alpha >= 0.01
+                    // in front of the entry (an approximate division takes a reciprocal as well, and
+                    // scales around it: 1178 us for 8 views of 500,000, 1140 without)
+                    const float2 inv = f2(rcp_approx(om.x), rcp_approx(om.y));
+                    T[h] = __fmul2_rn(T[h], inv);
+                    w[h] = __fmul2_rn(alpha, T[h]);
+                    if constexpr (kHuge) {
+                        const float2 ninv = __fmul2_rn(inv, mone);
+                        const float2 d0 = __ffma2_rn(f2(rg.x, rg.y), T[h], __fmul2_rn(S[0][h], ninv));
+                        const float2 d1 = __ffma2_rn(f2(rg.z, rg.w), T[h], __fmul2_rn(S[1][h], ninv));
+                        const float2 d2 = __ffma2_rn(bb, T[h], __fmul2_rn(S[2][h], ninv));
+                        const float2 dA = __ffma2_rn(g2[h], d2, __ffma2_rn(g1[h], d1, __fmul2_rn(g0[h], d0)));
+                        S[0][h] = __ffma2_rn(f2(rg.x, rg.y), w[h], S[0][h]);
+                        S[1][h] = __ffma2_rn(f2(rg.z, rg.w), w[h], S[1][h]);
+                        S[2][h] = __ffma2_rn(bb, w[h], S[2][h]);
+                        const float2 dp = __fmul2_rn(alpha, dA);
+                        dpow[h] = f2(ca && raw.x <= kAlphaMax ? dp.x : 0.0f, cb && raw.y <= kAlphaMax ? dp.y : 0.0f);
+                        continue;
+                    }
+                    const float2 gc =
+                        __ffma2_rn(g2[h], bb, __ffma2_rn(g1[h], f2(rg.z, rg.w), __fmul2_rn(g0[h], f2(rg.x, rg.y))));
+                    const float2 ad = __fmul2_rn(alpha, __fadd2_rn(gc, nA[h]));  // alpha (g.c - A)
+                    nA[h] = __ffma2_rn(mone, ad, nA[h]);
+                    const float2 dp = __fmul2_rn(T[h], ad);  // alpha dL/dalpha = dL/dpower, unless alpha is clamped
+                    dpow[h] = f2(ca && raw.x <= kAlphaMax ? dp.x : 0.0f, cb && raw.y <= kAlphaMax ? dp.y : 0.0f);
+                }
+                // w g over the lane's pixels (an infinite g times the zero weight
+                // of a pair that does not count would be a NaN)
+                auto weighted = [&](const float2 (&g)[2]) {
+                    if constexpr (kHuge) {
+                        auto of = [](float gi, float wi) { return wi > 0.0f ? gi * wi : 0.0f; };
+                        return (of(g[0].x, w[0].x) + of(g[0].y, w[0].y)) + (of(g[1].x, w[1].x) + of(g[1].y, w[1].y));
+                    } else {
+                        return hsum(__ffma2_rn(g[1], w[1], __fmul2_rn(g[0], w[0])));
+                    }
+                };
+                const float2 s0 = __fmul2_rn(dpow[0], dy[0]), s1 = __fmul2_rn(dpow[1], dy[1]);
+                const float p0 = hsum(__fadd2_rn(dpow[0], dpow[1])), py = hsum(__fadd2_rn(s0, s1));
+                const float pyy = hsum(__ffma2_rn(s1, dy[1], __fmul2_rn(s0, dy[0])));
+                const float px = p0 * dx;
+                const float v[8] = {px, py, px * dx, py * dx, pyy, p0, weighted(g0), weighted(g1)};
+                float v9 = weighted(g2);
+                SM.sums[block][jj * 8u + j] = group_sum8_transposed(v, lane);
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) v9 += __shfl_xor_sync(0xFFFFFFFFu, v9, o);
+                if (j == 0) SM.sum9[block][jj] = v9;
+            }
+            __syncthreads();  // the round's sums are complete
+            // warp 0: the record's first 16 bytes; warp 1: the other 20
+            for (uint32_t k = lane; k < n; k += 32u) {
+                const uint32_t met = uint32_t(SM.met[0][k]) | uint32_t(SM.met[1][k]) << 4;
+                if (!met) continue;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                float v9 = 0.f;
+#pragma unroll
+                for (uint32_t b = 0; b < kBlendBlocks; ++b) {
+                    if (!((met >> b) & 1u)) continue;
+                    const float4 x = *reinterpret_cast<const float4*>(&SM.sums[b][k * 8u + 4u * warp]);
+                    v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
+                    if (warp) v9 += SM.sum9[b][k];
+                }
+                const BlockStaged& E = SM.e[k];
+                float* rec = g2d_view + size_t(SM.idx[k]) * kG2DStride;
+                if (warp == 0) {
+                    // d power / d(dx, dy) = -ln2 (2 qa dx + qb dy, 2 qc dy + qb dx)
+                    const float qa = E.s.y, qb = E.yb.z, qc = E.qco.x;
+                    v = make_float4(-kLn2 * (2.0f * qa * v.x + qb * v.y), -kLn2 * (2.0f * qc * v.y + qb * v.x), -0.5f * v.z,
+                                    -v.w);
+                } else {
+                    v = make_float4(-0.5f * v.x, __fdividef(v.y, E.qco.z), v.z, v.w);  // alpha = opacity exp(power)
+                    if (v9 != 0.0f) atomicAdd(rec + 8, v9);
+                }
+                if (v.x != 0.0f || v.y != 0.0f || v.z != 0.0f || v.w != 0.0f)
+                    atomicAdd(reinterpret_cast<float4*>(rec) + warp, v);
+            }
+            __syncthreads();  // (the flush has read the entries that are staged over)
+            if (next_end) store_round(next_end, turn);
+            __syncthreads();
+            r_end = next_end;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) from[q] -= int(n);
+        }
+    };
+    if (any_huge)
+        walk_tile(std::true_type{});
+    else
+        walk_tile(std::false_type{});
 }
 
 // One CTA per tile, tile order[b] for CTA b; or (kPersistent) one CTA per
