@@ -87,9 +87,10 @@ __device__ __forceinline__ ItemRect item_rect(uint32_t item, bool valid, float4 
 //  2. the counts are scanned across the warp, then across the CTA;
 //  3. one warp resolves the partition's exclusive prefix with the bounded
 //     decoupled look-back (prefix.slang:100-114 as restated in tpd_scan.cuh):
-//     the last partition's inclusive prefix is the frame's key count K. The
-//     prefixes have 32 bits; a sum of the counts in 64 flags the frame that has
-//     2^31 keys or more, before anything is looked up by a wrapped prefix;
+//     the last partition's inclusive prefix is the frame's key count K. A
+//     prefix has 32 bits, so a frame of 2^31 keys or more is flagged where they
+//     are passed: the first partition to end past them has an exact exclusive
+//     prefix (whatever those after it come round to);
 //  4. each lane stores its items' key offsets (the scan's output), for
 //     expand_keys_kernel their rectangles, offsets and Gaussians (16 bytes an
 //     item), and, for every multiple of 4096 among an item's slots, the item's
@@ -186,20 +187,17 @@ __global__ void __launch_bounds__(kScanItemsThreads, 6)
                                               never_publish != 0);
             if (lane == 0) {
                 S.excl[warp] = ex;
+                uint64_t end = ex;  // (a warp's count is at most 2^31: 128 items of 2^24 tiles)
+#pragma unroll
+                for (uint32_t w = 0; w < kScanItemsWarps; ++w) end += S.wtot[0][w];
+                if (keys && end > 0x7FFFFFFFull) {
+                    atomicMax(&ctl->total_keys, 0xFFFFFFFFu);
+                    atomicOr(&ctl->status, kStatusKeyOverflow);
+                }
                 if (part == nparts - 1u) {
                     atomicMax(keys ? &ctl->total_keys : &ctl->total_strips, ex + sum);  // (0 at the frame's start)
                     if (keys && ex + sum > capacity) atomicOr(&ctl->status, kStatusKeyOverflow);
                 }
-            }
-        } else if (warp == kSums && lane == 0) {
-            // the prefixes wrap at 2^32 keys: the partition whose count takes
-            // the sum past 2^31 - 1 flags the frame
-            unsigned long long sum = 0;
-#pragma unroll
-            for (uint32_t w = 0; w < kScanItemsWarps; ++w) sum += S.wtot[0][w];  // (up to 2^31 each: 128 items)
-            if (atomicAdd(&ctl->keys_seen, sum) + sum > 0x7FFFFFFFull) {
-                atomicMax(&ctl->total_keys, 0xFFFFFFFFu);
-                atomicOr(&ctl->status, kStatusKeyOverflow);
             }
         }
         __syncthreads();

@@ -84,7 +84,6 @@ __global__ void frame_begin_kernel(FrameCtl* ctl, const float* transforms, uint3
         ctl->status = 0;
         ctl->total_keys = 0;
         ctl->total_strips = 0;
-        ctl->keys_seen = 0;
         ctl->visible = 0;
         ctl->depth_count = 0;
         ctl->depth_skips = 0;

@@ -31,7 +31,6 @@ struct FrameCtl {
     uint32_t tile_hist[128];    // tiles by class of their walk length (tile_class), counted by the blend
     uint32_t tile_cursor[128];  // tiles of each class that the tile order has placed (0 at rest)
     uint32_t list_class[32];    // tiles by class of their list length, as launch_list_classes places them
-    unsigned long long keys_seen;  // key counts of the scan's partitions so far, in 64 bits
 };
 constexpr uint32_t kListClasses = 16;
 
