@@ -65,7 +65,6 @@ constexpr uint32_t kDefaultSpin = 1u << 20;
 // descriptors whenever the frame tag reaches a multiple of this, and a stale
 // descriptor can then never carry the current frame's tag.
 constexpr uint64_t kTagWindow = 1ull << 25;
-constexpr uint32_t kScanTileStandalone = 1024;
 
 struct StatsHead {
     uint32_t status, tag, total_keys, visible;
@@ -267,7 +266,7 @@ int ensure_splat_buffers(tpd_engine* e) {
         TPD_CUDA(e, cudaMemset(e->d_desc_depth, 0, de * 8));
         e->splat_cap = need;
     }
-    const uint64_t parts = need / std::min(kScanTileStandalone, kKeygenPart) + 2;  // the frame's scan partitions
+    const uint64_t parts = need / kKeygenPart + 2;  // the frame's scan partitions
     if (parts > e->desc_pre_cap) {
         invalidate_graph(e);
         e->desc_pre_cap = 0;
@@ -1484,7 +1483,7 @@ int tpd_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t*
 }
 
 size_t tpd_scan_workspace_size(uint32_t n) {
-    return 256 * ((sizeof(FrameCtl) + 255) / 256) + (size_t(n) / kScanTileStandalone + 2) * 8;
+    return 256 * ((sizeof(FrameCtl) + 255) / 256) + (scan_tiles_desc_entries(n) + 1) * 8;
 }
 
 int tpd_scan_tiles(const void* splats, uint32_t n, uint32_t* offsets, uint32_t* total, void* workspace,

@@ -425,6 +425,7 @@ __global__ void __launch_bounds__(kPreThreads, kCtas) preprocess_kernel(Preproce
 // scan_items_kernel.)
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanItems = 16;
+static_assert(kScanThreads * kScanItems == kScanTilesPart, "the descriptors are counted for these partitions");
 
 // Clears what the scan starts from: the look-back descriptors, the ticket,
 // the status and the total (of no splats).
@@ -442,7 +443,7 @@ __global__ void scan_begin_kernel(uint64_t* desc, uint32_t entries, FrameCtl* ct
 __global__ void __launch_bounds__(kScanThreads)
     scan_tiles_kernel(const Splat* splats, uint32_t n, uint32_t* offsets, uint64_t* desc, FrameCtl* ctl,
                       uint32_t* status, uint32_t* total_out, uint32_t spin_limit, uint32_t never_publish) {
-    constexpr uint32_t kScanTile = kScanThreads * kScanItems;
+    constexpr uint32_t kScanTile = kScanTilesPart;
     constexpr uint32_t kTag = 1;  // (a cleared descriptor has tag 0)
     __shared__ uint32_t s_part, s_excl;
     __shared__ uint32_t s_warp[kScanThreads / 32];
@@ -550,7 +551,7 @@ void launch_preprocess(const PreprocessArgs& a, int num_sms, cudaStream_t s) {
 
 void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint32_t* total, uint64_t* desc,
                        FrameCtl* ctl, uint32_t* status, uint32_t spin_limit, uint32_t never_publish, cudaStream_t s) {
-    const uint32_t parts = uint32_t((uint64_t(n) + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems));
+    const uint32_t parts = uint32_t(scan_tiles_desc_entries(n));
     scan_begin_kernel<<<parts / 256 + 1, 256, 0, s>>>(desc, parts, ctl, status, total);
     if (n == 0) return;
     launch_dependent(scan_tiles_kernel, dim3(parts), dim3(kScanThreads), 0, s, splats, n, offsets, desc, ctl, status,

@@ -37,9 +37,8 @@ using namespace tpd;
 
 namespace {
 
-constexpr uint32_t kStaticScanTile = 1024;  // splats per look-back partition of the scan kernel
 constexpr size_t kCtlBytes = 256 * ((sizeof(FrameCtl) + 255) / 256);
-constexpr size_t kDescEntries = size_t(TPD_SCAN_STATIC_MAX_SPLATS) / kStaticScanTile + 2;
+constexpr size_t kDescEntries = scan_tiles_desc_entries(TPD_SCAN_STATIC_MAX_SPLATS);
 constexpr size_t kScratchBytes = kCtlBytes + kDescEntries * sizeof(uint64_t);
 constexpr uint32_t kStaticSpin = 1u << 20;
 constexpr int kMaxDevices = 64;

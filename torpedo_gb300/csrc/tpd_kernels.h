@@ -84,9 +84,12 @@ void launch_frame_begin(FrameCtl* ctl, const float* transforms, uint32_t n_ent, 
                         uint32_t n_views, float* ent_mats, cudaStream_t s);
 void launch_preprocess(const PreprocessArgs& a, int num_sms, cudaStream_t s);
 
+// Splats per partition of the standalone scan.
+constexpr uint32_t kScanTilesPart = 4096;
+constexpr size_t scan_tiles_desc_entries(uint64_t n) { return size_t((n + kScanTilesPart - 1) / kScanTilesPart); }
 // Standalone exclusive scan of Splat.tiles (prefix.slang) into offsets, total
 // into *total, device status into *status. Clears everything it starts from:
-// desc (ceil(n / 4096) descriptors) and ctl's ticket.
+// desc (scan_tiles_desc_entries(n) descriptors) and ctl's ticket.
 void launch_scan_tiles(const Splat* splats, uint32_t n, uint32_t* offsets, uint32_t* total, uint64_t* desc,
                        FrameCtl* ctl, uint32_t* status, uint32_t spin_limit, uint32_t never_publish, cudaStream_t s);
 
