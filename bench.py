@@ -248,12 +248,37 @@ def kernels_per_frame(views: int, tile_passes: int, counted: bool = True) -> int
     (a pass whose digit is the same for every key launches and returns), the
     depth-order scan, keygen (which counts the first tile-id pass), tile-id
     sort passes (counted passes: a scatter kernel each and, but for the first,
-    a counting one; the last scatter also writes the tile ranges), blend. Column
-    strips take as many launches as two counted passes; onesweep passes are one
-    launch each, and the tile counts' scan and keygen are counted as one beside
-    them."""
+    a counting one; the last scatter also writes the tile ranges), blend.
+    Onesweep passes are one launch each. Without the exceptions that
+    frame_launches adds."""
     depth_passes = math.ceil((32 + (views - 1).bit_length()) / 8)
     return 4 + depth_passes + tile_passes * (2 if counted else 1)
+
+
+def key_sort_form(views: int, gx: int, gy: int, settings: dict) -> tuple[str, int, int]:
+    """How a frame of views images of gx x gy tiles sorts its keys, as the engine
+    chooses: (form, digit bits, passes). "strips": column strips, by column and
+    by row; "counted": digits of 9 bits where that takes a pass less than 8;
+    "onesweep": 8 bits."""
+    bits = (views * gx * gy).bit_length()
+    if settings.get("key_sort_lookback"):
+        return "onesweep", 8, math.ceil(bits / 8)
+    if views == 1 and gx <= 256 and gy <= 256 and gx * gy > 4096 and settings.get("sort_ctas_per_sm", 0) != 2:
+        return "strips", 8, 2
+    digit = 9 if math.ceil(bits / 9) < math.ceil(bits / 8) else 8
+    return "counted", digit, math.ceil(bits / digit)
+
+
+def frame_launches(views: int, n: int, gx: int, gy: int, settings: dict, sms: int = 152) -> int:
+    """Kernel launches of a frame of n Gaussians: kernels_per_frame, with one launch
+    for the depth sort of up to 12288 items, one more for the look-back form's
+    key duplication (beside the scan), and one for the blend's list order (one
+    to five waves of 8 tiles per SM). Strips take as many as two counted passes."""
+    form, _, passes = key_sort_form(views, gx, gy, settings)
+    launches = kernels_per_frame(views, passes, form != "onesweep") + (form == "onesweep")
+    if views * n <= 12288:
+        launches -= math.ceil((32 + (views - 1).bit_length()) / 8) - 1
+    return launches + (8 * sms < views * gx * gy <= 5 * 8 * sms)
 
 
 def _params(sc, dev):
@@ -463,7 +488,9 @@ def run_ours(args):
         settings, tuned = autotune.tune(make_engine, lambda e, k: e.raster_frames_async(k), stream)
     eng = make_engine(settings)
     st = eng.raster_frame()
-    launches_per_frame = kernels_per_frame(1, int(st["sort_passes"]), not settings.get("key_sort_lookback", 0))
+    gx, gy = (cam.width + 15) // 16, (cam.height + 15) // 16
+    launches_per_frame = frame_launches(1, sc.records.shape[0], gx, gy, settings,
+                                        torch.cuda.get_device_properties(dev).multi_processor_count)
 
     def barrier():
         torch.cuda.synchronize(dev)
@@ -535,7 +562,8 @@ def run_ours(args):
                       "two frames in flight"}
 
     K = int(st["keys"])
-    passes = int(st["sort_passes"])  # tile-id passes of the key sort
+    form, digit, passes = key_sort_form(1, gx, gy, settings)
+    counted, strips = form != "onesweep", form == "strips"
     key_bits = int(st["key_bits"])
     hbm, peak_kind = peaks()
     sort_formula = K * (8 + 24 * math.ceil(key_bits / 8))
@@ -543,10 +571,6 @@ def run_ours(args):
     achieved = K * 24 / (pass_ms / 1000.0) / 1e9
     # DRAM bytes per key of one pass, from the committed ncu capture of the
     # pass's kernels (read + write), times K
-    counted = not settings.get("key_sort_lookback")
-    # one view this large sorts column strips and makes the keys in the last pass
-    gx, gy = (cam.width + 15) // 16, (cam.height + 15) // 16
-    strips = counted and settings.get("sort_ctas_per_sm", 0) != 2 and gx * gy > 4096 and max(gx, gy) <= 256
     traffic = None
     tfile = ROOT / "profiles" / "radix_pass_traffic.json"
     if tfile.exists() and not strips:
@@ -556,7 +580,7 @@ def run_ours(args):
     pass_kernel = ("scatter_kernel by column over strips, strip_rows_kernel + scatter_kernel by row over the keys "
                    "made from them (the key sort; one of its two passes on average)" if strips else
                    "partition_count_kernel (not in the first pass) + scatter_kernel "
-                   "(one counted 8-bit tile-id radix pass of the key sort)"
+                   f"(one counted {digit}-bit tile-id radix pass of the key sort)"
                    if counted else "onesweep_kernel (one 8-bit tile-id radix pass of the key sort)")
     general = general_sort(eng, K, key_bits, stream, args.steps) if not args.no_general_sort else None
     eng.close()
@@ -619,7 +643,7 @@ def run_ours(args):
                      "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                      "frac": round(achieved / hbm, 4), "traffic": traffic, "peak_kind": f"{peak_kind} copy bandwidth",
                      "bytes_per_launch": K * 24, "avg_launch_ms": round(pass_ms, 5),
-                     "basis": "K * 24 B per 8-bit pass: the per-pass term of the fixed sort formula "
+                     "basis": "K * 24 B per pass: the per-pass term of the fixed sort formula "
                               "K * (8 + 24 * ceil(B / 8)) for 64-bit keys and 32-bit values",
                      "moved_bytes_per_launch": None if strips else K * 16,
                      "moved_GBps": None if strips else round(K * 16 / (pass_ms / 1000.0) / 1e9, 1),

@@ -17,6 +17,7 @@ std::map<char*, size_t> live;  // device and pinned allocations
 long fail_at = -1;             // which allocation from now on fails (0: the next)
 long failed = 0;
 long device_syncs = 0;
+long launches = 0;
 bool capture_spoiled = false;
 cudaStream_t capturing = nullptr;
 std::thread::id capturer;
@@ -144,13 +145,15 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const
     return *n = 2, cudaSuccess;
 }
 cudaError_t cudaGetSymbolAddress(void** p, const void*) { return *p = nullptr, cudaErrorInvalidSymbol; }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) { return cudaSuccess; }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) { return ++fake::launches, cudaSuccess; }
 
 // what the compiler's stubs of <<<>>> launches and its registration code call
 unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, void*) { return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3*, dim3*, size_t*, void*) { return cudaSuccess; }
 cudaError_t __cudaGetKernel(cudaKernel_t* k, const void*) { return *k = nullptr, cudaSuccess; }
-cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void**, size_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void**, size_t, cudaStream_t) {
+    return ++fake::launches, cudaSuccess;
+}
 void** __cudaRegisterFatBinary(void*) {
     static void* none = nullptr;
     return &none;

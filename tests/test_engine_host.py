@@ -2,6 +2,7 @@
 stand-in for the CUDA runtime (cpp/fake_cudart.cpp), in which device memory is
 host memory and kernels do not run. Each program checks one property and prints
 "ok"."""
+import importlib.util
 import shutil
 import subprocess
 from pathlib import Path
@@ -32,6 +33,7 @@ def run(tmp_path_factory):
         assert r.returncode == 0, r.stderr
         r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
         assert r.returncode == 0 and r.stdout.endswith("ok\n"), r.stdout + r.stderr
+        return r.stdout.splitlines()[:-1]
 
     return go
 
@@ -42,3 +44,16 @@ def test_compile_beside_another_threads_capture(run):
 
 def test_failed_allocations_leave_nothing_stale(run):
     run("engine_alloc_failures")
+
+
+def test_bench_counts_the_launches_of_a_frame(run):
+    """The bench's launch count (frame_launches) against the launches that the engine makes."""
+    spec = importlib.util.spec_from_file_location("bench_under_test", ROOT / "bench.py")
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+    lines = run("engine_frame_launches")
+    assert len(lines) >= 20
+    for line in lines:
+        views, n, w, h, lookback, ctas, launches = map(int, line.split())
+        settings = {"key_sort_lookback": lookback, "sort_ctas_per_sm": ctas}
+        assert bench.frame_launches(views, n, (w + 15) // 16, (h + 15) // 16, settings) == launches, line
