@@ -44,3 +44,32 @@ def test_one_pixels_gradient_stays_with_its_entries(cuda, value, channels, round
         assert np.linalg.norm((a - b)[~counted]) <= tol.GRAD_REL * np.linalg.norm(b[~counted])
     if not np.isfinite(value):
         assert not np.isfinite(got[-1][counted][:, [6 + c for c in channels]]).any()
+
+
+def test_an_infinite_colour_stays_with_pixels_that_meet_it(cuda):
+    """A Gaussian of infinite colour makes the gradient undefined at the pixels whose block meets
+    it. An entry that such a pixel does not count takes nothing from it: with the gradient 0
+    outside those pixels, the geometry of every Gaussian that they do not count gets exactly 0."""
+    torch = cuda
+    sc = configs.scene("cfg2", N)
+    sh = np.ascontiguousarray(sc.sh).copy()
+    sh[5, :3] = np.inf
+    params = [torch.from_numpy(np.ascontiguousarray(a)).cuda()
+              for a in (sc.means, sc.log_scales, sc.quats, sc.opacity_logits, sh)]
+    eng = T.GaussianEngine()
+    eng.compile_params(*params)
+    eng.set_camera(T.Camera.orbit((0.0, 0.0, -5.0), W, H))
+    eng.raster_frame()
+    bad = ~np.isfinite(eng.read_image()[0]).all(-1)
+    assert 0 < bad.sum() < bad.size
+
+    def records(dimg):
+        eng.backward(torch.from_numpy(dimg).cuda().reshape(-1))
+        return eng.read_buffer(L.TPD_BUF_G2D, np.float32, N * 12).reshape(N, 12)[:, :9]
+
+    dimg = np.where(bad[..., None], np.float32(1.0), np.float32(0.0)) * np.ones((1, 1, 3), np.float32)
+    got = records(dimg)
+    eng.close()
+    counted = got[:, 6] > 0.0  # weights of those pixels
+    assert 0 < counted.sum() < N
+    assert not np.any(got[~counted])

@@ -1269,6 +1269,7 @@ void enqueue_backward(tpd_engine* e, const float* dL_dimage, const BackwardOut& 
     bb.g2d_view_stride = uint64_t(e->n) * kG2DStride;
     // longest walks first: the adjoint's cost per tile varies more than the forward's
     launch_tile_order(e->d_tile_len, e->total_tiles, e->d_ctl, e->d_tile_order, e->stream);
+    bb.tile_len = e->d_tile_len;
     bb.tile_order = e->d_tile_order;
     mark(TPD_STAGE_BACKWARD_SETUP + 1);
     launch_blend_backward(bb, blend_launch(e), e->stream);

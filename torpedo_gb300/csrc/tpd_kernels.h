@@ -262,7 +262,8 @@ struct BlendArgs {
     float* final_T;
     uint32_t* n_contrib;
     // with them: per tile, the list entries up to its last contributor, whose
-    // classes are counted in ctl->tile_hist (for launch_tile_order)
+    // classes are counted in ctl->tile_hist (for launch_tile_order); the top bit
+    // is set where a pixel's colour is infinite or close to it
     uint32_t* tile_len;
     // nullable: the image also as RGBA8 UNORM (alpha 255), packed like image
     // (launch_pack_rgba8's conversion), written with it
@@ -300,6 +301,7 @@ struct BlendBackwardArgs {
     const float* dL_dimage;   // HWC float3
     float* g2d;               // n x kG2DStride (px, py, conic.xyz, opacity, rgb, 3 pad), accumulated
     uint64_t g2d_view_stride; // floats between views' g2d (n * kG2DStride)
+    const uint32_t* tile_len;    // as the blend left it
     const uint32_t* tile_order;  // nullable: CTA b differentiates tile tile_order[b] (launch_tile_order)
 };
 void launch_blend_backward(const BlendBackwardArgs& a, const BlendLaunch& l, cudaStream_t s);
