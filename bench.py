@@ -573,10 +573,11 @@ def run_ours(args):
     # pass's kernels (read + write), times K
     traffic = None
     tfile = ROOT / "profiles" / "radix_pass_traffic.json"
-    if tfile.exists() and not strips:
-        t = json.loads(tfile.read_text())
-        per_key = t.get("counted" if counted else "onesweep")
+    if tfile.exists():
+        per_key = json.loads(tfile.read_text()).get(form)
         traffic = int(per_key * K) if per_key else None
+    # bytes a pass moves on average: strips by the profile
+    moved = traffic if strips else K * ((12 + 20 * (passes - 1)) // passes if counted else 16)
     pass_kernel = ("scatter_kernel by column over strips, strip_rows_kernel + scatter_kernel by row over the keys "
                    "made from them (the key sort; one of its two passes on average)" if strips else
                    "partition_count_kernel (not in the first pass) + scatter_kernel "
@@ -645,13 +646,14 @@ def run_ours(args):
                      "bytes_per_launch": K * 24, "avg_launch_ms": round(pass_ms, 5),
                      "basis": "K * 24 B per pass: the per-pass term of the fixed sort formula "
                               "K * (8 + 24 * ceil(B / 8)) for 64-bit keys and 32-bit values",
-                     "moved_bytes_per_launch": None if strips else K * 16,
-                     "moved_GBps": None if strips else round(K * 16 / (pass_ms / 1000.0) / 1e9, 1),
-                     "moved_frac": None if strips else round(K * 16 / (pass_ms / 1000.0) / 1e9 / hbm, 4),
+                     "moved_bytes_per_launch": moved,
+                     "moved_GBps": moved and round(moved / (pass_ms / 1000.0) / 1e9, 1),
+                     "moved_frac": moved and round(moved / (pass_ms / 1000.0) / 1e9 / hbm, 4),
                      "moved_note": ("column strips (12 B each, several keys to a strip) are sorted, and the keys made "
-                                    "from them in the last pass, which writes 4 B per key; " if strips else
-                                    "the pass itself reads and writes 32-bit tile ids and 32-bit values (16 B per "
-                                    "key); ") + "the depth half of the keys is ordered by the depth presort",
+                                    "from them in the last pass, which writes 4 B per key: the frame does not report how "
+                                    "many strips there are, so the bytes are the profile's (ncu, DRAM); " if strips else
+                                    "a pass reads and writes 32-bit tile ids and 32-bit values (16 B per key; the last "
+                                    "counted pass writes no tile ids, and counting reads 4 B); ") + "the depth half of the keys is ordered by the depth presort",
                      "time_note": "avg_launch_ms = the key-sort stage / its passes; with counted passes the first "
                                   "pass's digits are counted as its keys (or strips) are written (in the keygen "
                                   "stage), so that pass has no counting launch"},
