@@ -14,21 +14,22 @@
 // per pixel the final transmittance and the number of list entries up to the
 // last contributor are kept for the adjoint. The adjoint walks each tile's
 // list back to front, recomputing transmittance as T / (1 - alpha) from the
-// final T (no per-pixel lists), and accumulates per-Gaussian gradients
-// warp-reduced, then in shared memory, then with one global atomic per
-// (round, Gaussian, field).
+// final T (no per-pixel lists). It stores each entry's sums per 8x4 block in
+// shared memory and adds them to the Gaussian's record with vector atomics, once
+// per round and entry.
 //
 // Every per-pixel operation (n2, alpha, the skip and stop tests) has the same
 // operations and explicit rounding in the forward and in the adjoint, so both
 // take identical decisions.
 //
-// Warp culling: a warp owns an 8x8 pixel block of the tile. The thread that
+// Block culling: the tile is four blocks of 8x8 pixels (the forward: one per
+// warp) or eight of 8x4 (the adjoint: four per warp). The thread that
 // stages a list entry also works out, once for the whole CTA, which of the
-// tile's four blocks the entry can reach: for each block row (a slab of
+// tile's blocks the entry can reach: for each block row (a slab of
 // pixel rows) it takes the x extent of the entry's alpha >= 1/255 ellipse
 // within the slab (closed form, two square roots), enlarged for rounding,
-// and compares it with the two block columns. A warp then walks only the
-// entries whose bit for its block is set (one ballot per 32 entries). A
+// and compares it with the two block columns. Only the entries whose bit for
+// a block is set are walked for it (found by one ballot per 32 entries). A
 // culled pair lies outside that ellipse, where the pair's own test finds
 // alpha below 1/255 and skips it, as the reference does; so the culling
 // changes which skipped pairs are visited, never a result.

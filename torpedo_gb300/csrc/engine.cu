@@ -106,7 +106,8 @@ struct tpd_engine {
     uint32_t total_tiles = 0;
     uint64_t total_pixels = 0;
     uint32_t* d_tile_view = nullptr;
-    uint32_t* d_tile_len = nullptr;    // per tile, list entries up to its last contributor (frames keeping the adjoint's inputs)
+    // per tile, list entries up to its last contributor (frames keeping the adjoint's inputs)
+    uint32_t* d_tile_len = nullptr;
     uint32_t* d_list_buckets = nullptr;  // tiles by class of their list length, for the blend
     uint64_t list_bucket_cap = 0;
     uint32_t* d_tile_order = nullptr;  // tiles by decreasing d_tile_len, for the blend adjoint
@@ -1359,8 +1360,8 @@ namespace {
 // The sorted (tile | depth) keys of the last frame, for read-back: the frame
 // itself sorts tile ids only (their depth order comes from the presort) and
 // ends with their ranges, and a key's depth is that of its value's splat, so
-// the keys are rebuilt here
-// into a buffer of their own, allocated on first use. Waits for the stream.
+// the keys are rebuilt here into a buffer of their own, allocated on first use.
+// Waits for the stream.
 int rebuild_keys(tpd_engine* e) {
     cudaSetDevice(e->device);
     if (e->keys64_cap < e->capacity) {
@@ -1470,11 +1471,11 @@ int tpd_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* keys_alt, uint32_t*
     plan.key_bits = key_bits;
     plan.hist = ctl->sort_hist;
     plan.hist_ready = false;
-    // onesweep passes of 256 threads x 16 keys (ballot ranking, 2 CTAs per SM)
-    // with a look-back: on 64-bit keys faster than 512 x 8 keys with match
-    // ranking (0.845 against 0.910 ms for 9M random keys of 45 bits, the
-    // histogram kernel included) and than the counted passes that serve the
-    // frame's 32-bit key sort
+    // onesweep passes of 256 threads with a look-back, 16 keys a thread from
+    // 524289 pairs on (2 CTAs per SM): on 64-bit keys faster than 512 x 8 keys
+    // with match ranking (9M random keys of 45 bits, all with ballots: 0.845
+    // against 0.910 ms) and than the counted passes that serve the frame's
+    // 32-bit key sort
     plan.threads = 256;
     plan.items = sort_items_for(n);
     plan.ctas_per_sm = 2;

@@ -107,16 +107,16 @@ struct ScanItemsSmem {
 
 // kStrips: the items' strips (one per column of the rectangle) are scanned as
 // well, by a second look-back beside the first, and item_info and part_first
-// are those of the strip slots. (Registers for six CTAs per SM, as without: 48 ->
-// 45 us with the expansion, 1M Gaussians at 1080p.)
+// are those of the strip slots. (Registers for six CTAs per SM, as without,
+// with 12 bytes spilled: 48 -> 45 us with the expansion, 1M Gaussians at 1080p.)
 template <bool kStrips>
 __global__ void __launch_bounds__(kScanItemsThreads, 6)
     scan_items_kernel(const Splat* __restrict__ splats, const uint32_t* __restrict__ items,
                       const uint32_t* __restrict__ items_other, uint32_t n_items, uint32_t n,
                       const ViewConst* __restrict__ views, uint32_t* __restrict__ offsets,
                       uint4* __restrict__ item_info, uint32_t* __restrict__ part_first, uint32_t capacity,
-                      uint32_t* __restrict__ ranges, uint32_t n_tiles, uint64_t* desc, uint64_t* strip_desc, FrameCtl* ctl, uint32_t spin_limit,
-                      uint32_t never_publish) {
+                      uint32_t* __restrict__ ranges, uint32_t n_tiles, uint64_t* desc, uint64_t* strip_desc,
+                      FrameCtl* ctl, uint32_t spin_limit, uint32_t never_publish) {
     constexpr uint32_t kSums = kStrips ? 2u : 1u;
     __shared__ ScanItemsSmem S;
     pdl_wait();     // launched as a dependent of the depth sort's last pass: its order is read below
@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(kScanItemsThreads, 6)
 // Bound by latency and issue; the stores are 8 bytes a key. With one key per
 // thread and step (35 instructions a key, two dependent loads) 1M Gaussians at
 // 1080p took 67 us with the scan, 8 views of 500,000 at 720p 216; now 55 and
-// 162, with registers for four CTAs per SM (71 registers, three CTAs: 59 and
-// 171; five: 57 and 164).
+// 162, with 64 registers for four CTAs per SM, which spill 8 to 16 bytes (71
+// registers, three CTAs: 59 and 171; five: 57 and 164).
 constexpr uint32_t kExpandThreads = 256;
 constexpr uint32_t kExpandSlots = kCountedTile / kExpandThreads;
 constexpr uint32_t kTileDigitsMax = 4;
@@ -255,8 +255,8 @@ constexpr uint32_t kTileDigitsMax = 4;
 template <uint32_t kDig>
 __global__ void __launch_bounds__(kExpandThreads, 4)
     expand_keys_kernel(const uint4* __restrict__ item_info, const uint32_t* __restrict__ part_first,
-                       uint32_t* __restrict__ tiles, uint32_t* __restrict__ vals, uint32_t n_items, uint32_t capacity, uint32_t max_parts,
-                       uint32_t tile_bits, uint32_t* __restrict__ work, FrameCtl* ctl) {
+                       uint32_t* __restrict__ tiles, uint32_t* __restrict__ vals, uint32_t n_items,
+                       uint32_t capacity, uint32_t max_parts, uint32_t tile_bits, uint32_t* __restrict__ work, FrameCtl* ctl) {
     __shared__ __align__(16) uint16_t owner[kCountedTile];  // item of each slot, from the partition's first
     constexpr bool kCounted = kDig != 0;
     constexpr uint32_t kRows = kCounted ? 1u : kTileDigitsMax, kWidth = kCounted ? kDig : 256u;
@@ -432,9 +432,10 @@ void launch_keygen(const KeygenArgs& a, int num_sms, cudaStream_t s) {
     const int per_sm = device_once(scan_items_setup);  // resident CTAs per SM
     const uint64_t cap = uint64_t(num_sms > 0 ? num_sms : 148) * uint64_t(per_sm);  // persistent
     const uint64_t blocks = parts < cap ? parts : cap;
-    launch_dependent(a.strips ? scan_items_kernel<true> : scan_items_kernel<false>, dim3(unsigned(blocks)), dim3(kScanItemsThreads), 0, s, a.splats, a.items,
-                     a.items_other, a.n_items, a.n, a.views, a.offsets, a.item_info, a.part_first, a.capacity,
-                     a.ranges, a.n_tiles, a.desc, a.strip_desc, a.ctl, a.spin_limit, a.never_publish);
+    launch_dependent(a.strips ? scan_items_kernel<true> : scan_items_kernel<false>, dim3(unsigned(blocks)),
+                     dim3(kScanItemsThreads), 0, s, a.splats, a.items, a.items_other, a.n_items, a.n, a.views,
+                     a.offsets, a.item_info, a.part_first, a.capacity, a.ranges, a.n_tiles, a.desc, a.strip_desc,
+                     a.ctl, a.spin_limit, a.never_publish);
     const uint32_t max_parts = std::max(1u, uint32_t((uint64_t(a.capacity) + kCountedTile - 1) / kCountedTile));
     if (a.strips) {
         launch_dependent(expand_strips_kernel, dim3(max_parts), dim3(kExpandThreads), 0, s,
@@ -445,9 +446,9 @@ void launch_keygen(const KeygenArgs& a, int num_sms, cudaStream_t s) {
     const auto expand = !a.counted_work                                ? expand_keys_kernel<0>
                         : counted_digit_bits(a.tile_bits) > 8 ? expand_keys_kernel<512>
                                                               : expand_keys_kernel<256>;
-    launch_dependent(expand, dim3(max_parts),
-                     dim3(kExpandThreads), 0, s, static_cast<const uint4*>(a.item_info),
-                     static_cast<const uint32_t*>(a.part_first), a.tiles, a.vals, a.n_items, a.capacity, max_parts, a.tile_bits, a.counted_work, a.ctl);
+    launch_dependent(expand, dim3(max_parts), dim3(kExpandThreads), 0, s, static_cast<const uint4*>(a.item_info),
+                     static_cast<const uint32_t*>(a.part_first), a.tiles, a.vals, a.n_items, a.capacity, max_parts,
+                     a.tile_bits, a.counted_work, a.ctl);
 }
 
 namespace {

@@ -10,13 +10,13 @@
 // passes instead of 23.
 //  1. In the frame the digit histograms come from earlier kernels (the
 //     preprocess counts the depth keys' digits, key duplication those of the
-//     tile ids for look-back passes); sort_histogram_kernel builds them for standalone sorts (one
-//     read of the keys).
+//     tile ids for look-back passes); sort_histogram_kernel builds them for
+//     standalone sorts (one read of the keys).
 //  2. onesweep_kernel, once per pass: a persistent CTA takes 4096-key
 //     partitions by atomic ticket, loads them with coalesced warp-striped
 //     loads, ranks keys per warp (shared atomics where the digits are spread,
-//     else bit ballots, or match-any in the 512-thread variant; stable within the warp-striped order), combines warps per
-//     digit, publishes its digit counts, reorders the partition in shared
+//     else bit ballots, or match-any in the 512-thread variant; stable within
+//     the warp-striped order), combines warps per digit, publishes its digit counts, reorders the partition in shared
 //     memory while predecessors publish, resolves each digit's global prefix
 //     by a decoupled look-back (one thread per digit, four predecessors per
 //     round trip, bounded spin) and writes digit runs out coalesced.
@@ -26,7 +26,8 @@
 // In the frame the depth presort sorts 64-bit (view | depth) keys with
 // onesweep passes and the key sort 32-bit tile ids (their depth order is
 // already fixed) with counted passes; the standalone sort takes 64-bit keys
-// (onesweep, 256 threads x 16 keys).
+// (onesweep, 256 threads x 4, 8 or 16 keys by their number). Both 64-bit sorts
+// are one counting launch up to 12288 pairs (sort_small.cu).
 // The result is the stable sort of the pairs by the low key_bits bits, the
 // same permutation as the reference's sort.
 #include <algorithm>
@@ -46,7 +47,7 @@ constexpr uint32_t kRadix = 1u << kRadixBits;
 constexpr uint32_t kSortThreads = 256;
 // Keys per thread of a radix pass: 16 (4096-key partitions) for large sorts;
 // 8 or 4 give more, shorter partitions when the sort is too small to fill the
-// GPU with 4096-key partitions (the depth sort of 1M Gaussians).
+// GPU with 4096-key partitions (sort_items_for).
 constexpr uint32_t kSortItemsMax = 16;
 constexpr uint32_t kInvalidDigit = kRadix;                  // keys past K (and dropped keys)
 
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     // must be placed on empty SMs, not onto the first ones this grid frees
     pdl_wait();
     // digits ranked with match-any in the 512-thread variant (32 warps per SM
-    // hide its latency), with bit ballots otherwise (fixed cost)
+    // hide its latency), with shared atomics or bit ballots otherwise (below)
     constexpr bool kMatchRank = kThreads == 512;
     OnesweepSmem<kItems, kThreads, KeyT>& S = *reinterpret_cast<OnesweepSmem<kItems, kThreads, KeyT>*>(smem_raw);
     const bool digit_thread = threadIdx.x < kRadix;
@@ -511,12 +512,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 //     work area and scanned by the last CTAs to arrive (counted_finish in
 //     tpd_counted.cuh; nobody waits). The first pass of the frame's key sort
 //     is counted by the kernel that writes its keys (keygen.cu) instead.
-//  2. scatter_kernel, one CTA per partition: load, rank (bit ballots, stable
-//     in warp-striped order), reorder in shared memory and write out at the
+//  2. scatter_kernel, one CTA per partition: load, rank (bit ballots, or shared
+//     atomics over strips; stable in warp-striped order), reorder in shared memory and write out at the
 //     partition's global digit offsets, as onesweep_kernel does but with them
 //     known: no partition waits for another.
 // The permutation is the same stable one.
-// Digits have 8 bits, or 9 (kDig = 512) where that takes a pass less.
+// Digits have 8 bits, or 9 (kDig = 512) where that takes a pass less. (The
+// count's 40 registers for six CTAs per SM spill 4 bytes, 16 with 9 bits; the
+// 9-bit scatters spill 4.)
 template <int kItems, uint32_t kDig, typename KeyT>
 __global__ void __launch_bounds__(256, 6) partition_count_kernel(const KeyT* __restrict__ keys, uint32_t capacity,
                                                               uint32_t shift, uint32_t bits, uint32_t fixed_count,
@@ -600,7 +603,8 @@ struct StripList {
 // it spends, of the loads and of the arrivals (keygen + key sort with 1 / 2 / 4
 // / 8 of them: 817 / 798 / 789 / 816 us for 3M Gaussians at 2160p, 150 / 148 /
 // 151 / 154 for 1M at 1080p, 98 / 101 / 102 / 106 for 2M seen from inside).
-// (Registers for six CTAs per SM spill: 2 us more.)
+// (48 registers for five CTAs per SM spill 12 bytes; registers for six spill
+// more: 2 us slower.)
 template <uint32_t kParts>
 __global__ void __launch_bounds__(256, 5) strip_rows_kernel(StripList strips, uint32_t capacity, uint32_t max_parts,
                                                             uint32_t* __restrict__ work, FrameCtl* ctl,
@@ -671,7 +675,8 @@ struct ScatterSmem {
     uint32_t whist[8][kDig];        // per-warp digit counts, then the first slot of the warp's keys of each digit
     uint32_t gmap[kDig];            // global position of local index 0 of each digit
     uint32_t wsum[8];
-    uint32_t match[kMode >= kScatterColumns ? 8 : 1][kDig];  // strips: per warp and digit, the lanes that have it (0 at rest)
+    // strips: per warp and digit, the lanes that have it (0 at rest)
+    uint32_t match[kMode >= kScatterColumns ? 8 : 1][kDig];
     // columns: the local prefix of the heights, and the columns' offsets (strips,
     // heights), then the key slot of local height 0 of each column
     uint32_t hpre[kMode == kScatterColumns ? 4096 + 4096 / 16 : 1];
@@ -706,7 +711,8 @@ __global__ void __launch_bounds__(256, kMinBlocks)
     scatter_kernel(const KeyT* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, KeyT* __restrict__ keys_out,
                    uint32_t* __restrict__ vals_out, uint32_t capacity, uint32_t shift, uint32_t bits,
                    uint32_t fixed_count, uint32_t max_parts, uint32_t* __restrict__ work, FrameCtl* ctl,
-                   uint32_t* __restrict__ ranges, uint32_t n_tiles, uint32_t abort_mask, bool keys_just_written, StripList strips) {
+                   uint32_t* __restrict__ ranges, uint32_t n_tiles, uint32_t abort_mask, bool keys_just_written,
+                   StripList strips) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr bool kLast = kMode == kScatterLast || kMode == kScatterRows;
     constexpr bool kMatch = kMode >= kScatterColumns;  // lanes of one digit by shared atomics, not by ballots
@@ -747,7 +753,8 @@ __global__ void __launch_bounds__(256, kMinBlocks)
             // a strip's column << 8 | the row that it would have at the partition's slot 0, and its value
             slot_owners(owner, m, cnt, S.wsum, [&](uint32_t q) {
                 const uint32_t strip = strips.keys[first + q], slot = strips.starts[first + q] - base;
-                S.pairs[q] = make_uint2(strip_col(strip) << 8 | ((strip_row(strip) - slot) & 0xFFu), strips.vals[first + q]);
+                const uint32_t key = strip_col(strip) << 8 | ((strip_row(strip) - slot) & 0xFFu);
+                S.pairs[q] = make_uint2(key, strips.vals[first + q]);
                 return slot;
             });
             col0 = S.pairs[0].x >> 8;
@@ -809,16 +816,16 @@ __global__ void __launch_bounds__(256, kMinBlocks)
                 if (kFull || d < kDig) peers = S.match[warp][d];
             } else {
 #pragma unroll
-            for (int b = 0; b < kBits; ++b) {
-                const bool on = (d >> b) & 1u;
-                const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
-                peers &= on ? bal : ~bal;
-            }
-            if constexpr (!kFull) {
-                const bool on = d >= kDig;
-                const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
-                peers &= on ? bal : ~bal;
-            }
+                for (int b = 0; b < kBits; ++b) {
+                    const bool on = (d >> b) & 1u;
+                    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
+                    peers &= on ? bal : ~bal;
+                }
+                if constexpr (!kFull) {
+                    const bool on = d >= kDig;
+                    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, on);
+                    peers &= on ? bal : ~bal;
+                }
             }
             const uint32_t leader = __ffs(peers) - 1;
             uint32_t prev = 0;
@@ -1024,7 +1031,9 @@ void launch_counted_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout,
                              shift, bits, plan.fixed_count, max_parts, work, ctl, plan.ranges, plan.n_tiles, abort,
                              counted, StripList{});
         };
-        auto either = [&](auto bits_tag) { last ? scatter(bits_tag, std::true_type{}) : scatter(bits_tag, std::false_type{}); };
+        auto either = [&](auto bits_tag) {
+            last ? scatter(bits_tag, std::true_type{}) : scatter(bits_tag, std::false_type{});
+        };
         if (kMinBlocks == 2 && bits <= 8) {
             either(std::integral_constant<int, 8>{});
         } else {
@@ -1046,8 +1055,8 @@ void launch_counted_passes(KeyT* kin, uint32_t* vin, KeyT* kout, uint32_t* vout,
 }
 
 template <int kBits, int kMode>
-void launch_strip_scatter(const StripSort& a, const StripList& strips, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
-                          uint32_t* vout, uint32_t bits, cudaStream_t s) {
+void launch_strip_scatter(const StripSort& a, const StripList& strips, const uint32_t* kin, const uint32_t* vin,
+                          uint32_t* kout, uint32_t* vout, uint32_t bits, cudaStream_t s) {
     device_once(scatter_setup<3, kBits, kMode, uint32_t>);
     launch_dependent(scatter_kernel<3, kBits, kMode, uint32_t>, dim3(a.max_parts()), dim3(256),
                      sizeof(ScatterSmem<256, kMode>), s, kin, vin, kout, vout, a.capacity, 0u, bits, 0u,
@@ -1098,15 +1107,17 @@ void launch_strip_sort(const StripSort& a, cudaStream_t s) {
         launch_strip_scatter<7, kScatterColumns>(a, strips, a.strips, a.vals, a.strips_alt, a.vals_alt, 7, s);
     else
         launch_strip_scatter<8, kScatterColumns>(a, strips, a.strips, a.vals, a.strips_alt, a.vals_alt, 8, s);
-    launch_dependent(strip_rows_kernel<kStripParts>, dim3((a.max_parts() + kStripParts - 1) / kStripParts), dim3(256), 0, s, strips, a.capacity, a.max_parts(),
-                     a.work, a.ctl, kStatusFatal | kStatusKeyOverflow);
+    launch_dependent(strip_rows_kernel<kStripParts>, dim3((a.max_parts() + kStripParts - 1) / kStripParts), dim3(256),
+                     0, s, strips, a.capacity, a.max_parts(), a.work, a.ctl, kStatusFatal | kStatusKeyOverflow);
     if (a.n_tiles <= 128 * a.gx)
         launch_strip_scatter<7, kScatterRows>(a, strips, nullptr, nullptr, nullptr, a.vals, 7, s);
     else
         launch_strip_scatter<8, kScatterRows>(a, strips, nullptr, nullptr, nullptr, a.vals, 8, s);
 }
 
-void launch_sort_begin(FrameCtl* ctl, uint32_t total, cudaStream_t s) { sort_begin_kernel<<<1, 256, 0, s>>>(ctl, total); }
+void launch_sort_begin(FrameCtl* ctl, uint32_t total, cudaStream_t s) {
+    sort_begin_kernel<<<1, 256, 0, s>>>(ctl, total);
+}
 
 namespace {
 template <typename KeyT>
